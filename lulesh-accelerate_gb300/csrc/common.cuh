@@ -481,6 +481,7 @@ __device__ __forceinline__ void constraint_keys(double ss, double vdov, double a
 // The same candidates with the arithmetic in double-float pairs (the
 // default plain path): the comparisons that decide which terms enter stay
 // on the FP64 values.
+template <class Fn>
 __device__ __forceinline__ void constraint_keys_df(double ss, double vdov, double arealg,
                                                    const lulesh_params &P,
                                                    unsigned long long &kc, unsigned long long &kh)
@@ -491,8 +492,8 @@ __device__ __forceinline__ void constraint_keys_df(double ss, double vdov, doubl
         const df64 s = to_df(ss), a = to_df(arealg), v = to_df(vdov);
         df64 dtf = s * s;
         if (lt(vdov, 0.)) dtf = fma(to_df(64.0 * P.qqc * P.qqc) * (a * a), v * v, dtf);
-        kc = order_key(to_double(a * df_rsqrt(dtf)));          // arealg / sqrt(dtf)
-        kh = order_key(to_double(df_div(to_df(P.dvovmax), fabs(v) + df64(1.e-20))));
+        kc = order_key(to_double(a * Fn::rsqrt(dtf)));          // arealg / sqrt(dtf)
+        kh = order_key(to_double(Fn::div(to_df(P.dvovmax), fabs(v) + df64(1.e-20))));
     }
 }
 

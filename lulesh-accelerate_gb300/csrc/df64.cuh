@@ -16,8 +16,8 @@
 //     double-word product of Hida, Li and Bailey's QD library (2001) --
 //     addition through two_sum of the high words, product through two_prod
 //     plus the cross terms, each renormalised by fast_two_sum;
-//   - reciprocal, quotient and inverse square root: an FP32 estimate refined
-//     by Newton steps carried out in double-float.
+//   - reciprocal, quotient and square roots: an FP32 estimate corrected by
+//     one step of its power series, the residual formed exactly.
 // Every operation is written with the _rn intrinsics, which the compiler
 // neither contracts nor reorders, so any kernel that inlines them rounds the
 // same way.
@@ -123,44 +123,149 @@ __device__ __forceinline__ df64 fabs(df64 a) { return a.hi < 0.f ? -a : a; }
 __device__ __forceinline__ bool df_gt(df64 a, df64 b) { return a.hi > b.hi || (a.hi == b.hi && a.lo > b.lo); }
 __device__ __forceinline__ df64 fmax(df64 a, df64 b) { return df_gt(b, a) ? b : a; }
 
-// Reciprocal: r0 = the FP32 reciprocal, then two Newton steps
-// r <- r + r (1 - b r) with the residual formed in double-float; each step
-// squares the relative error (2^-23 -> 2^-46 -> below the format's
-// rounding).
-__device__ __forceinline__ df64 df_rcp(df64 b)
+// The FP32 estimates that the functions below refine (the hardware's
+// approximate reciprocal and inverse square root, a few units in the last
+// place; subnormal arguments included).
+__device__ __forceinline__ float rcp_estimate(float b)
 {
-    const float r0 = __frcp_rn(b.hi);
-    df64 r{r0, 0.f};
-#pragma unroll
-    for (int it = 0; it < 2; ++it) {
-        const df64 e = df_add(df64(1.0), -df_mul(b, r));
-        r = df_fma(r, e, r);
-    }
+    float r;
+    asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(b));
+    return r;
+}
+__device__ __forceinline__ float rsqrt_estimate(float a)
+{
+    float r;
+    asm("rsqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(a));
     return r;
 }
 
-// a / b: the quotient through the reciprocal, corrected once by the
-// remainder a - q b.
+// Reciprocal, quotient and roots: one series step from the FP32 estimate
+// instead of two Newton steps carried out in pairs.  The estimate is first
+// refined to a correctly rounded float or next to one; with y that float and
+// e = 1 - b y (or 1 - a y^2) its residual, formed by fused multiply-adds
+// whose large terms cancel exactly, |e| is near 2^-23, so the correction
+// needs only FP32: its roundings enter at 2^-24 |e|, near 2^-47 of the
+// result, and the first neglected term of the series is of order e^3.  Each
+// takes 9-15 FP32 operations where the Newton forms take 72-110 and the
+// reciprocal's correctly rounded estimate is a software routine of its own.
+// Root-mean-square errors over random pairs: 1/b 2^-49.0, a/b 2^-48.5,
+// 1/sqrt(a) 2^-49.1, sqrt(a) 2^-48.5, within a quarter bit of the Newton
+// forms' (tests/test_df_functions.py).
+
+// y + s t (|s t| << |y|) with one rounding of each word
+__device__ __forceinline__ df64 df_corrected(float y, float s, float t)
+{
+    const float hi = __fmaf_rn(s, t, y);
+    return {hi, __fmaf_rn(s, t, __fsub_rn(y, hi))};
+}
+
+// 1/b = y (1 + e + e^2 + ...)
+__device__ __forceinline__ df64 df_rcp(df64 b)
+{
+    const float y0 = rcp_estimate(b.hi);
+    const float y = __fmaf_rn(y0, __fmaf_rn(-b.hi, y0, 1.f), y0);
+    const float e = __fmaf_rn(-b.lo, y, __fmaf_rn(-b.hi, y, 1.f));
+    return df_corrected(y, y, __fmaf_rn(e, e, e));
+}
+
+// a/b: the FP32 quotient q by the refined reciprocal y, then its remainder
+// a - b q (exact in its high words) times y (1 + e)
 __device__ __forceinline__ df64 df_div(df64 a, df64 b)
 {
-    const df64 r = df_rcp(b);
+    const float y0 = rcp_estimate(b.hi);
+    const float y = __fmaf_rn(y0, __fmaf_rn(-b.hi, y0, 1.f), y0);
+    const float e = __fmaf_rn(-b.lo, y, __fmaf_rn(-b.hi, y, 1.f));
+    const float q = __fmul_rn(a.hi, y);
+    const float r = __fadd_rn(__fmaf_rn(-b.hi, q, a.hi), __fmaf_rn(-b.lo, q, a.lo));
+    return df_corrected(q, y, __fmaf_rn(r, e, r));
+}
+
+// 1/sqrt(a) = y (1 + e/2 + 3 e^2/8 + ...), a > 0
+__device__ __forceinline__ df64 df_rsqrt(df64 a)
+{
+    const float y0 = rsqrt_estimate(a.hi);
+    const float y = __fmaf_rn(__fmul_rn(0.5f, y0), __fmaf_rn(-a.hi, __fmul_rn(y0, y0), 1.f), y0);
+    const df64 s = two_prod(y, y);
+    const float e = __fadd_rn(__fmaf_rn(-a.hi, s.hi, 1.f), __fmaf_rn(-a.lo, s.hi, __fmul_rn(-a.hi, s.lo)));
+    return df_corrected(y, __fmul_rn(0.5f, y), __fmaf_rn(__fmul_rn(0.75f, e), e, e));
+}
+
+// sqrt(a), a > 0: the FP32 root x by the refined inverse root y, then its
+// remainder a - x^2 (exact in its high words) times y/2
+__device__ __forceinline__ df64 df_sqrt(df64 a)
+{
+    const float y0 = rsqrt_estimate(a.hi);
+    const float y = __fmaf_rn(__fmul_rn(0.5f, y0), __fmaf_rn(-a.hi, __fmul_rn(y0, y0), 1.f), y0);
+    const float x = __fmul_rn(a.hi, y);
+    const float r = __fadd_rn(__fmaf_rn(-x, x, a.hi), a.lo);
+    return df_corrected(x, __fmul_rn(0.5f, y), r);
+}
+
+// The Newton forms: two steps r <- r + r (1 - b r) or y <- y + y (1 - a y^2)/2
+// in pairs from the FP32 value.  The split-precision kernels keep them: their
+// FP32 forces magnify a change in the last bit of a time step or volume to
+// 1e-7 of the state within tens of cycles, so these kernels' results stay
+// bit for bit what they were.  Written out with what is known about the
+// operands: 1 - m with m near 1 is exact in its high words, the correction
+// is smaller than what it corrects (fast_two_sum), and the first step's
+// low word is zero; the same bits as the general operations in 43-50 FP32
+// operations instead of 66-80.
+__device__ __forceinline__ df64 df_one_minus(df64 m) { return fast_two_sum(__fsub_rn(1.f, m.hi), -m.lo); }
+
+// c + a b, |a b| < |c|
+__device__ __forceinline__ df64 df_fma_small(df64 a, df64 b, df64 c)
+{
+    const df64 p = two_prod(a.hi, b.hi);
+    const float t = __fmaf_rn(a.hi, b.lo, __fmaf_rn(a.lo, b.hi, p.lo));
+    const df64 s = fast_two_sum(c.hi, p.hi);
+    return fast_two_sum(s.hi, __fadd_rn(__fadd_rn(s.lo, t), c.lo));
+}
+
+// c + c e for a float c, |e| < 1
+__device__ __forceinline__ df64 df_fma_small(float a, df64 b, float c)
+{
+    const df64 p = two_prod(a, b.hi);
+    const df64 s = fast_two_sum(c, p.hi);
+    return fast_two_sum(s.hi, __fadd_rn(s.lo, __fmaf_rn(a, b.lo, p.lo)));
+}
+
+__device__ __forceinline__ df64 df_rcp_newton(df64 b)
+{
+    const float r0 = __frcp_rn(b.hi);
+    const df64 r = df_fma_small(r0, df_one_minus(df_mul_f(b, r0)), r0);
+    return df_fma_small(r, df_one_minus(df_mul(b, r)), r);
+}
+
+// a / b: the quotient through the reciprocal, corrected once by the
+// remainder a - q b
+__device__ __forceinline__ df64 df_div_newton(df64 a, df64 b)
+{
+    const df64 r = df_rcp_newton(b);
     const df64 q = df_mul(a, r);
     const df64 rem = df_add(a, -df_mul(q, b));
     return df_fma(rem, r, q);
 }
 
-// 1 / sqrt(a), a > 0: the FP32 estimate, then two Newton steps
-// y <- y + y (1 - a y^2) / 2 in double-float.
-__device__ __forceinline__ df64 df_rsqrt(df64 a)
+__device__ __forceinline__ df64 df_rsqrt_newton(df64 a)
 {
-    df64 y{rsqrtf(a.hi), 0.f};
-#pragma unroll
-    for (int it = 0; it < 2; ++it) {
-        const df64 e = df_add(df64(1.0), -df_mul(a, df_mul(y, y)));
-        y = df_fma(df_scale(y, 0.5f), e, y);
-    }
-    return y;
+    const float y0 = rsqrtf(a.hi);
+    const df64 y = df_fma_small(__fmul_rn(0.5f, y0), df_one_minus(df_mul(a, two_prod(y0, y0))), y0);
+    return df_fma_small(df_scale(y, 0.5f), df_one_minus(df_mul(a, df_mul(y, y))), y);
 }
+
+// The two sets, for the code that both precisions share
+struct SeriesFn {
+    static __device__ __forceinline__ df64 rcp(df64 b) { return df_rcp(b); }
+    static __device__ __forceinline__ df64 div(df64 a, df64 b) { return df_div(a, b); }
+    static __device__ __forceinline__ df64 rsqrt(df64 a) { return df_rsqrt(a); }
+    static __device__ __forceinline__ df64 sqrt(df64 a) { return df_sqrt(a); }
+};
+struct NewtonFn {
+    static __device__ __forceinline__ df64 rcp(df64 b) { return df_rcp_newton(b); }
+    static __device__ __forceinline__ df64 div(df64 a, df64 b) { return df_div_newton(a, b); }
+    static __device__ __forceinline__ df64 rsqrt(df64 a) { return df_rsqrt_newton(a); }
+    static __device__ __forceinline__ df64 sqrt(df64 a) { return df_mul(a, df_rsqrt_newton(a)); }
+};
 
 // ---- conversions --------------------------------------------------------
 
@@ -210,9 +315,6 @@ __device__ __forceinline__ double df_f2d(float f)
 
 // pair -> double: one FP64 addition (the correctly rounded sum of the words)
 __device__ __forceinline__ double to_double(df64 a) { return df_f2d(a.hi) + df_f2d(a.lo); }
-
-// quotient overload for the geometry templates (hexmodes.cuh)
-__device__ __forceinline__ df64 quot_fast(df64 a, df64 b) { return df_div(a, b); }
 
 __device__ __forceinline__ float2 as_float2(df64 a) { return make_float2(a.hi, a.lo); }
 __device__ __forceinline__ df64 as_df(float2 f) { return {f.x, f.y}; }

@@ -30,12 +30,13 @@ __device__ __forceinline__ df64 eos_pressure_df(df64 &bvc, df64 e, df64 comp, bo
 }
 
 // sqrt((pbvc e + vv^2 bvc p) / rho0) with the reference's floor (:2485-2493)
+template <class Fn>
 __device__ __forceinline__ df64 sound_term_df(df64 e, df64 vv, df64 bvc, df64 p, double rho0, bool unit_rho0)
 {
     df64 ssc = fma(df64(2.0 / 3.0), e, vv * vv * bvc * p);
-    if (!unit_rho0) ssc = df_div(ssc, to_df(rho0));
+    if (!unit_rho0) ssc = Fn::div(ssc, to_df(rho0));
     if (!df_gt(ssc, df64(.111111e-36))) return df64(.333333e-18);
-    return ssc * df_rsqrt(ssc);
+    return Fn::sqrt(ssc);
 }
 
 __device__ __forceinline__ void opaque_df(df64 &v) { asm volatile("" : "+f"(v.hi), "+f"(v.lo)); }
@@ -49,6 +50,8 @@ __device__ __forceinline__ void opaque_df(df64 &v) { asm volatile("" : "+f"(v.hi
 // addition: the energy keeps its FP64 precision, and only the increments
 // carry the pairs' ~2^-47.  The comparisons against the cuts and bounds use
 // the same quantities as the FP64 kernel, in whichever form they are held.
+// Fn: the reciprocal and root functions (SeriesFn, NewtonFn).
+template <class Fn>
 __device__ __forceinline__ double material_update_df(const Dom &d, int k, DevScalars *sc, double vnew,
                                                      df64 qlin_in, df64 qquad_in, int rep)
 {
@@ -83,9 +86,9 @@ __device__ __forceinline__ double material_update_df(const Dom &d, int k, DevSca
         }
         const df64 one(1.f, 0.f);
         const df64 dvc = to_df(delvc), vn = to_df(vnewc);
-        df64 compression = df_rcp(vn) - one;
+        df64 compression = Fn::rcp(vn) - one;
         const df64 vchalf = vn - df_scale(dvc, 0.5f);
-        df64 comp_half = df_rcp(vchalf) - one;
+        df64 comp_half = Fn::rcp(vchalf) - one;
         df64 vhalf = vchalf;
         if (has_vmin && le(vnewc, eosvmin)) {
             comp_half = compression;
@@ -106,7 +109,7 @@ __device__ __forceinline__ double material_update_df(const Dom &d, int k, DevSca
         df64 e_df = to_df(e_new);
         const df64 p_half = eos_pressure_df(bvc, e_df, comp_half, p_zero, cut);
         q_new = df64(0.f, 0.f);
-        if (!gt(delvc, 0.)) q_new = fma(sound_term_df(e_df, vhalf, bvc, p_half, rho0, unit_rho0), qlin, qquad);
+        if (!gt(delvc, 0.)) q_new = fma(sound_term_df<Fn>(e_df, vhalf, bvc, p_half, rho0, unit_rho0), qlin, qquad);
         const df64 pq_half = p_half + q_new;
         e_new = e_new + to_double(df_scale(dvc * (df_mul_f(pq_old, 3.f) - df_mul_f(pq_half, 4.f)), 0.5f));
         if (abs_lt(e_new, e_cut)) e_new = 0.;
@@ -115,7 +118,7 @@ __device__ __forceinline__ double material_update_df(const Dom &d, int k, DevSca
         e_df = to_df(e_new);
         p_new = eos_pressure_df(bvc, e_df, compression, p_zero, cut);
         df64 q_tilde(0.f, 0.f);
-        if (!gt(delvc, 0.)) q_tilde = fma(sound_term_df(e_df, vn, bvc, p_new, rho0, unit_rho0), qlin, qquad);
+        if (!gt(delvc, 0.)) q_tilde = fma(sound_term_df<Fn>(e_df, vn, bvc, p_new, rho0, unit_rho0), qlin, qquad);
         const df64 combo = (df_mul_f(pq_old, 7.f) - df_mul_f(pq_half, 8.f)) + (p_new + q_tilde);
         e_new = e_new - to_double(combo * dvc * df64(1.0 / 6.0));
         if (abs_lt(e_new, e_cut)) e_new = 0.;
@@ -123,7 +126,7 @@ __device__ __forceinline__ double material_update_df(const Dom &d, int k, DevSca
 
         e_df = to_df(e_new);
         p_new = eos_pressure_df(bvc, e_df, compression, p_zero, cut);
-        ssn = sound_term_df(e_df, vn, bvc, p_new, rho0, unit_rho0);
+        ssn = sound_term_df<Fn>(e_df, vn, bvc, p_new, rho0, unit_rho0);
         if (le(delvc, 0.)) {
             q_new = fma(ssn, qlin, qquad);
             if (df_gt(cut.q_cut, fabs(q_new))) q_new = df64(0.f, 0.f);

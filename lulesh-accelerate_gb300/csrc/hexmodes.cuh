@@ -246,16 +246,17 @@ __device__ __forceinline__ T max_face_cross2_64(const V3<T> &M1, const V3<T> &M2
 // trace, LULESH-OMP.cc:1864-1925, 1975-2020): the half-step Jacobian has
 // columns (M - dt2 Mv)/8 for the position modes M1..M3 and velocity modes
 // V1..V3, and the trace is sum(cofactor . velocity mode) / det.
-template <typename T>
+// rate = quotient(num, det), the division left to the caller's arithmetic.
+template <typename T, class Quot>
 __device__ __forceinline__ T strain_rate(const V3<T> &M1, const V3<T> &M2, const V3<T> &M3, const V3<T> &V1,
-                                         const V3<T> &V2, const V3<T> &V3m, T dt2)
+                                         const V3<T> &V2, const V3<T> &V3m, T dt2, Quot &&quotient)
 {
     const V3<T> A{M1.x - dt2 * V1.x, M1.y - dt2 * V1.y, M1.z - dt2 * V1.z};
     const V3<T> B{M2.x - dt2 * V2.x, M2.y - dt2 * V2.y, M2.z - dt2 * V2.z};
     const V3<T> C{M3.x - dt2 * V3m.x, M3.y - dt2 * V3m.y, M3.z - dt2 * V3m.z};
     const V3<T> cxi = cross3(B, C), cet = cross3(C, A), cze = cross3(A, B);
     const T num = dot3_acc(cze, V3m, dot3_acc(cet, V2, dot3(cxi, V1)));
-    return quot_fast(num, dot3(B, cet));
+    return quotient(num, dot3(B, cet));
 }
 
 }  // namespace lulesh

@@ -289,7 +289,8 @@ __device__ __forceinline__ void elem_kinematics_df(const Dom &d, int k, DevScala
     }
 
     // CalcKinematicsForElems, strain-rate part (:1975-2020)
-    d.vdov[k] = to_double(strain_rate(M1, M2, M3, V1, V2, V3v, to_df(0.5 * sc->deltatime)));
+    d.vdov[k] = to_double(strain_rate(M1, M2, M3, V1, V2, V3v, to_df(0.5 * sc->deltatime),
+                                      [](df64 a, df64 b) { return df_div(a, b); }));
 }
 
 __global__ void __launch_bounds__(kKinBlockFactor * kBlockElem, 2) k_elem_kinematics_df(const __grid_constant__ Dom d)
@@ -387,8 +388,8 @@ __device__ __forceinline__ void elem_material_df(const Dom &d, int k, DevScalars
         d.ql[k] = to_double(qlin);
         d.qq[k] = to_double(qquad);
     }
-    const double ssn = material_update_df(d, k, sc, vnew, qlin, qquad, d.reps ? __ldg(d.reps + k) : 1);
-    if (kConstraints) constraint_keys_df(ssn, vdov, d.arealg[k], P, kc, kh);
+    const double ssn = material_update_df<SeriesFn>(d, k, sc, vnew, qlin, qquad, d.reps ? __ldg(d.reps + k) : 1);
+    if (kConstraints) constraint_keys_df<SeriesFn>(ssn, vdov, d.arealg[k], P, kc, kh);
 }
 
 // Eight blocks per SM (64 registers, ~40 bytes spilled; 80 registers at six

@@ -328,7 +328,8 @@ __device__ __forceinline__ void elem_kinematics_fp64(const Dom &d, int k, DevSca
     }
 
     // CalcKinematicsForElems, strain-rate part (:1975-2020)
-    d.vdov[k] = strain_rate(M1, M2, M3, V1, V2, V3v, 0.5 * sc->deltatime);
+    d.vdov[k] = strain_rate(M1, M2, M3, V1, V2, V3v, 0.5 * sc->deltatime,
+                            [](double a, double b) { return quot_fast(a, b); });
 }
 
 __global__ void __launch_bounds__(kBlockElem) k_elem_kinematics(const __grid_constant__ Dom d)
@@ -415,7 +416,7 @@ __global__ void __launch_bounds__(kBlockElem) k_time_constraints(const __grid_co
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     unsigned long long kc = ~0ULL, kh = ~0ULL;
     if (k < d.ne && !skip_step(d)) {
-        if (d.df == kArithDF64) constraint_keys_df(d.ss[k], d.vdov[k], d.arealg[k], d.prm, kc, kh);
+        if (d.df == kArithDF64) constraint_keys_df<SeriesFn>(d.ss[k], d.vdov[k], d.arealg[k], d.prm, kc, kh);
         else constraint_keys(d.ss[k], d.vdov[k], d.arealg[k], d.prm, kc, kh);
     }
     block_min_publish(kc, kh, d.sc);

@@ -458,8 +458,9 @@ __device__ __forceinline__ void elem_kinematics_split(const Dom &d, int k, DevSc
     const double rel = to_double(rel_df);
     d.vnew[k] = rel;
     d.delv[k] = rel - d.v[k];
-    d.vdov[k] = to_double(strain_rate(M[0], M[1], M[2], V[0], V[1], V[2], to_df(0.5 * sc->deltatime)));
-    d.arealg[k] = to_double(df_scale(vol64, 0.25f) * df_rsqrt(max_face_cross2_64(M[0], M[1], M[2], M[3], M[4], M[5], X)));
+    d.vdov[k] = to_double(strain_rate(M[0], M[1], M[2], V[0], V[1], V[2], to_df(0.5 * sc->deltatime),
+                                      [](df64 a, df64 b) { return df_div_newton(a, b); }));
+    d.arealg[k] = to_double(df_scale(vol64, 0.25f) * df_rsqrt_newton(max_face_cross2_64(M[0], M[1], M[2], M[3], M[4], M[5], X)));
     if (rel <= 0.0) flag_error(sc, ERR_K3_VNEW, k);
 
     // FP32: monotonic-Q gradients (:2034-2180) through the high words of the
@@ -538,9 +539,9 @@ __device__ __forceinline__ void elem_material_split(const Dom &d, int k, DevScal
         }
         // the EOS, energy, sound speed and constraint candidates in pairs,
         // the energy accumulated in FP64 (eos_df.cuh)
-        const double ssn = material_update_df(d, k, sc, vnew, df64(qlin, 0.f), df64(qquad, 0.f),
+        const double ssn = material_update_df<NewtonFn>(d, k, sc, vnew, df64(qlin, 0.f), df64(qquad, 0.f),
                                               d.reps ? __ldg(d.reps + k) : 1);
-        if (kConstraints) constraint_keys_df(ssn, vdov, d.arealg[k], P, kc, kh);
+        if (kConstraints) constraint_keys_df<NewtonFn>(ssn, vdov, d.arealg[k], P, kc, kh);
     }
 }
 
