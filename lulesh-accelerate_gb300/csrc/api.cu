@@ -381,7 +381,7 @@ int create_from_mesh(const HostMesh &m, int precision, const lulesh_params *para
     d.df = arith_of(precision);
     if (precision != LULESH_PRECISION_SPLIT) {
         A(d.fcx, 8 * ne); A(d.fcy, 8 * ne); A(d.fcz, 8 * ne);
-        A(d.geo, (size_t)kGeoWords * ne);
+        A(d.geo, geo_words(d.df) * ne);
     } else {
         A(d.f32x, 8 * ne); A(d.f32y, 8 * ne); A(d.f32z, 8 * ne);
         A(d.xs, nn); A(d.ys, nn); A(d.zs, nn); A(d.xds, nn); A(d.yds, nn); A(d.zds, nn);
@@ -408,10 +408,8 @@ int create_from_mesh(const HostMesh &m, int precision, const lulesh_params *para
         const int k = m.node_elem_corner_list[i];
         slots[i] = (k & 7) * (int)ne + (k >> 3);
     }
-    std::vector<double> zeros(ne, 0.0), ones(ne, 1.0), e(ne, 0.0), inv_mass(nn);
-    for (size_t i = 0; i < nn; ++i) inv_mass[i] = 1.0 / m.nodal_mass[i];
-    std::vector<double> inv_volo(ne);
-    for (size_t i = 0; i < ne; ++i) inv_volo[i] = 1.0 / m.volo[i];
+    std::vector<double> ones(ne, 1.0), e(ne, 0.0), inv_mass, inv_volo;
+    m.reciprocals(d.df == kArithDF64, inv_volo, inv_mass);
     e[m.origin] = m.e0;
     cudaStream_t st = ctx->stream;
     auto up = [&](void *dst, const void *src, size_t bytes) {
@@ -727,6 +725,7 @@ int lulesh_get_field(lulesh_ctx *ctx, const char *name, double *host, long n)
     }
     CK(cudaMemcpyAsync(host, f, n * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
+    if (ctx->dom.df == kArithDF64 && pair_field_name(name)) pairs_to_doubles(host, n);
     return LULESH_OK;
 }
 
@@ -737,6 +736,12 @@ int lulesh_set_field(lulesh_ctx *ctx, const char *name, const double *host, long
     double *f = find_field(ctx, name, &node, &writable);
     if (!f) return fail(ctx, LULESH_ERR_ARG, std::string("unknown field ") + name);
     if (n != (node ? ctx->nn : ctx->ne)) return fail(ctx, LULESH_ERR_ARG, std::string("wrong length for field ") + name);
+    std::vector<double> pairs;
+    if (ctx->dom.df == kArithDF64 && pair_field_name(name)) {
+        pairs.resize((size_t)n);
+        doubles_to_pairs(host, n, pairs.data());
+        host = pairs.data();
+    }
     CK(cudaMemcpyAsync(f, host, n * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
     int rc = clear_errors(ctx);

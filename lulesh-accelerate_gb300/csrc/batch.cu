@@ -553,7 +553,7 @@ int lulesh_batch_create(int n, const int *sizes, const double *e0_scale, int ini
     d.df = arith_of(precision);
     if (precision != LULESH_PRECISION_SPLIT) {
         A(d.fcx, 8 * ne); A(d.fcy, 8 * ne); A(d.fcz, 8 * ne);
-        A(d.geo, (size_t)kGeoWords * ne);
+        A(d.geo, geo_words(d.df) * ne);
     } else {
         A(d.f32x, 8 * ne); A(d.f32y, 8 * ne); A(d.f32z, 8 * ne);
         A(d.xs, nn); A(d.ys, nn); A(d.zs, nn); A(d.xds, nn); A(d.yds, nn); A(d.zds, nn);
@@ -622,11 +622,9 @@ int lulesh_batch_create(int n, const int *sizes, const double *e0_scale, int ini
         up(volo + eo_i, m.volo.data(), nei * 8);
         up(emass + eo_i, m.elem_mass.data(), nei * 8);
         up(nmass + no_i, m.nodal_mass.data(), nni * 8);
-        std::vector<double> im(nni);
-        for (long k2 = 0; k2 < nni; ++k2) im[k2] = 1.0 / m.nodal_mass[k2];
+        std::vector<double> im, iv;
+        m.reciprocals(d.df == kArithDF64, iv, im);
         up(d.inv_mass + no_i, im.data(), nni * 8);
-        std::vector<double> iv(nei);
-        for (long k2 = 0; k2 < nei; ++k2) iv[k2] = 1.0 / m.volo[k2];
         up(d.inv_volo + eo_i, iv.data(), nei * 8);
         up(d.x + no_i, m.x.data(), nni * 8);
         up(d.y + no_i, m.y.data(), nni * 8);
@@ -876,6 +874,7 @@ int lulesh_batch_get_field(lulesh_batch *b, int i, const char *name, double *hos
             const long off = f.node ? b->noff[i] : b->eoff[i];
             BCK(cudaMemcpyAsync(host, f.p + off, n * sizeof(double), cudaMemcpyDeviceToHost, b->stream));
             BCK(cudaStreamSynchronize(b->stream));
+            if (d.df == kArithDF64 && pair_field_name(name)) pairs_to_doubles(host, n);
             return LULESH_OK;
         }
     return bfail(b, LULESH_ERR_ARG, std::string("unknown field ") + name);

@@ -202,16 +202,48 @@ __device__ __forceinline__ FaceNeighbours face_neighbours(const Dom &d, const De
 // node's coordinates -- the element below, behind and left of the node
 // first -- instead of loaded from the corner tables, which takes the
 // tables' loads and their dependent level off the node update.
+// A node's place in its cube: column, row and plane, and the cube's first
+// element.
+struct NodePlace {
+    int c, r, p, e0;
+    // the element dp planes, dr rows and dc columns (0 or 1 each) before the
+    // node, of which the node is the corner at that offset
+    __device__ bool inside(int s, int dp, int dr, int dc) const
+    {
+        return (unsigned)(p - dp) < (unsigned)s && (unsigned)(r - dr) < (unsigned)s && (unsigned)(c - dc) < (unsigned)s;
+    }
+    __device__ size_t element(int s, int dp, int dr, int dc) const
+    {
+        return (size_t)(e0 + ((p - dp) * s + (r - dr)) * s + (c - dc));
+    }
+};
+__device__ __forceinline__ NodePlace node_place(const Dom &d, const DevScalars *sc, int s, int n)
+{
+    const int en = s + 1;
+    if (d.s <= 0) n -= sc->node_begin;
+    return {n % en, (n / en) % en, n / (en * en), d.s > 0 ? 0 : sc->elem_begin};
+}
+// the corner at that offset, in the reference's corner order
+// (LULESH-OMP.cc:3023-3040)
+__device__ constexpr int corner_of(int dp, int dr, int dc)
+{
+    return dp ? (dr ? (dc ? 6 : 7) : (dc ? 5 : 4)) : (dr ? (dc ? 2 : 3) : (dc ? 1 : 0));
+}
+
+template <class F>
+__device__ __forceinline__ void for_listed_corners(const Dom &d, int n, F &&f)
+{
+    const int st = __ldg(d.corner_start + n), en = __ldg(d.corner_start + n + 1);
+    for (int i = st; i < en; ++i) f(__ldg(d.corner_list + i), i == st);
+}
+
 template <class F>
 __device__ __forceinline__ void for_node_corners(const Dom &d, const DevScalars *sc, int n, F &&f)
 {
     const int s = d.s > 0 ? d.s : sc->edge;
     if (s > 0) {
-        const int en = s + 1;
+        const NodePlace at = node_place(d, sc, s, n);
         const size_t ne = (size_t)d.ne;
-        const int e0 = d.s > 0 ? 0 : sc->elem_begin;
-        if (d.s <= 0) n -= sc->node_begin;
-        const int c = n % en, r = (n / en) % en, p = n / (en * en);
         bool first = true;
 #pragma unroll
         for (int dp = 1; dp >= 0; --dp)
@@ -219,17 +251,13 @@ __device__ __forceinline__ void for_node_corners(const Dom &d, const DevScalars 
             for (int dr = 1; dr >= 0; --dr)
 #pragma unroll
                 for (int dc = 1; dc >= 0; --dc) {
-                    const int ep = p - dp, er = r - dr, ec = c - dc;
-                    if (ep < 0 || ep >= s || er < 0 || er >= s || ec < 0 || ec >= s) continue;
-                    // the node is the corner at offset (dc, dr, dp) of its element
-                    const int corner = dp ? (dr ? (dc ? 6 : 7) : (dc ? 5 : 4)) : (dr ? (dc ? 2 : 3) : (dc ? 1 : 0));
-                    f((int)(corner * ne + (size_t)(e0 + (ep * s + er) * s + ec)), first);
+                    if (!at.inside(s, dp, dr, dc)) continue;
+                    f((int)(corner_of(dp, dr, dc) * ne + at.element(s, dp, dr, dc)), first);
                     first = false;
                 }
         return;
     }
-    const int st = __ldg(d.corner_start + n), en = __ldg(d.corner_start + n + 1);
-    for (int i = st; i < en; ++i) f(__ldg(d.corner_list + i), i == st);
+    for_listed_corners(d, n, f);
 }
 
 // One direction of the monotonic limiter (:2198-2228).
@@ -478,22 +506,21 @@ __device__ __forceinline__ void constraint_keys(double ss, double vdov, double a
     }
 }
 
-// The same candidates with the arithmetic in double-float pairs (the
-// default plain path): the comparisons that decide which terms enter stay
-// on the FP64 values.
+// The same candidates with the arithmetic in double-float pairs; the
+// comparisons that decide which terms enter (vdov != 0, vdov < 0) are the
+// caller's.
 template <class Fn>
-__device__ __forceinline__ void constraint_keys_df(double ss, double vdov, double arealg,
+__device__ __forceinline__ void constraint_keys_df(df64 ss, df64 vdov, df64 arealg, bool moving, bool compressing,
                                                    const lulesh_params &P,
                                                    unsigned long long &kc, unsigned long long &kh)
 {
     kc = ~0ULL;
     kh = ~0ULL;
-    if (iabs(vdov) != 0ULL) {
-        const df64 s = to_df(ss), a = to_df(arealg), v = to_df(vdov);
-        df64 dtf = s * s;
-        if (lt(vdov, 0.)) dtf = fma(to_df(64.0 * P.qqc * P.qqc) * (a * a), v * v, dtf);
-        kc = order_key(to_double(a * Fn::rsqrt(dtf)));          // arealg / sqrt(dtf)
-        kh = order_key(to_double(Fn::div(to_df(P.dvovmax), fabs(v) + df64(1.e-20))));
+    if (moving) {
+        df64 dtf = ss * ss;
+        if (compressing) dtf = fma(to_df(64.0 * P.qqc * P.qqc) * (arealg * arealg), vdov * vdov, dtf);
+        kc = order_key(to_double(arealg * Fn::rsqrt(dtf)));          // arealg / sqrt(dtf)
+        kh = order_key(to_double(Fn::div(to_df(P.dvovmax), fabs(vdov) + df64(1.e-20))));
     }
 }
 

@@ -64,6 +64,13 @@ struct HostMesh {
     void build(int s, int init_mode);
     // LULESH_OK, or LULESH_ERR_ARG with a message in *err
     int build_unstructured(const lulesh_unstructured_mesh &u, std::string *err);
+    // Reciprocal reference volumes and nodal masses for the kernels.  With
+    // even set, on the cube, each is taken of the mean of the entity's value
+    // and its mirror image's (rows and columns exchanged), which the set-up's
+    // sums leave an ulp apart: the double-float kernels keep a mirror-
+    // symmetric state exactly symmetric (dfpack.cuh), and these are the only
+    // data that would disturb it.
+    void reciprocals(bool even, std::vector<double> &inv_volo, std::vector<double> &inv_mass) const;
 
   private:
     void derive();                       // corner lists, volumes, masses
@@ -86,6 +93,12 @@ int region_reps(int r, int nr, int cost);
 // order x y z xd yd zd e p v q; LULESH_OK or LULESH_ERR_ARG with *err set.
 int write_domain_file(const char *basename, int s, long ne, long nn, const int *nodelist, int step,
                       double time, const double *const fields[10], std::string *err);
+// Fields that the double-float kernels keep as pairs of floats, by name, and
+// the conversions of their accessors: a pair is its exact sum, a double its
+// FP32 rounding and the remainder's.
+bool pair_field_name(const char *name);
+void pairs_to_doubles(double *a, long n);          // in place
+void doubles_to_pairs(const double *a, long n, double *out);
 // The message lulesh_last_error(NULL) returns.
 void set_last_error(const std::string &msg);
 void default_params(lulesh_params *p);
@@ -102,10 +115,11 @@ inline int arith_of(int precision)
     return precision == LULESH_PRECISION_FP64 ? kArithDF64 : kArithIEEE;
 }
 
-// Everything one kernel launch needs, passed by value.
-// Words per element of the FP64 path's geometry cache (Dom::geo).
-constexpr int kGeoWords = 39;
+// Words per element of the geometry cache (Dom::geo): in IEEE FP64 the modes
+// and the cross products, in pairs the modes alone.
+inline int geo_words(int df) { return df == kArithDF64 ? 21 : 39; }
 
+// Everything one kernel launch needs, passed by value.
 struct Dom {
     int s, ne, nn;
     int keep;                            // bit0: store nodal forces, bit1: store ql/qq
@@ -145,13 +159,15 @@ struct Dom {
     float2 *xs, *ys, *zs, *xds, *yds, *zds;
     double *inv_mass;
     double *inv_volo;                    // [ne] 1/volo (the element kernels need it)
-    // FP64 path: element geometry of the current positions, left by the
-    // kinematics kernel for the next cycle's force kernel (the positions do
-    // not change between the two): the Walsh modes M1..M7 (21 words) and the
-    // six shared cross products (18 words), [kGeoWords][ne]; valid while
-    // DevScalars::geo_valid is set.  Null: not kept.  With df set each word
-    // is a double-float pair (float2) instead of a double, and so are the
-    // corner forces fcx/fcy/fcz.
+    // FP64-state paths: element geometry of the current positions, left by
+    // the kinematics kernel for the next cycle's force kernel (the positions
+    // do not change between the two); valid while DevScalars::geo_valid is
+    // set.  Null: not kept.  In IEEE FP64 the Walsh modes M1..M7 (21 words)
+    // and the six shared cross products (18 words), [39][ne]; with df set the
+    // modes as packed pairs (store_geometry_df).  With df set each word of
+    // the corner forces fcx/fcy/fcz, of vdov and arealg and of the six
+    // monotonic-Q gradients is a double-float pair (float2) as well: only the
+    // step's own kernels read them, and the accessors convert.
     double *geo;
     float *gq;
     DevScalars *sc;

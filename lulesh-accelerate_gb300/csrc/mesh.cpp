@@ -76,6 +76,50 @@ void default_params(lulesh_params *p)
     p->refdens = 1.0;
 }
 
+bool pair_field_name(const char *name)
+{
+    for (const char *n : {"vdov", "arealg", "delv_xi", "delv_eta", "delv_zeta", "delx_xi", "delx_eta", "delx_zeta"})
+        if (!std::strcmp(name, n)) return true;
+    return false;
+}
+
+void pairs_to_doubles(double *a, long n)
+{
+    for (long i = 0; i < n; ++i) {
+        float w[2];
+        std::memcpy(w, a + i, sizeof w);
+        a[i] = (double)w[0] + (double)w[1];
+    }
+}
+
+void doubles_to_pairs(const double *a, long n, double *out)
+{
+    for (long i = 0; i < n; ++i) {
+        const float hi = (float)a[i];
+        const float w[2] = {hi, std::isfinite(hi) ? (float)(a[i] - (double)hi) : 0.f};
+        std::memcpy(out + i, w, sizeof w);
+    }
+}
+
+void HostMesh::reciprocals(bool even, std::vector<double> &inv_volo, std::vector<double> &inv_mass) const
+{
+    inv_volo.resize(ne);
+    inv_mass.resize(nn);
+    if (!even || s <= 0) {
+        for (long i = 0; i < ne; ++i) inv_volo[i] = 1.0 / volo[i];
+        for (long i = 0; i < nn; ++i) inv_mass[i] = 1.0 / nodal_mass[i];
+        return;
+    }
+    auto fill = [](const std::vector<double> &a, long n, std::vector<double> &out) {
+        for (long p = 0; p < n; ++p)
+            for (long r = 0; r < n; ++r)
+                for (long c = 0; c < n; ++c)
+                    out[(p * n + r) * n + c] = 1.0 / (0.5 * (a[(p * n + r) * n + c] + a[(p * n + c) * n + r]));
+    };
+    fill(volo, s, inv_volo);
+    fill(nodal_mass, s + 1, inv_mass);
+}
+
 // Node-to-corner lists in (element, corner) order, reference volumes and the
 // element and nodal masses of a filled-in nodelist.
 void HostMesh::derive()

@@ -28,9 +28,8 @@
 // absolute coordinates carries it to 2^-53 of the coordinates).
 #include "lulesh_internal.h"
 #include "kernels.h"
-#include "hexmodes.cuh"
 #include "common.cuh"
-#include "hourglass_df.cuh"
+#include "dfpack.cuh"
 #include "eos_df.cuh"
 #include "batch_kernels.cuh"
 
@@ -38,74 +37,83 @@
 
 namespace lulesh {
 
-// Modes M1..M7 of one coordinate of the 8 corners: the corners relative to
-// corner 0 formed in FP64 and split into pairs (the modes do not see a
-// translation).
-__device__ __forceinline__ void rel_modes_df(const double *__restrict__ f, const int nl[8], df64 m[7])
+// The modes of one coordinate of an element's corners.
+__device__ __forceinline__ ModePacks field_modes(const double *__restrict__ f, const int nl[8])
 {
     double c[8];
     gather8(f, nl, c);
-    df64 r[8];
-    r[0] = df64(0.f, 0.f);
-#pragma unroll
-    for (int i = 1; i < 8; ++i) r[i] = to_df(c[i] - c[0]);
-    walsh8(r, m);
+    return walsh_packs(corners_of(c));
 }
 
-// The three linear modes of the 8 corner velocities, likewise.
-__device__ __forceinline__ void rel_linear_df(const double *__restrict__ f, const int nl[8], df64 m[3])
+// Geometry cache (Dom::geo): the modes of x, y, z in the pairs that the
+// kernels hold them in, three 16-byte planes per coordinate, then the three
+// M4.  The cross products are formed again from them: 170 instructions
+// against 288 more bytes per element written and read.
+__device__ __forceinline__ void store_geometry_df(double *geo, size_t ne, int k, int field, const ModePacks &m)
 {
-    double c[8];
-    gather8(f, nl, c);
-    df64 r[8];
-    r[0] = df64(0.f, 0.f);
-#pragma unroll
-    for (int i = 1; i < 8; ++i) r[i] = to_df(c[i] - c[0]);
-    walsh_linear(r, m);
+    ulonglong2 *g = reinterpret_cast<ulonglong2 *>(geo) + (size_t)(3 * field) * ne + k;
+    g[0] = make_ulonglong2(m.m12.hi, m.m12.lo);
+    g[ne] = make_ulonglong2(m.m56.hi, m.m56.lo);
+    g[2 * ne] = make_ulonglong2(m.m73.hi, m.m73.lo);
+    reinterpret_cast<float2 *>(geo + 18 * ne)[field * ne + k] = as_float2(m.m4);
+}
+__device__ __forceinline__ ModePacks load_geometry_df(const double *geo, size_t ne, int k, int field)
+{
+    const ulonglong2 *g = reinterpret_cast<const ulonglong2 *>(geo) + (size_t)(3 * field) * ne + k;
+    const ulonglong2 a = __ldg(g), b = __ldg(g + ne), c = __ldg(g + 2 * ne);
+    return {{a.x, a.y}, {b.x, b.y}, {c.x, c.y}, as_df(__ldg(reinterpret_cast<const float2 *>(geo + 18 * ne) + field * ne + k))};
 }
 
-// Geometry cache as pairs: the layout of step_fp64.cu's store_geometry, one
-// float2 per word.
-__device__ __forceinline__ void store_geometry_df(double *__restrict__ geo, size_t ne, int k, const df64 mx[7],
-                                                  const df64 my[7], const df64 mz[7], const ModeCrosses<df64> &X)
+// The modes of the three coordinates as vectors.
+struct Modes {
+    V2x3n m12, m56;
+    V1x3 m3, m4;
+};
+__device__ __forceinline__ Modes modes_of(const ModePacks &x, const ModePacks &y, const ModePacks &z)
 {
-    float2 *g = reinterpret_cast<float2 *>(geo);
-#pragma unroll
-    for (int i = 0; i < 7; ++i) {
-        g[(3 * i + 0) * ne + k] = as_float2(mx[i]);
-        g[(3 * i + 1) * ne + k] = as_float2(my[i]);
-        g[(3 * i + 2) * ne + k] = as_float2(mz[i]);
-    }
-    const V3<df64> c[6] = {X.c23, X.c31, X.c12, X.c45, X.c64, X.c56};
-#pragma unroll
-    for (int i = 0; i < 6; ++i) {
-        g[(21 + 3 * i) * ne + k] = as_float2(c[i].x);
-        g[(22 + 3 * i) * ne + k] = as_float2(c[i].y);
-        g[(23 + 3 * i) * ne + k] = as_float2(c[i].z);
-    }
+    return {both(V2x3{x.m12, y.m12, z.m12}), both(V2x3{x.m56, y.m56, z.m56}),
+            {df2_y(x.m73), df2_y(y.m73), df2_y(z.m73)}, {x.m4, y.m4, z.m4}};
 }
 
-__device__ __forceinline__ void load_geometry_df(const double *__restrict__ geo, size_t ne, int k, df64 mx[7],
-                                                 df64 my[7], df64 mz[7], ModeCrosses<df64> &X)
+// The six cross products that the geometry is made of, in pairs: q1 =
+// (M4xM5, M4xM6), q2 = (M3xM1, M3xM2), q3 = (M1xM2, M5xM6), and the normal
+// generators n1 = M2xM3 + M4xM5, n2 = M3xM1 + M6xM4, n3 = M1xM2 + M5xM6.
+struct Crosses {
+    V2x3 q1, q2, q3;
+    V1x3 n1, n2, n3;
+};
+__device__ __forceinline__ Crosses crosses_of(const Modes &m)
 {
-    const float2 *g = reinterpret_cast<const float2 *>(geo);
-#pragma unroll
-    for (int i = 0; i < 7; ++i) {
-        mx[i] = as_df(__ldg(g + (3 * i + 0) * ne + k));
-        my[i] = as_df(__ldg(g + (3 * i + 1) * ne + k));
-        mz[i] = as_df(__ldg(g + (3 * i + 2) * ne + k));
-    }
-    V3<df64> c[6];
-#pragma unroll
-    for (int i = 0; i < 6; ++i)
-        c[i] = {as_df(__ldg(g + (21 + 3 * i) * ne + k)), as_df(__ldg(g + (22 + 3 * i) * ne + k)),
-                as_df(__ldg(g + (23 + 3 * i) * ne + k))};
-    X = {c[0], c[1], c[2], c[3], c[4], c[5]};
+    Crosses c;
+    const V2x3 d = first_of(m.m12), e = first_of(m.m56);
+    c.q1 = cross2(dup3(m.m4), m.m56);
+    c.q2 = cross2(dup3(m.m3), m.m12);
+    c.q3 = cross2_even(pack3(half_x(d), half_x(e)), both(pack3(half_y(d), half_y(e))));
+    c.n1 = sum1(half_x(c.q1), minus(half_y(c.q2)));
+    c.n2 = sum1(half_x(c.q2), minus(half_y(c.q1)));
+    c.n3 = sum1(half_x(c.q3), half_y(c.q3));
+    return c;
 }
 
 // ---------------------------------------------------------------------
-// Element force: stress + Flanagan-Belytschko hourglass, as pairs
+// Element force: stress + Flanagan-Belytschko hourglass, as pairs, in the
+// space of the Walsh modes
 // ---------------------------------------------------------------------
+//
+// The hourglass shape vectors are hourgam_m(c) = gamma_m(c) - (dV/dx_c . H_m)/V
+// (CalcFBHourglassForceForElems, LULESH-OMP.cc:1291-1473), with gamma_m the
+// corner signs of modes 4..7, H_m = M4..M7 and 192 dV/dx_c = sum_i s_i(c) W_i
+// over the modes 1..6.  Both contractions with them need only sums over
+// modes, never over corners.  With U_i the modes of one velocity component,
+//   G   = sum_i W_i U_i                        (192 sum_c dV/dx_c u_c)
+//   h_m = coefficient (U_m - (H_m/(192 V)) . G)
+//   K   = sum_m (H_m/(192 V)) h_m
+// and the corner forces are the inverse transform of
+//   F_i = h_i - W_i . K  (h_i = 0 for i < 4; no W_7)
+// plus the stress forces, which are linear in the corner signs: (p + q)/64
+// times the normal generators in F_1..F_3.  60 products per component
+// instead of 64 and the 96 that the shape vectors take, and the transforms
+// are additions.  Everything runs on pairs of modes (dfpack.cuh).
 __device__ __forceinline__ void elem_force_df(const Dom &d, int k, DevScalars *sc)
 {
     const size_t ne = (size_t)d.ne;
@@ -114,88 +122,121 @@ __device__ __forceinline__ void elem_force_df(const Dom &d, int k, DevScalars *s
     const double ssk = __ldg(d.ss + k), massk = __ldg(d.elem_mass + k);
     int nl[8];
     load_nodelist(d.nodelist, k, nl);
-    // the modes and shared cross products: kept by the previous cycle's
-    // kinematics kernel for these positions, else formed here by the same
-    // functions (the same bits either way)
-    df64 mx[7], my[7], mz[7];
-    ModeCrosses<df64> X;
+    // the modes: kept by the previous cycle's kinematics kernel for these
+    // positions, else formed here by the same function (the same bits)
+    ModePacks mx, my, mz;
     if (d.geo && sc->geo_valid) {
-        load_geometry_df(d.geo, ne, k, mx, my, mz, X);
+        mx = load_geometry_df(d.geo, ne, k, 0);
+        my = load_geometry_df(d.geo, ne, k, 1);
+        mz = load_geometry_df(d.geo, ne, k, 2);
     } else {
-        rel_modes_df(d.x, nl, mx);
-        rel_modes_df(d.y, nl, my);
-        rel_modes_df(d.z, nl, mz);
-        X = mode_crosses(mode(mx, my, mz, 0), mode(mx, my, mz, 1), mode(mx, my, mz, 2), mode(mx, my, mz, 3),
-                         mode(mx, my, mz, 4), mode(mx, my, mz, 5));
+        mx = field_modes(d.x, nl);
+        my = field_modes(d.y, nl);
+        mz = field_modes(d.z, nl);
     }
-    const V3<df64> M1 = mode(mx, my, mz, 0), M2 = mode(mx, my, mz, 1), M3 = mode(mx, my, mz, 2);
-    const V3<df64> M4 = mode(mx, my, mz, 3), M5 = mode(mx, my, mz, 4), M6 = mode(mx, my, mz, 5);
-    df64 dvdx[8], dvdy[8], dvdz[8];
-    V3<df64> nx[3];
-    force_geometry(M1, M2, M3, M4, M5, M6, X, dvdx, dvdy, dvdz, nx);   // 192 x dV/dx, normal generators
+    // the first velocity component's corners, in flight during the geometry
+    double un[8];
+    gather8(d.xd, nl, un);
 
-    // IntegrateStressForElems (LULESH-OMP.cc:853-903), as in step_fp64.cu:
-    // the stress forces are s . (Y1, Y2, Y3) with Y = ((p + q)/64) X; corners
-    // 4..7 carry the forces of corners 2, 3, 0, 1 negated; only the sign of
-    // the Jacobian volume M2.(M3 x M1)/64 is tested.
-    df64 Y[3][3];
+    V2x3 W12, W56, W34;
+    V1x3 n1, n2, n3;   // normal generators, times (p + q)/64
     {
+        const Modes M = modes_of(mx, my, mz);
+        const Crosses X = crosses_of(M);
+        const V2x3 d12 = first_of(M.m12), d56 = first_of(M.m56);
+        const V1x3 c31 = half_x(X.q2), c32 = half_y(X.q2), c12 = half_x(X.q3);
+        // only the sign of the Jacobian volume M3.(M1 x M2)/64 is tested
+        // (IntegrateStressForElems, LULESH-OMP.cc:853-903)
+        if (dot1(M.m3, c12).value().hi <= 0.f) flag_error(sc, ERR_K1_DETERM, k);
+        // W_1..3 = 3 (M2xM3) + M4xM5 and so on, W6 = M3xM5 + M4xM2 and -W5 =
+        // M3xM6 + M4xM1 in the halves of a pair, W4 = M2xM6 - M1xM5
+        auto scaled = [](const V1x3 &v, float s) { return V1x3{df_scale(v.x, s), df_scale(v.y, s), df_scale(v.z, s)}; };
+        const V2x3 w65 = cross2_sum(dup3(M.m3), M.m56, dup3(M.m4), swapped(M.m12));
+        const V1x3 w4 = cross1_sum(half_y(d12), half_y(d56), minus(half_x(d12)), half_x(d56));
+        W12 = pack3(sum1(X.n1, scaled(c32, -2.f)), sum1(X.n2, scaled(c31, 2.f)));
+        W34 = pack3(sum1(X.n3, scaled(c12, 2.f)), w4);
+        W56 = pack3(minus(half_y(w65)), half_x(w65));
         const df64 w = to_df((1.0 / 64.0) * (pk + qk));
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            Y[i][0] = w * nx[i].x;
-            Y[i][1] = w * nx[i].y;
-            Y[i][2] = w * nx[i].z;
-        }
-        if (dot3(M2, X.c31).hi <= 0.f) flag_error(sc, ERR_K1_DETERM, k);
+        auto times = [&](const V1x3 &v) { return V1x3{w * v.x, w * v.y, w * v.z}; };
+        n1 = times(X.n1);
+        n2 = times(X.n2);
+        n3 = times(X.n3);
     }
-    // (dim may be a run-time value: the component is selected, not indexed,
-    // so that Y stays in registers)
-    auto comp = [&](int i, int dim) { return dim == 0 ? Y[i][0] : (dim == 1 ? Y[i][1] : Y[i][2]); };
-    auto stress8 = [&](int dim, df64 f[8]) {
-        const df64 y0 = comp(0, dim), y1 = comp(1, dim);
-        const df64 a = y0 + y1, b = y0 - y1, z = comp(2, dim);
-        f[0] = -(a + z);   // (-,-,-)
-        f[1] = b - z;      // (+,-,-)
-        f[2] = a - z;      // (+,+,-)
-        f[3] = -(b + z);   // (-,+,-)
-        f[4] = -f[2];
-        f[5] = -f[3];
-        f[6] = -f[0];
-        f[7] = -f[1];
-    };
-    auto out_of = [&](int dim) {
-        return reinterpret_cast<float2 *>(dim == 0 ? d.fcx : (dim == 1 ? d.fcy : d.fcz));
-    };
-
     // CalcHourglassControlForElems (:1503-1558)
     const double determ = volok * vk;
     if (vk <= 0.0) flag_error(sc, ERR_K1_VOLUME, k);
-
     const double hourg = d.prm.hgcoef;
-    if (!gt(hourg, 0.0)) {
-#pragma unroll
-        for (int dim = 0; dim < 3; ++dim) {
-            df64 f[8];
-            stress8(dim, f);
-#pragma unroll
-            for (int c = 0; c < 8; ++c) out_of(dim)[c * ne + k] = as_float2(f[c]);
-        }
-        return;
+    const bool hourglass = gt(hourg, 0.0);
+    // H_m/(192 V) in pairs (M5, M6), (M4, M7), and the coefficient; the
+    // scalar factors are FP64 (a handful of operations)
+    V2x3 H56, H47;
+    df2n coef;
+    {
+        const double r = hourglass ? rcbrt_fast(determ) : 0.0;   // determ^(-1/3)
+        const df2n vi = df2_both(df2_dup(to_df((r * r * r) * (1.0 / 192.0))));
+        H56 = {df2_mul(mx.m56, vi), df2_mul(my.m56, vi), df2_mul(mz.m56, vi)};
+        H47 = {df2_mul(df2_pack(mx.m4, df2_x(mx.m73)), vi), df2_mul(df2_pack(my.m4, df2_x(my.m73)), vi),
+               df2_mul(df2_pack(mz.m4, df2_x(mz.m73)), vi)};
+        coef = df2_both(df2_dup(to_df(-hourg * 0.01 * ssk * massk * r)));
     }
 
-    // CalcFBHourglassForceForElems (:1291-1473); the scalar factors are FP64
-    // (a handful of operations), everything per corner is pairs
-    const double r = rcbrt_fast(determ);                    // determ^(-1/3)
-    const V3<df64> H[4] = {M6, M5, M4, mode(mx, my, mz, 6)};
-    fb_hourglass_df(d, nl, dvdx, dvdy, dvdz, H, to_df((r * r * r) * (1.0 / 192.0)),
-                    to_df(-hourg * 0.01 * ssk * massk * r), [&](int dim, const df64 hgf[8]) {
-                        // each corner's stress force plus its hourglass force
-                        df64 f[8];
-                        stress8(dim, f);
+    // One velocity component per iteration, the loop kept rolled (its body
+    // is most of the kernel's instructions); each iteration issues the next
+    // component's corner gather before its own arithmetic.
+#pragma unroll 1
+    for (int dim = 0; dim < 3; ++dim) {
+        // (the component is selected, not indexed, so that it stays in
+        // registers)
+        auto comp = [&](const V1x3 &v) {
+            return df64(dim == 0 ? v.x.hi : (dim == 1 ? v.y.hi : v.z.hi), dim == 0 ? v.x.lo : (dim == 1 ? v.y.lo : v.z.lo));
+        };
+        const df64 y1 = comp(n1), y2 = comp(n2), y3 = comp(n3);
+        df2 F12, F56;
+        df64 F3, F4, F7;
+        if (hourglass) {
+            const ModePacks u = walsh_packs(corners_of(un));
+            if (dim < 2) gather8(dim == 0 ? d.yd : d.zd, nl, un);
+            const df2n u12 = df2_both(u.m12), u56 = df2_both(u.m56), u34 = df2_both(df2_pack(df2_y(u.m73), u.m4));
+            auto modes_dot = [&](df2 a, df2 b, df2 c) {
+                return df2_both(df2_dup(joined(Dot2(a, u12).add(b, u56)).plus(joined(Dot2(c, u34))).value()));
+            };
+            const df2n Gx = modes_dot(W12.x, W56.x, W34.x);
+            const df2n Gy = modes_dot(W12.y, W56.y, W34.y);
+            const df2n Gz = modes_dot(W12.z, W56.z, W34.z);
+            // c - v.g
+            auto less = [](df2 c, const V2x3 &v, const df2n &gx, const df2n &gy, const df2n &gz) {
+                return Dot2(v.x, df2_minus(gx)).sub(v.y, gy).sub(v.z, gz).plus(c);
+            };
+            const df2 h56 = df2_mul(less(u.m56, H56, Gx, Gy, Gz).value(), coef);
+            const df2 h47 = df2_mul(less(df2_pack(u.m4, df2_x(u.m73)), H47, Gx, Gy, Gz).value(), coef);
+            const df2n h56n = df2_both(h56), h47n = df2_both(h47);
+            auto shape_dot = [&](df2 a, df2 b) {
+                return df2_both(df2_dup(joined(Dot2(a, h56n)).plus(joined(Dot2(b, h47n))).value()));
+            };
+            const df2n Kx = shape_dot(H56.x, H47.x), Ky = shape_dot(H56.y, H47.y), Kz = shape_dot(H56.z, H47.z);
+            F12 = less(df2_pack(y1, y2), W12, Kx, Ky, Kz).raw();
+            F56 = less(h56, W56, Kx, Ky, Kz).raw();
+            const df2 F34 = less(df2_pack(y3, df2_x(h47)), W34, Kx, Ky, Kz).raw();
+            F3 = df2_x(F34);
+            F4 = df2_y(F34);
+            F7 = df2_y(h47);
+        } else {
+            const df64 zero(0.f, 0.f);
+            F12 = df2_pack(y1, y2);
+            F56 = df2_pack(zero, zero);
+            F3 = y3;
+            F4 = F7 = zero;
+        }
+        df2 f[4];
+        inverse_walsh_packs(F12, F56, F3, F4, F7, f);
+        float2 *out = reinterpret_cast<float2 *>(dim == 0 ? d.fcx : (dim == 1 ? d.fcy : d.fcz)) + k;
+        const int corner[4][2] = {{2, 1}, {0, 3}, {6, 5}, {4, 7}};
 #pragma unroll
-                        for (int c = 0; c < 8; ++c) out_of(dim)[c * ne + k] = as_float2(f[c] + hgf[c]);
-                    });
+        for (int c = 0; c < 4; ++c) {
+            out[corner[c][0] * ne] = as_float2(df2_x(f[c]));
+            out[corner[c][1] * ne] = as_float2(df2_y(f[c]));
+        }
+    }
 }
 
 __global__ void __launch_bounds__(kBlockElem) k_elem_force_df(const __grid_constant__ Dom d)
@@ -209,24 +250,36 @@ __global__ void __launch_bounds__(kBlockElem) k_elem_force_df(const __grid_const
 // ---------------------------------------------------------------------
 // Node update: the corner gather as pairs, joined once in FP64
 // ---------------------------------------------------------------------
+//
+// On the structured cube the sum is a tree: in each plane of elements the
+// two on the diagonal and the two off it, so that exchanging rows and columns
+// exchanges operands only and the mirror symmetry that the element kernels
+// keep (dfpack.cuh) is not lost here.
 __device__ __forceinline__ void node_update_df(const Dom &d, int n, const DevScalars *sc)
 {
-    const float2 *cx = reinterpret_cast<const float2 *>(d.fcx);
-    const float2 *cy = reinterpret_cast<const float2 *>(d.fcy);
-    const float2 *cz = reinterpret_cast<const float2 *>(d.fcz);
-    df64 fx(0.f, 0.f), fy(0.f, 0.f), fz(0.f, 0.f);
-    for_node_corners(d, sc, n, [&](int c, bool first) {
-        if (first) {
-            fx = as_df(cx[c]);
-            fy = as_df(cy[c]);
-            fz = as_df(cz[c]);
-        } else {
-            fx = fx + as_df(cx[c]);
-            fy = fy + as_df(cy[c]);
-            fz = fz + as_df(cz[c]);
+    const float2 *const fc[3] = {reinterpret_cast<const float2 *>(d.fcx), reinterpret_cast<const float2 *>(d.fcy),
+                                 reinterpret_cast<const float2 *>(d.fcz)};
+    df64 f[3] = {df64(0.f, 0.f), df64(0.f, 0.f), df64(0.f, 0.f)};
+    const int s = d.s > 0 ? d.s : sc->edge;
+    if (s > 0) {
+        const NodePlace at = node_place(d, sc, s, n);
+        const size_t ne = (size_t)d.ne;
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            auto corner = [&](int dp, int dr, int dc) {
+                return at.inside(s, dp, dr, dc) ? as_df(fc[i][corner_of(dp, dr, dc) * ne + at.element(s, dp, dr, dc)])
+                                                : df64(0.f, 0.f);
+            };
+            auto plane = [&](int dp) { return (corner(dp, 1, 1) + corner(dp, 0, 0)) + (corner(dp, 1, 0) + corner(dp, 0, 1)); };
+            f[i] = plane(1) + plane(0);
         }
-    });
-    node_integrate(d, n, sc, to_double(fx), to_double(fy), to_double(fz));
+    } else {
+        for_listed_corners(d, n, [&](int c, bool first) {
+#pragma unroll
+            for (int i = 0; i < 3; ++i) f[i] = first ? as_df(fc[i][c]) : f[i] + as_df(fc[i][c]);
+        });
+    }
+    node_integrate(d, n, sc, to_double(f[0]), to_double(f[1]), to_double(f[2]));
 }
 
 __global__ void __launch_bounds__(kBlockNode) k_node_update_df(const __grid_constant__ Dom d)
@@ -241,56 +294,120 @@ __global__ void __launch_bounds__(kBlockNode) k_node_update_df(const __grid_cons
 // ---------------------------------------------------------------------
 // Element kinematics + monotonic-Q gradients, as pairs
 // ---------------------------------------------------------------------
+
+// 64 x the larger |u x v|^2 of the two faces of one direction (hexmodes.cuh):
+// |X + Y|^2 and |X - Y|^2 in the halves of a pair.
+__device__ __forceinline__ df64 face_pair_max(const V1x3 &X, const V1x3 &Y)
+{
+    auto comp = [](df64 x, df64 y) {
+        const df2 z = df2_add(df2_dup(x), df2_pack(y, -y));
+        const f2 h = f2_add(z.hi, z.lo);
+        return df2{h, f2_sub(z.lo, f2_sub(h, z.hi))};
+    };
+    const df2 x = comp(X.x, Y.x), y = comp(X.y, Y.y), z = comp(X.z, Y.z);
+    const V2x3 v{x, y, z};
+    const df2 n = dot2(v, both(v)).value();
+    return fmax(df2_x(n), df2_y(n));
+}
+
 __device__ __forceinline__ void elem_kinematics_df(const Dom &d, int k, DevScalars *sc)
 {
+    const size_t ne = (size_t)d.ne;
     int nl[8];
     load_nodelist(d.nodelist, k, nl);
-    df64 mx[7], my[7], mz[7];
-    rel_modes_df(d.x, nl, mx);
-    rel_modes_df(d.y, nl, my);
-    rel_modes_df(d.z, nl, mz);
-    df64 vx[3], vy[3], vz[3];
-    rel_linear_df(d.xd, nl, vx);
-    rel_linear_df(d.yd, nl, vy);
-    rel_linear_df(d.zd, nl, vz);
-    const V3<df64> M1 = mode(mx, my, mz, 0), M2 = mode(mx, my, mz, 1), M3 = mode(mx, my, mz, 2);
-    const V3<df64> M4 = mode(mx, my, mz, 3), M5 = mode(mx, my, mz, 4), M6 = mode(mx, my, mz, 5);
-    const V3<df64> V1{vx[0], vy[0], vz[0]}, V2{vx[1], vy[1], vz[1]}, V3v{vx[2], vy[2], vz[2]};
-
-    // CalcKinematicsForElems, volume part (:1950-1964)
-    const ModeCrosses<df64> X = mode_crosses(M1, M2, M3, M4, M5, M6);
-    store_geometry_df(d.geo, (size_t)d.ne, k, mx, my, mz, X);
+    const ModePacks mx = field_modes(d.x, nl), my = field_modes(d.y, nl), mz = field_modes(d.z, nl);
+    // the next cycle's force kernel works on these same positions; every
+    // context that runs this kernel keeps the cache
+    store_geometry_df(d.geo, ne, k, 0, mx);
+    store_geometry_df(d.geo, ne, k, 1, my);
+    store_geometry_df(d.geo, ne, k, 2, mz);
     if (k == sc->elem_begin) sc->geo_valid = 1;
-    const df64 vol64 = volume64_shared(M1, M2, M3, X);
-    // volume / volo, as a product with the reciprocal taken at set-up
-    const df64 rel_df = df_scale(vol64 * to_df(__ldg(d.inv_volo + k)), 1.f / 64.f);
-    const double rel = to_double(rel_df);
+
+    const Modes M = modes_of(mx, my, mz);
+    const Crosses X = crosses_of(M);
+    const V2x3 d12 = first_of(M.m12), d56 = first_of(M.m56);
+
+    // CalcKinematicsForElems, volume part (:1950-1964): 64 V = M3.(M1xM2) +
+    // (M1.(M4xM5) + M2.(M6xM4) + M3.(M5xM6))/3 (hexmodes.cuh), in the sums
+    // that a mirrored element shares (dfpack.cuh)
+    const df64 vol64 = [&] {
+        const df64 s = difference(dot2(d12, both(X.q1))).plus(dot1(M.m3, half_y(X.q3))).value();
+        return Dot1(s, df64(1.0 / 3.0)).plus(dot1(M.m3, half_x(X.q3))).value();
+    }();
+    // volume / volo, as a product with the reciprocal taken at set-up, in
+    // FP64: it is state, and one product costs less than its two conversions
+    const double rel = to_double(df_scale(vol64, 1.f / 64.f)) * __ldg(d.inv_volo + k);
     d.vnew[k] = rel;
     d.delv[k] = rel - d.v[k];
-    // CalcElemCharacteristicLength (:1821-1862): 4V / sqrt(max AreaFace)
-    d.arealg[k] = to_double(df_scale(vol64, 0.25f) * df_rsqrt(max_face_cross2_64(M1, M2, M3, M4, M5, M6, X)));
     if (rel <= 0.0) flag_error(sc, ERR_K3_VNEW, k);
+
+    // CalcElemCharacteristicLength (:1821-1862): 4V / sqrt(max AreaFace)
+    {
+        // a = M3xM4, -b = M5xM2, c = M6xM1; Y1 = b - a, Y2 = c + a, Y3 = c + b
+        const V2x3 bc = cross2(d56, swapped(M.m12));
+        const V1x3 a = cross1(M.m3, M.m4), nb = half_x(bc), c = half_y(bc);
+        const df64 f = fmax(fmax(face_pair_max(X.n1, sum1(nb, a)), face_pair_max(X.n2, sum1(c, a))),
+                            face_pair_max(X.n3, sum1(c, minus(nb))));
+        reinterpret_cast<float2 *>(d.arealg)[k] = as_float2(df_scale(vol64, 0.25f) * df_rsqrt(f));
+    }
+
+    V2x3 V12;   // velocity modes (V1, V2) and V3
+    V1x3 V3v;
+    {
+        double c[8];
+        LinearPacks u;
+        gather8(d.xd, nl, c);
+        u = walsh_linear_packs(corners_of(c));
+        V12.x = u.m12;
+        V3v.x = u.m3;
+        gather8(d.yd, nl, c);
+        u = walsh_linear_packs(corners_of(c));
+        V12.y = u.m12;
+        V3v.y = u.m3;
+        gather8(d.zd, nl, c);
+        u = walsh_linear_packs(corners_of(c));
+        V12.z = u.m12;
+        V3v.z = u.m3;
+    }
+    const V2x3n V21 = swapped(both(V12));
 
     // CalcMonotonicQGradientsForElems (:2034-2180): the logical differences
     // are M/4, so each cross product is (M x M')/16 and each velocity
-    // difference Mv/4
+    // difference Mv/4; volo vnew is the volume.  eta and xi in the halves of
+    // a pair (M3xM1, M3xM2), zeta beside them.  Kept as pairs (Dom::delv_xi).
     {
         const df64 ptiny(1.e-36);
-        const df64 vol = to_df(d.volo[k]) * rel_df;
+        const df64 vol = df_scale(vol64, 1.f / 64.f);
         // (1/16) (1/4) / (vol + ptiny)
         const df64 vscale = df_rcp(df_scale(vol + ptiny, 64.f));
-        const V3<df64> &Az = X.c12, &Ax = X.c23, &Ae = X.c31;
-        d.delx_zeta[k] = to_double(vol * df_rsqrt(df_scale(dot3(Az, Az), 0.00390625f) + ptiny));
-        d.delv_zeta[k] = to_double(vscale * dot3(Az, V3v));
-        d.delx_xi[k] = to_double(vol * df_rsqrt(df_scale(dot3(Ax, Ax), 0.00390625f) + ptiny));
-        d.delv_xi[k] = to_double(vscale * dot3(Ax, V1));
-        d.delx_eta[k] = to_double(vol * df_rsqrt(df_scale(dot3(Ae, Ae), 0.00390625f) + ptiny));
-        d.delv_eta[k] = to_double(vscale * dot3(Ae, V2));
+        const df2 nn = dot2(X.q2, both(X.q2)).value();
+        const df2 dv = dot2(X.q2, V21).value();
+        const V1x3 c12 = half_x(X.q3);
+        auto delx = [&](df64 n) { return as_float2(vol * df_rsqrt(df_scale(n, 0.00390625f) + ptiny)); };
+        auto at = [&](double *f) { return reinterpret_cast<float2 *>(f) + k; };
+        *at(d.delx_eta) = delx(df2_x(nn));
+        *at(d.delx_xi) = delx(df2_y(nn));
+        *at(d.delx_zeta) = delx(dot1(c12, c12).value());
+        *at(d.delv_eta) = as_float2(vscale * df2_x(dv));
+        *at(d.delv_xi) = as_float2(vscale * -df2_y(dv));   // M2xM3 = -M3xM2
+        *at(d.delv_zeta) = as_float2(vscale * dot1(c12, V3v).value());
     }
 
-    // CalcKinematicsForElems, strain-rate part (:1975-2020)
-    d.vdov[k] = to_double(strain_rate(M1, M2, M3, V1, V2, V3v, to_df(0.5 * sc->deltatime),
-                                      [](df64 a, df64 b) { return df_div(a, b); }));
+    // CalcKinematicsForElems, strain-rate part (:1975-2020): the half-step
+    // Jacobian's columns (M - dt/2 V)/8, the rate their cofactors . V over
+    // their determinant (strain_rate, hexmodes.cuh); cof = (CxA, CxB)
+    {
+        const df64 dt2 = to_df(0.5 * sc->deltatime);
+        const df2n nd = df2_both(df2_dup(dt2));
+        auto back2 = [&](df2 m, df2 v) { return Dot2(v, df2_minus(nd)).plus(m).value(); };
+        auto back1 = [&](df64 m, df64 v) { return Dot1(v, -dt2).plus(Dot1(m.hi, m.lo)).value(); };
+        const V2x3 AB{back2(d12.x, V12.x), back2(d12.y, V12.y), back2(d12.z, V12.z)};
+        const V1x3 C{back1(M.m3.x, V3v.x), back1(M.m3.y, V3v.y), back1(M.m3.z, V3v.z)};
+        const V2x3 cof = cross2(dup3(C), both(AB));
+        const V1x3 cze = cross1_even(half_x(AB), half_y(AB));
+        const df64 num = dot1(cze, V3v).plus(difference(dot2(cof, V21))).value();
+        reinterpret_cast<float2 *>(d.vdov)[k] = as_float2(df_div(num, dot1(C, cze).value()));
+    }
 }
 
 __global__ void __launch_bounds__(kKinBlockFactor * kBlockElem, 2) k_elem_kinematics_df(const __grid_constant__ Dom d)
@@ -315,22 +432,17 @@ __global__ void __launch_bounds__(kKinBlockFactor * kBlockElem, 2) k_elem_kinema
 // taken as +-2^100.  That changes no outcome: a ratio beyond it is never the
 // minimum unless both are, and then the result is max_slope either way; a
 // negative one makes the result 0 either way.
-__device__ __forceinline__ df64 limiter_phi_df(const double *__restrict__ delv, int i, int bm, int bp,
-                                               int m_symm, int m_free, int p_symm, int p_free, int lm, int lp,
-                                               df64 limiter, df64 max_slope)
+__device__ __forceinline__ df64 limiter_phi_df(const float2 *__restrict__ delv, df64 own, int bm, int bp,
+                                               int m_symm, int p_symm, int lm, int lp, df64 limiter, df64 max_slope)
 {
-    const double own = delv[i];
-    const df64 norm = df_rcp(to_df(own) + df64(1.e-36));
-    double dm = 0.0, dp = 0.0;
-    if (bm == 0) dm = delv[lm];
+    const df64 norm = df_rcp(own + df64(1.e-36));
+    df64 dm(0.f, 0.f), dp(0.f, 0.f);   // 0 beyond a free face
+    if (bm == 0) dm = as_df(delv[lm]);
     else if (bm == m_symm) dm = own;
-    if (bp == 0) dp = delv[lp];
+    if (bp == 0) dp = as_df(delv[lp]);
     else if (bp == p_symm) dp = own;
-    (void)m_free;
-    (void)p_free;
     const float big = 1.2676506e30f;   // 2^100
-    auto ratio = [&](double x) {
-        const df64 a = to_df(x);
+    auto ratio = [&](df64 a) {
         if (fabsf(a.hi) * fabsf(norm.hi) > big)   // may be inf: still > big
             return (a.hi < 0.f) != (norm.hi < 0.f) ? df64(-big, 0.f) : df64(big, 0.f);
         return a * norm;
@@ -357,25 +469,27 @@ __device__ __forceinline__ void elem_material_df(const Dom &d, int k, DevScalars
     const int bc = __ldg(d.elem_bc + k);
     const FaceNeighbours nb = face_neighbours(d, sc, k);
     const df64 lim = to_df(P.monoq_limiter_mult), maxs = to_df(P.monoq_max_slope);
-    const df64 phixi = limiter_phi_df(d.delv_xi, k, bc & BC_XI_M, bc & BC_XI_P, BC_XI_M_SYMM, BC_XI_M_FREE,
-                                      BC_XI_P_SYMM, BC_XI_P_FREE, nb.xim, nb.xip, lim, maxs);
-    const df64 phieta = limiter_phi_df(d.delv_eta, k, bc & BC_ETA_M, bc & BC_ETA_P, BC_ETA_M_SYMM, BC_ETA_M_FREE,
-                                       BC_ETA_P_SYMM, BC_ETA_P_FREE, nb.etam, nb.etap, lim,
-                                       maxs);
-    const df64 phizeta = limiter_phi_df(d.delv_zeta, k, bc & BC_ZETA_M, bc & BC_ZETA_P, BC_ZETA_M_SYMM,
-                                        BC_ZETA_M_FREE, BC_ZETA_P_SYMM, BC_ZETA_P_FREE, nb.zetam,
-                                        nb.zetap, lim, maxs);
-    const double vnew = d.vnew[k], vdov = d.vdov[k];
+    auto pairs = [](const double *f) { return reinterpret_cast<const float2 *>(f); };
+    const float2 *dv_xi = pairs(d.delv_xi), *dv_eta = pairs(d.delv_eta), *dv_zeta = pairs(d.delv_zeta);
+    const df64 own_xi = as_df(dv_xi[k]), own_eta = as_df(dv_eta[k]), own_zeta = as_df(dv_zeta[k]);
+    const df64 phixi = limiter_phi_df(dv_xi, own_xi, bc & BC_XI_M, bc & BC_XI_P, BC_XI_M_SYMM, BC_XI_P_SYMM, nb.xim,
+                                      nb.xip, lim, maxs);
+    const df64 phieta = limiter_phi_df(dv_eta, own_eta, bc & BC_ETA_M, bc & BC_ETA_P, BC_ETA_M_SYMM, BC_ETA_P_SYMM,
+                                       nb.etam, nb.etap, lim, maxs);
+    const df64 phizeta = limiter_phi_df(dv_zeta, own_zeta, bc & BC_ZETA_M, bc & BC_ZETA_P, BC_ZETA_M_SYMM,
+                                        BC_ZETA_P_SYMM, nb.zetam, nb.zetap, lim, maxs);
+    const double vnew = d.vnew[k];
+    const df64 vdov = as_df(pairs(d.vdov)[k]);
     df64 qlin(0.f, 0.f), qquad(0.f, 0.f);
-    if (!gt(vdov, 0.)) {
+    if (!(vdov.hi > 0.f)) {
         // the products delv * delx; a positive one contributes nothing
-        auto prod = [](double dv, double dx) {
-            const df64 p = to_df(dv) * to_df(dx);
+        auto prod = [](df64 dv, df64 dx) {
+            const df64 p = dv * dx;
             return p.hi > 0.f ? df64(0.f, 0.f) : p;
         };
-        const df64 dxi = prod(d.delv_xi[k], d.delx_xi[k]);
-        const df64 deta = prod(d.delv_eta[k], d.delx_eta[k]);
-        const df64 dzeta = prod(d.delv_zeta[k], d.delx_zeta[k]);
+        const df64 dxi = prod(own_xi, as_df(pairs(d.delx_xi)[k]));
+        const df64 deta = prod(own_eta, as_df(pairs(d.delx_eta)[k]));
+        const df64 dzeta = prod(own_zeta, as_df(pairs(d.delx_zeta)[k]));
         const df64 rho = df_div(to_df(d.elem_mass[k]), to_df(d.volo[k]) * to_df(vnew));
         const df64 one(1.f, 0.f);
         const df64 lin = (dxi * (one - phixi) + deta * (one - phieta)) + dzeta * (one - phizeta);
@@ -389,7 +503,8 @@ __device__ __forceinline__ void elem_material_df(const Dom &d, int k, DevScalars
         d.qq[k] = to_double(qquad);
     }
     const double ssn = material_update_df<SeriesFn>(d, k, sc, vnew, qlin, qquad, d.reps ? __ldg(d.reps + k) : 1);
-    if (kConstraints) constraint_keys_df<SeriesFn>(ssn, vdov, d.arealg[k], P, kc, kh);
+    if (kConstraints)
+        constraint_keys_df<SeriesFn>(to_df(ssn), vdov, as_df(pairs(d.arealg)[k]), vdov.hi != 0.f, vdov.hi < 0.f, P, kc, kh);
 }
 
 // Eight blocks per SM (64 registers, ~40 bytes spilled; 80 registers at six

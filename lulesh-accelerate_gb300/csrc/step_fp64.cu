@@ -416,7 +416,12 @@ __global__ void __launch_bounds__(kBlockElem) k_time_constraints(const __grid_co
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     unsigned long long kc = ~0ULL, kh = ~0ULL;
     if (k < d.ne && !skip_step(d)) {
-        if (d.df == kArithDF64) constraint_keys_df<SeriesFn>(d.ss[k], d.vdov[k], d.arealg[k], d.prm, kc, kh);
+        if (d.df == kArithDF64) {
+            // vdov and arealg are pairs there (Dom::vdov)
+            const df64 v = as_df(reinterpret_cast<const float2 *>(d.vdov)[k]);
+            const df64 a = as_df(reinterpret_cast<const float2 *>(d.arealg)[k]);
+            constraint_keys_df<SeriesFn>(to_df(d.ss[k]), v, a, v.hi != 0.f, v.hi < 0.f, d.prm, kc, kh);
+        }
         else constraint_keys(d.ss[k], d.vdov[k], d.arealg[k], d.prm, kc, kh);
     }
     block_min_publish(kc, kh, d.sc);

@@ -541,7 +541,9 @@ __device__ __forceinline__ void elem_material_split(const Dom &d, int k, DevScal
         // the energy accumulated in FP64 (eos_df.cuh)
         const double ssn = material_update_df<NewtonFn>(d, k, sc, vnew, df64(qlin, 0.f), df64(qquad, 0.f),
                                               d.reps ? __ldg(d.reps + k) : 1);
-        if (kConstraints) constraint_keys_df<NewtonFn>(ssn, vdov, d.arealg[k], P, kc, kh);
+        if (kConstraints)
+            constraint_keys_df<NewtonFn>(to_df(ssn), to_df(vdov), to_df(d.arealg[k]), iabs(vdov) != 0ULL, lt(vdov, 0.), P,
+                                         kc, kh);
     }
 }
 
