@@ -140,11 +140,25 @@ __device__ __forceinline__ float d2f(double v)
 // float -> double, exact (FP32 subnormals become zeros).
 __device__ __forceinline__ double f2d(float f) { return df_f2d(f); }
 
+// A node's state and constants, loaded before anything of the node is
+// stored: the compiler keeps a load behind every store that might alias it,
+// and loads taken between the stores (velocity, position, velocity, ...) make
+// six memory latencies of one.
+struct NodeState {
+    double x, y, z, xd, yd, zd, m;   // m: the mass or its reciprocal
+    unsigned bc;
+};
+__device__ __forceinline__ NodeState load_node(const Dom &d, int n)
+{
+    return {d.x[n], d.y[n], d.z[n], d.xd[n], d.yd[n], d.zd[n], __ldg((d.inv_mass ? d.inv_mass : d.nodal_mass) + n),
+            __ldg(d.node_bc + n)};
+}
+
 // The node update after the corner gather: CalcAccelerationForNodes, the
 // symmetry-plane conditions, CalcVelocityForNodes and CalcPositionForNodes
 // (LULESH-OMP.cc:1613-1683) for node n with nodal force (fx, fy, fz).
-__device__ __forceinline__ void node_integrate(const Dom &d, int n, const DevScalars *sc, double fx, double fy,
-                                               double fz)
+__device__ __forceinline__ void node_integrate(const Dom &d, int n, const DevScalars *sc, NodeState s, double fx,
+                                               double fy, double fz)
 {
     if (d.keep & 1) {
         d.fx[n] = fx;
@@ -152,24 +166,24 @@ __device__ __forceinline__ void node_integrate(const Dom &d, int n, const DevSca
         d.fz[n] = fz;
     }
     const double dt = sc->deltatime, u_cut = d.prm.u_cut;
-    const unsigned bc = __ldg(d.node_bc + n);
-    double ax, ay, az;
-    if (d.inv_mass) {
-        // f * (1/m) with the reciprocal precomputed: within an ulp of f / m
-        const double im = __ldg(d.inv_mass + n);
-        ax = (bc & 1) ? 0.0 : fx * im;
-        ay = (bc & 2) ? 0.0 : fy * im;
-        az = (bc & 4) ? 0.0 : fz * im;
-    } else {
-        const double m = __ldg(d.nodal_mass + n);
-        ax = (bc & 1) ? 0.0 : fx / m;
-        ay = (bc & 2) ? 0.0 : fy / m;
-        az = (bc & 4) ? 0.0 : fz / m;
-    }
-    double t;
-    t = d.xd[n] + ax * dt; if (abs_lt(t, u_cut)) t = 0.0; d.xd[n] = t; d.x[n] += t * dt;
-    t = d.yd[n] + ay * dt; if (abs_lt(t, u_cut)) t = 0.0; d.yd[n] = t; d.y[n] += t * dt;
-    t = d.zd[n] + az * dt; if (abs_lt(t, u_cut)) t = 0.0; d.zd[n] = t; d.z[n] += t * dt;
+    // f * (1/m) with the reciprocal precomputed (within an ulp of f / m), or
+    // f / m where the caller's masses are all there is
+    const bool reciprocal = d.inv_mass != nullptr;
+    const double ax = (s.bc & 1) ? 0.0 : (reciprocal ? fx * s.m : fx / s.m);
+    const double ay = (s.bc & 2) ? 0.0 : (reciprocal ? fy * s.m : fy / s.m);
+    const double az = (s.bc & 4) ? 0.0 : (reciprocal ? fz * s.m : fz / s.m);
+    s.xd += ax * dt;
+    s.yd += ay * dt;
+    s.zd += az * dt;
+    if (abs_lt(s.xd, u_cut)) s.xd = 0.0;
+    if (abs_lt(s.yd, u_cut)) s.yd = 0.0;
+    if (abs_lt(s.zd, u_cut)) s.zd = 0.0;
+    d.xd[n] = s.xd;
+    d.yd[n] = s.yd;
+    d.zd[n] = s.zd;
+    d.x[n] = s.x + s.xd * dt;
+    d.y[n] = s.y + s.yd * dt;
+    d.z[n] = s.z + s.zd * dt;
 }
 
 // The six face neighbours of element k (lxim, lxip, letam, letap, lzetam,
@@ -344,17 +358,27 @@ __device__ __forceinline__ double q_term(double pbvc, double e, double vv, doubl
 // rep from :2410-2424): the results are those of one evaluation, and the
 // empty asm statements keep the compiler from merging or dropping the
 // repeated evaluations.
+// An element's state before the material update, loaded with the limiter's
+// inputs (ahead of the error flags and results, which the compiler would
+// otherwise keep the loads behind).
+struct MaterialIn {
+    double q, v, delv, e, p;
+};
+__device__ __forceinline__ MaterialIn load_material(const Dom &d, int k)
+{
+    return {d.q[k], d.v[k], d.delv[k], d.e[k], d.p[k]};
+}
 __device__ __forceinline__ void opaque(double &v) { asm volatile("" : "+d"(v)); }
 __device__ __forceinline__ void consume(double v) { asm volatile("" ::"d"(v)); }
 
 template <bool kF32Q = false>
-__device__ __forceinline__ double material_update(const Dom &d, int k, DevScalars *sc, double vnew,
+__device__ __forceinline__ double material_update(const Dom &d, int k, DevScalars *sc, const MaterialIn &in, double vnew,
                                                   double qlin, double qquad, int rep = 1)
 {
     const lulesh_params &P = d.prm;
     if (rep < 1) rep = 1;
     // CalcQForElems qstop test on the old q (:2369-2381)
-    const double q_old_in = d.q[k];
+    const double q_old_in = in.q;
     if (q_old_in > P.qstop) flag_error(sc, ERR_K3_QSTOP, k);
 
     // ApplyMaterialPropertiesForElems (:2703-2761)
@@ -365,14 +389,13 @@ __device__ __forceinline__ double material_update(const Dom &d, int k, DevScalar
     if (has_vmin && lt(vnewc_in, eosvmin)) vnewc_in = eosvmin;
     if (has_vmax && gt(vnewc_in, eosvmax)) vnewc_in = eosvmax;
     const double qlin_in = qlin, qquad_in = qquad;
-    const double v_old = d.v[k];
-    double vc = v_old;
+    double vc = in.v;
     if (has_vmin && lt(vc, eosvmin)) vc = eosvmin;
     if (has_vmax && gt(vc, eosvmax)) vc = eosvmax;
     if (vc <= 0.) flag_error(sc, ERR_K3_MATV, k);
 
     // EvalEOSForElems + CalcEnergyForElems (:2415-2701); work == 0
-    const double delvc_in = d.delv[k], e_old_in = d.e[k], p_old_in = d.p[k];
+    const double delvc_in = in.delv, e_old_in = in.e, p_old_in = in.p;
     const double rho0 = P.refdens;
     const bool unit_rho0 = ikey(rho0) == ikey(1.0);
     const double pbvc = 2.0 / 3.0;

@@ -75,17 +75,17 @@ __device__ __forceinline__ f2 f2_neg(f2 a) { return a ^ 0x8000000080000000ULL; }
 struct df2 {
     f2 hi, lo;
 };
-// a value with its negative
+// a value with its high word's negative
 struct df2n {
-    f2 hi, lo, nhi, nlo;
+    f2 hi, lo, nhi;
 };
 
 __device__ __forceinline__ df2 df2_pack(df64 x, df64 y) { return {f2_pack(x.hi, y.hi), f2_pack(x.lo, y.lo)}; }
 __device__ __forceinline__ df2 df2_dup(df64 x) { return df2_pack(x, x); }
 __device__ __forceinline__ df64 df2_x(df2 a) { return {f2_x(a.hi), f2_x(a.lo)}; }
 __device__ __forceinline__ df64 df2_y(df2 a) { return {f2_y(a.hi), f2_y(a.lo)}; }
-__device__ __forceinline__ df2n df2_both(df2 a) { return {a.hi, a.lo, f2_neg(a.hi), f2_neg(a.lo)}; }
-__device__ __forceinline__ df2n df2_minus(df2n a) { return {a.nhi, a.nlo, a.hi, a.lo}; }
+__device__ __forceinline__ df2n df2_both(df2 a) { return {a.hi, a.lo, f2_neg(a.hi)}; }
+__device__ __forceinline__ df2 df2_first(df2n a) { return {a.hi, a.lo}; }
 
 __device__ __forceinline__ df2 f2_two_sum(f2 a, f2 b)
 {
@@ -126,44 +126,58 @@ __device__ __forceinline__ df64 df_tidy(df64 a) { return fast_two_sum(a.hi, a.lo
 
 // Sums of products (the compensated dot product of Ogita, Rump and Oishi,
 // 2005, on pairs) in both halves: each product's high word joins the running
-// high word through two_sum and every low-order term collects, negated, in
-// one word; 12 operations per term, renormalised once at the end.  The
-// low-order words are added before the rounding error of the high words'
-// sum, so that two terms, or two partial sums, give the same bits in either
-// order.
+// high word through two_sum and every low-order term collects in one word;
+// 12 operations per term, renormalised once at the end.  The low-order words
+// are added before the rounding error of the high words' sum, so that two
+// terms, or two partial sums, give the same bits in either order.  The high
+// word is held negated: -a b and its exact remainder a b - (-(-a b)) then
+// need no more than the factor's negative, once for all of its products.
 struct Dot2 {
-    f2 s, e;   // the sum is s - e
+    f2 ns, e;   // the sum is e - ns
     // a b, the first term
     __device__ __forceinline__ Dot2(df2 a, df2n b)
     {
-        s = f2_mul(a.hi, b.hi);
-        e = f2_fma(a.hi, b.nlo, f2_fma(a.lo, b.nhi, f2_fma(a.hi, b.nhi, s)));
+        ns = f2_mul(a.hi, b.nhi);
+        e = f2_fma(a.hi, b.lo, f2_fma(a.lo, b.hi, f2_fma(a.hi, b.hi, ns)));
     }
-    __device__ __forceinline__ Dot2(f2 hi, f2 minus_lo) : s(hi), e(minus_lo) {}
+    __device__ __forceinline__ Dot2(f2 minus_hi, f2 lo) : ns(minus_hi), e(lo) {}
     __device__ __forceinline__ Dot2 &plus(Dot2 t)
     {
-        const df2 q = f2_two_sum(s, t.s);
-        s = q.hi;
+        const df2 q = f2_two_sum(ns, t.ns);
+        ns = q.hi;
         e = f2_sub(f2_add(e, t.e), q.lo);
         return *this;
     }
-    __device__ __forceinline__ Dot2 &plus(df2 c)
+    __device__ __forceinline__ Dot2 &minus(Dot2 t)
     {
-        const df2 q = f2_two_sum(s, c.hi);
-        s = q.hi;
+        const df2 q = f2_two_diff(ns, t.ns);
+        ns = q.hi;
+        e = f2_sub(f2_sub(e, t.e), q.lo);
+        return *this;
+    }
+    __device__ __forceinline__ Dot2 &minus(df2 c)
+    {
+        const df2 q = f2_two_sum(ns, c.hi);
+        ns = q.hi;
         e = f2_sub(f2_sub(e, c.lo), q.lo);
         return *this;
     }
     __device__ __forceinline__ Dot2 &add(df2 a, df2n b) { return plus(Dot2(a, b)); }
-    __device__ __forceinline__ Dot2 &sub(df2 a, df2n b) { return add(a, df2_minus(b)); }
-    // renormalised for |s| >= |e|; when the high words cancel further than
-    // that, the error stays at 2^-24 |e|, the sum's own
+    __device__ __forceinline__ Dot2 &sub(df2 a, df2n b) { return minus(Dot2(a, b)); }
+    // the sum and its negative, renormalised for |ns| >= |e|; when the high
+    // words cancel further than that, the error stays at 2^-24 |e|, the
+    // sum's own
     __device__ __forceinline__ df2 value() const
     {
-        const f2 h = f2_sub(s, e);
-        return {h, f2_sub(f2_sub(s, h), e)};
+        const f2 h = f2_sub(e, ns);
+        return {h, f2_sub(e, f2_add(h, ns))};
     }
-    __device__ __forceinline__ df2 raw() const { return {s, f2_neg(e)}; }
+    __device__ __forceinline__ df2 negative() const
+    {
+        const f2 h = f2_sub(ns, e);
+        return {h, f2_sub(f2_sub(ns, h), e)};
+    }
+    __device__ __forceinline__ df2 raw_negative() const { return {ns, f2_neg(e)}; }
 };
 
 // a times b, renormalised
@@ -191,8 +205,8 @@ struct Dot1 {
     __device__ __forceinline__ df64 value() const { return fast_two_sum(s, e); }
 };
 // the two halves of a sum
-__device__ __forceinline__ Dot1 dot_x(const Dot2 &d) { return {f2_x(d.s), -f2_x(d.e)}; }
-__device__ __forceinline__ Dot1 dot_y(const Dot2 &d) { return {f2_y(d.s), -f2_y(d.e)}; }
+__device__ __forceinline__ Dot1 dot_x(const Dot2 &d) { return {-f2_x(d.ns), f2_x(d.e)}; }
+__device__ __forceinline__ Dot1 dot_y(const Dot2 &d) { return {-f2_y(d.ns), f2_y(d.e)}; }
 __device__ __forceinline__ Dot1 minus(const Dot1 &d) { return {-d.s, -d.e}; }
 __device__ __forceinline__ Dot1 joined(const Dot2 &d) { return dot_x(d).plus(dot_y(d)); }
 __device__ __forceinline__ Dot1 difference(const Dot2 &d) { return dot_x(d).plus(minus(dot_y(d))); }
@@ -221,7 +235,7 @@ __device__ __forceinline__ V2x3 dup3(const V1x3 &a) { return {df2_dup(a.x), df2_
 __device__ __forceinline__ V2x3n swapped(const V2x3n &a)
 {
     auto sw = [](f2 v) { return f2_pack(f2_y(v), f2_x(v)); };
-    auto comp = [&](const df2n &v) { return df2n{sw(v.hi), sw(v.lo), sw(v.nhi), sw(v.nlo)}; };
+    auto comp = [&](const df2n &v) { return df2n{sw(v.hi), sw(v.lo), sw(v.nhi)}; };
     return {comp(a.x), comp(a.y), comp(a.z)};
 }
 
@@ -241,8 +255,8 @@ __device__ __forceinline__ V1x3 cross1(const V1x3 &a, const V1x3 &b)
 }
 __device__ __forceinline__ Dot2 even_product(df2 u, df2n v)
 {
-    const f2 p = f2_mul(u.hi, v.hi);
-    return {p, f2_add(f2_fma(u.hi, v.nhi, p), f2_add(f2_mul(u.hi, v.nlo), f2_mul(u.lo, v.nhi)))};
+    const f2 np = f2_mul(u.hi, v.nhi);
+    return {np, f2_add(f2_fma(u.hi, v.hi, np), f2_add(f2_mul(u.hi, v.lo), f2_mul(u.lo, v.hi)))};
 }
 __device__ __forceinline__ Dot1 even_product(df64 u, df64 v)
 {
@@ -251,7 +265,7 @@ __device__ __forceinline__ Dot1 even_product(df64 u, df64 v)
 }
 __device__ __forceinline__ V2x3 cross2_even(const V2x3 &a, const V2x3n &b)
 {
-    auto minor = [](df2 u, df2n v, df2 w, df2n x) { return even_product(u, v).plus(even_product(w, df2_minus(x))).value(); };
+    auto minor = [](df2 u, df2n v, df2 w, df2n x) { return even_product(u, v).minus(even_product(w, x)).value(); };
     return {minor(a.y, b.z, a.z, b.y), minor(a.z, b.x, a.x, b.z), minor(a.x, b.y, a.y, b.x)};
 }
 __device__ __forceinline__ V1x3 cross1_even(const V1x3 &a, const V1x3 &b)

@@ -52,12 +52,12 @@ __device__ __forceinline__ void opaque_df(df64 &v) { asm volatile("" : "+f"(v.hi
 // the same quantities as the FP64 kernel, in whichever form they are held.
 // Fn: the reciprocal and root functions (SeriesFn, NewtonFn).
 template <class Fn>
-__device__ __forceinline__ double material_update_df(const Dom &d, int k, DevScalars *sc, double vnew,
+__device__ __forceinline__ double material_update_df(const Dom &d, int k, DevScalars *sc, const MaterialIn &in, double vnew,
                                                      df64 qlin_in, df64 qquad_in, int rep)
 {
     const lulesh_params &P = d.prm;
     if (rep < 1) rep = 1;
-    const double q_old_in = d.q[k];
+    const double q_old_in = in.q;
     if (q_old_in > P.qstop) flag_error(sc, ERR_K3_QSTOP, k);
 
     const double eosvmin = P.eosvmin, eosvmax = P.eosvmax;
@@ -65,12 +65,12 @@ __device__ __forceinline__ double material_update_df(const Dom &d, int k, DevSca
     const bool has_vmin = iabs(eosvmin) != 0ULL, has_vmax = iabs(eosvmax) != 0ULL;
     if (has_vmin && lt(vnewc_in, eosvmin)) vnewc_in = eosvmin;
     if (has_vmax && gt(vnewc_in, eosvmax)) vnewc_in = eosvmax;
-    double vc = d.v[k];
+    double vc = in.v;
     if (has_vmin && lt(vc, eosvmin)) vc = eosvmin;
     if (has_vmax && gt(vc, eosvmax)) vc = eosvmax;
     if (vc <= 0.) flag_error(sc, ERR_K3_MATV, k);
 
-    const double delvc_in = d.delv[k], e_old_in = d.e[k], p_old_in = d.p[k];
+    const double delvc_in = in.delv, e_old_in = in.e, p_old_in = in.p;
     const double rho0 = P.refdens;
     const bool unit_rho0 = ikey(rho0) == ikey(1.0);
     const double emin = P.emin, e_cut = P.e_cut;

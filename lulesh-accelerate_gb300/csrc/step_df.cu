@@ -203,20 +203,20 @@ __device__ __forceinline__ void elem_force_df(const Dom &d, int k, DevScalars *s
             const df2n Gx = modes_dot(W12.x, W56.x, W34.x);
             const df2n Gy = modes_dot(W12.y, W56.y, W34.y);
             const df2n Gz = modes_dot(W12.z, W56.z, W34.z);
-            // c - v.g
-            auto less = [](df2 c, const V2x3 &v, const df2n &gx, const df2n &gy, const df2n &gz) {
-                return Dot2(v.x, df2_minus(gx)).sub(v.y, gy).sub(v.z, gz).plus(c);
+            // v.g - c
+            auto excess = [](df2 c, const V2x3 &v, const df2n &gx, const df2n &gy, const df2n &gz) {
+                return Dot2(v.x, gx).add(v.y, gy).add(v.z, gz).minus(c);
             };
-            const df2 h56 = df2_mul(less(u.m56, H56, Gx, Gy, Gz).value(), coef);
-            const df2 h47 = df2_mul(less(df2_pack(u.m4, df2_x(u.m73)), H47, Gx, Gy, Gz).value(), coef);
+            const df2 h56 = df2_mul(excess(u.m56, H56, Gx, Gy, Gz).negative(), coef);
+            const df2 h47 = df2_mul(excess(df2_pack(u.m4, df2_x(u.m73)), H47, Gx, Gy, Gz).negative(), coef);
             const df2n h56n = df2_both(h56), h47n = df2_both(h47);
             auto shape_dot = [&](df2 a, df2 b) {
                 return df2_both(df2_dup(joined(Dot2(a, h56n)).plus(joined(Dot2(b, h47n))).value()));
             };
             const df2n Kx = shape_dot(H56.x, H47.x), Ky = shape_dot(H56.y, H47.y), Kz = shape_dot(H56.z, H47.z);
-            F12 = less(df2_pack(y1, y2), W12, Kx, Ky, Kz).raw();
-            F56 = less(h56, W56, Kx, Ky, Kz).raw();
-            const df2 F34 = less(df2_pack(y3, df2_x(h47)), W34, Kx, Ky, Kz).raw();
+            F12 = excess(df2_pack(y1, y2), W12, Kx, Ky, Kz).raw_negative();
+            F56 = excess(h56, W56, Kx, Ky, Kz).raw_negative();
+            const df2 F34 = excess(df2_pack(y3, df2_x(h47)), W34, Kx, Ky, Kz).raw_negative();
             F3 = df2_x(F34);
             F4 = df2_y(F34);
             F7 = df2_y(h47);
@@ -259,6 +259,7 @@ __device__ __forceinline__ void node_update_df(const Dom &d, int n, const DevSca
 {
     const float2 *const fc[3] = {reinterpret_cast<const float2 *>(d.fcx), reinterpret_cast<const float2 *>(d.fcy),
                                  reinterpret_cast<const float2 *>(d.fcz)};
+    const NodeState state = load_node(d, n);
     df64 f[3] = {df64(0.f, 0.f), df64(0.f, 0.f), df64(0.f, 0.f)};
     const int s = d.s > 0 ? d.s : sc->edge;
     if (s > 0) {
@@ -279,10 +280,14 @@ __device__ __forceinline__ void node_update_df(const Dom &d, int n, const DevSca
             for (int i = 0; i < 3; ++i) f[i] = first ? as_df(fc[i][c]) : f[i] + as_df(fc[i][c]);
         });
     }
-    node_integrate(d, n, sc, to_double(f[0]), to_double(f[1]), to_double(f[2]));
+    node_integrate(d, n, sc, state, to_double(f[0]), to_double(f[1]), to_double(f[2]));
 }
 
-__global__ void __launch_bounds__(kBlockNode) k_node_update_df(const __grid_constant__ Dom d)
+// Twelve blocks per SM (40 registers, 24 bytes spilled): the gather waits on
+// memory, and the early loads of load_node (0.387 -> 0.379 ms at s=192) cost
+// registers that the compiler would otherwise take 54 of; 0.355 ms at the
+// cap, 0.380 at 32 registers.
+__global__ void __launch_bounds__(kBlockNode, 12) k_node_update_df(const __grid_constant__ Dom d)
 {
     if (skip_step(d)) return;
     const int n = blockIdx.x * blockDim.x + threadIdx.x;
@@ -399,7 +404,7 @@ __device__ __forceinline__ void elem_kinematics_df(const Dom &d, int k, DevScala
     {
         const df64 dt2 = to_df(0.5 * sc->deltatime);
         const df2n nd = df2_both(df2_dup(dt2));
-        auto back2 = [&](df2 m, df2 v) { return Dot2(v, df2_minus(nd)).plus(m).value(); };
+        auto back2 = [&](df2 m, df2 v) { return Dot2(v, nd).minus(m).negative(); };
         auto back1 = [&](df64 m, df64 v) { return Dot1(v, -dt2).plus(Dot1(m.hi, m.lo)).value(); };
         const V2x3 AB{back2(d12.x, V12.x), back2(d12.y, V12.y), back2(d12.z, V12.z)};
         const V1x3 C{back1(M.m3.x, V3v.x), back1(M.m3.y, V3v.y), back1(M.m3.z, V3v.z)};
@@ -467,9 +472,12 @@ __device__ __forceinline__ void elem_material_df(const Dom &d, int k, DevScalars
 {
     const lulesh_params &P = d.prm;
     const int bc = __ldg(d.elem_bc + k);
+    const MaterialIn in = load_material(d, k);
+    const double vnew = d.vnew[k], mass = __ldg(d.elem_mass + k), volo = __ldg(d.volo + k);
+    auto pairs = [](const double *f) { return reinterpret_cast<const float2 *>(f); };
+    const df64 vdov = as_df(pairs(d.vdov)[k]), arealg = as_df(pairs(d.arealg)[k]);
     const FaceNeighbours nb = face_neighbours(d, sc, k);
     const df64 lim = to_df(P.monoq_limiter_mult), maxs = to_df(P.monoq_max_slope);
-    auto pairs = [](const double *f) { return reinterpret_cast<const float2 *>(f); };
     const float2 *dv_xi = pairs(d.delv_xi), *dv_eta = pairs(d.delv_eta), *dv_zeta = pairs(d.delv_zeta);
     const df64 own_xi = as_df(dv_xi[k]), own_eta = as_df(dv_eta[k]), own_zeta = as_df(dv_zeta[k]);
     const df64 phixi = limiter_phi_df(dv_xi, own_xi, bc & BC_XI_M, bc & BC_XI_P, BC_XI_M_SYMM, BC_XI_P_SYMM, nb.xim,
@@ -478,8 +486,6 @@ __device__ __forceinline__ void elem_material_df(const Dom &d, int k, DevScalars
                                        nb.etam, nb.etap, lim, maxs);
     const df64 phizeta = limiter_phi_df(dv_zeta, own_zeta, bc & BC_ZETA_M, bc & BC_ZETA_P, BC_ZETA_M_SYMM,
                                         BC_ZETA_P_SYMM, nb.zetam, nb.zetap, lim, maxs);
-    const double vnew = d.vnew[k];
-    const df64 vdov = as_df(pairs(d.vdov)[k]);
     df64 qlin(0.f, 0.f), qquad(0.f, 0.f);
     if (!(vdov.hi > 0.f)) {
         // the products delv * delx; a positive one contributes nothing
@@ -490,7 +496,7 @@ __device__ __forceinline__ void elem_material_df(const Dom &d, int k, DevScalars
         const df64 dxi = prod(own_xi, as_df(pairs(d.delx_xi)[k]));
         const df64 deta = prod(own_eta, as_df(pairs(d.delx_eta)[k]));
         const df64 dzeta = prod(own_zeta, as_df(pairs(d.delx_zeta)[k]));
-        const df64 rho = df_div(to_df(d.elem_mass[k]), to_df(d.volo[k]) * to_df(vnew));
+        const df64 rho = df_div(to_df(mass), to_df(volo) * to_df(vnew));
         const df64 one(1.f, 0.f);
         const df64 lin = (dxi * (one - phixi) + deta * (one - phieta)) + dzeta * (one - phizeta);
         const df64 quad = (dxi * dxi * (one - phixi * phixi) + deta * deta * (one - phieta * phieta)) +
@@ -502,9 +508,9 @@ __device__ __forceinline__ void elem_material_df(const Dom &d, int k, DevScalars
         d.ql[k] = to_double(qlin);
         d.qq[k] = to_double(qquad);
     }
-    const double ssn = material_update_df<SeriesFn>(d, k, sc, vnew, qlin, qquad, d.reps ? __ldg(d.reps + k) : 1);
+    const double ssn = material_update_df<SeriesFn>(d, k, sc, in, vnew, qlin, qquad, d.reps ? __ldg(d.reps + k) : 1);
     if (kConstraints)
-        constraint_keys_df<SeriesFn>(to_df(ssn), vdov, as_df(pairs(d.arealg)[k]), vdov.hi != 0.f, vdov.hi < 0.f, P, kc, kh);
+        constraint_keys_df<SeriesFn>(to_df(ssn), vdov, arealg, vdov.hi != 0.f, vdov.hi < 0.f, P, kc, kh);
 }
 
 // Eight blocks per SM (64 registers, ~40 bytes spilled; 80 registers at six

@@ -236,6 +236,7 @@ __device__ __forceinline__ void node_update_fp64(const Dom &d, int n, const DevS
     // the sums start from the first corner rather than from 0.0 (the same
     // value: x + 0.0 == x, up to the sign of a zero sum), one FP64 add fewer
     // per component; every node belongs to at least one element
+    const NodeState state = load_node(d, n);
     double fx = 0.0, fy = 0.0, fz = 0.0;
     for_node_corners(d, sc, n, [&](int c, bool first) {
         if (first) {
@@ -248,7 +249,7 @@ __device__ __forceinline__ void node_update_fp64(const Dom &d, int n, const DevS
             fz += d.fcz[c];
         }
     });
-    node_integrate(d, n, sc, fx, fy, fz);
+    node_integrate(d, n, sc, state, fx, fy, fz);
 }
 
 __global__ void __launch_bounds__(kBlockNode) k_node_update(const __grid_constant__ Dom d)
@@ -354,6 +355,7 @@ __device__ __forceinline__ void elem_material_fp64(const Dom &d, int k, DevScala
     {
         // CalcMonotonicQRegionForElems (:2182-2320)
         const int bc = __ldg(d.elem_bc + k);
+        const MaterialIn in = load_material(d, k);
         const FaceNeighbours nb = face_neighbours(d, sc, k);
         const double lim = P.monoq_limiter_mult, maxs = P.monoq_max_slope;
         const double phixi = limiter_phi(d.delv_xi, k, bc & BC_XI_M, bc & BC_XI_P, BC_XI_M_SYMM,
@@ -390,7 +392,7 @@ __device__ __forceinline__ void elem_material_fp64(const Dom &d, int k, DevScala
             d.qq[k] = qquad;
         }
 
-        const double ssn = material_update(d, k, sc, vnew, qlin, qquad, d.reps ? __ldg(d.reps + k) : 1);
+        const double ssn = material_update(d, k, sc, in, vnew, qlin, qquad, d.reps ? __ldg(d.reps + k) : 1);
 
         if (kConstraints) constraint_keys(ssn, vdov, d.arealg[k], P, kc, kh);
     }

@@ -375,9 +375,17 @@ __device__ __forceinline__ void kahan_add(float &s, float &c, float v)
     s = t;
 }
 
-__device__ __forceinline__ void node_update_split(const Dom &d, int n, const DevScalars *sc)
+// kEarly loads the node's state before its corners (load_node): on meshes
+// that leave most of an SM idle the update is its chain of memory latencies,
+// and this shortens it (a cycle of s=30 37.7 -> 36.9 us).  On large ones the
+// registers that it holds through the gather cost more (s=192 0.31 -> 0.40
+// ms: 56 registers, or 40 with spills, instead of 32), and each component is
+// loaded where it is used.
+template <bool kEarly>
+__device__ __forceinline__ void node_update_split_from(const Dom &d, int n, const DevScalars *sc)
 {
-
+    NodeState s{};
+    if (kEarly) s = load_node(d, n);
     float sx = 0.f, sy = 0.f, sz = 0.f, cx = 0.f, cy = 0.f, cz = 0.f;
     for_node_corners(d, sc, n, [&](int c, bool) {
         kahan_add(sx, cx, d.f32x[c]);
@@ -393,26 +401,33 @@ __device__ __forceinline__ void node_update_split(const Dom &d, int n, const Dev
         d.fz[n] = fz;
     }
     const double dt = sc->deltatime, u_cut = d.prm.u_cut;
-    const double im = d.inv_mass[n];
-    const unsigned bc = __ldg(d.node_bc + n);
-    const double ax = (bc & 1) ? 0.0 : fx * im;
-    const double ay = (bc & 2) ? 0.0 : fy * im;
-    const double az = (bc & 4) ? 0.0 : fz * im;
-    double t, p;
-    t = d.xd[n] + ax * dt; if (abs_lt(t, u_cut)) t = 0.0; p = d.x[n] + t * dt;
-    d.xd[n] = t; d.x[n] = p; d.xds[n] = split_hi_lo(t); d.xs[n] = split_hi_lo(p);
-    t = d.yd[n] + ay * dt; if (abs_lt(t, u_cut)) t = 0.0; p = d.y[n] + t * dt;
-    d.yd[n] = t; d.y[n] = p; d.yds[n] = split_hi_lo(t); d.ys[n] = split_hi_lo(p);
-    t = d.zd[n] + az * dt; if (abs_lt(t, u_cut)) t = 0.0; p = d.z[n] + t * dt;
-    d.zd[n] = t; d.z[n] = p; d.zds[n] = split_hi_lo(t); d.zs[n] = split_hi_lo(p);
+    const double im = kEarly ? s.m : d.inv_mass[n];
+    const unsigned bc = kEarly ? s.bc : __ldg(d.node_bc + n);
+    auto move = [&](double f, unsigned plane, double *v, double *x, float2 *vs, float2 *xs, double v0, double x0) {
+        double t = (kEarly ? v0 : v[n]) + ((bc & plane) ? 0.0 : f * im) * dt;
+        if (abs_lt(t, u_cut)) t = 0.0;
+        const double p = (kEarly ? x0 : x[n]) + t * dt;
+        v[n] = t;
+        x[n] = p;
+        vs[n] = split_hi_lo(t);
+        xs[n] = split_hi_lo(p);
+    };
+    move(fx, 1, d.xd, d.x, d.xds, d.xs, s.xd, s.x);
+    move(fy, 2, d.yd, d.y, d.yds, d.ys, s.yd, s.y);
+    move(fz, 4, d.zd, d.z, d.zds, d.zs, s.zd, s.z);
+}
+__device__ __forceinline__ void node_update_split(const Dom &d, int n, const DevScalars *sc)
+{
+    node_update_split_from<false>(d, n, sc);
 }
 
+template <bool kEarly>
 __global__ void __launch_bounds__(kBlockNode) k_node_update_split(const __grid_constant__ Dom d)
 {
     if (skip_step(d)) return;
     const int n = blockIdx.x * blockDim.x + threadIdx.x;
     if (n >= d.nn) return;
-    node_update_split(d, n, d.sc);
+    node_update_split_from<kEarly>(d, n, d.sc);
 }
 
 // ---------------------------------------------------------------------
@@ -505,6 +520,8 @@ __device__ __forceinline__ void elem_material_split(const Dom &d, int k, DevScal
         const size_t ne = (size_t)d.ne;
         const float *dv_xi = d.gq, *dv_eta = d.gq + ne, *dv_zeta = d.gq + 2 * ne;
         const int bc = __ldg(d.elem_bc + k);
+        const MaterialIn in = load_material(d, k);
+        const double vnew = d.vnew[k], vdov = d.vdov[k], arealg = d.arealg[k];
         const FaceNeighbours nb = face_neighbours(d, sc, k);
         const float lim = d2f(P.monoq_limiter_mult), maxs = d2f(P.monoq_max_slope);
         const float phixi = limiter_phi<float>(dv_xi, k, bc & BC_XI_M, bc & BC_XI_P, BC_XI_M_SYMM,
@@ -517,7 +534,6 @@ __device__ __forceinline__ void elem_material_split(const Dom &d, int k, DevScal
                                                  BC_ZETA_M_SYMM, BC_ZETA_M_FREE, BC_ZETA_P_SYMM,
                                                  BC_ZETA_P_FREE, nb.zetam, nb.zetap,
                                                  lim, maxs);
-        const double vnew = d.vnew[k], vdov = d.vdov[k];
         float qlin = 0.f, qquad = 0.f;
         if (!gt(vdov, 0.)) {
             float dxi = dv_xi[k] * d.gq[3 * ne + k];
@@ -539,10 +555,10 @@ __device__ __forceinline__ void elem_material_split(const Dom &d, int k, DevScal
         }
         // the EOS, energy, sound speed and constraint candidates in pairs,
         // the energy accumulated in FP64 (eos_df.cuh)
-        const double ssn = material_update_df<NewtonFn>(d, k, sc, vnew, df64(qlin, 0.f), df64(qquad, 0.f),
+        const double ssn = material_update_df<NewtonFn>(d, k, sc, in, vnew, df64(qlin, 0.f), df64(qquad, 0.f),
                                               d.reps ? __ldg(d.reps + k) : 1);
         if (kConstraints)
-            constraint_keys_df<NewtonFn>(to_df(ssn), to_df(vdov), to_df(d.arealg[k]), iabs(vdov) != 0ULL, lt(vdov, 0.), P,
+            constraint_keys_df<NewtonFn>(to_df(ssn), to_df(vdov), to_df(arealg), iabs(vdov) != 0ULL, lt(vdov, 0.), P,
                                          kc, kh);
     }
 }
@@ -584,10 +600,19 @@ void launch_split_sync(const Dom &d, cudaStream_t st)
     k_split_sync<<<blocks_for(d.nn, node_block(d)), node_block(d), 0, st>>>(d);
 }
 
+// (a mesh whose blocks choose_blocks has cut is one that does not fill the
+// SMs)
+static void launch_node_update_split(const Dom &d, cudaStream_t st)
+{
+    const unsigned grid = blocks_for(d.nn, node_block(d));
+    if (node_block(d) < kBlockNode) k_node_update_split<true><<<grid, node_block(d), 0, st>>>(d);
+    else k_node_update_split<false><<<grid, node_block(d), 0, st>>>(d);
+}
+
 void launch_lagrange_nodal_split(const Dom &d, cudaStream_t st)
 {
     launch_elem_force_split(d, st);
-    k_node_update_split<<<blocks_for(d.nn, node_block(d)), node_block(d), 0, st>>>(d);
+    launch_node_update_split(d, st);
 }
 
 void launch_lagrange_elements_split(const Dom &d, cudaStream_t st, bool with_constraints)
@@ -614,7 +639,7 @@ void launch_cycle_timed_split(const Dom &d, cudaStream_t st, cudaEvent_t ev[kTim
     cudaEventRecord(ev[1], st);
     launch_elem_force_split(d, st);
     cudaEventRecord(ev[2], st);
-    k_node_update_split<<<blocks_for(d.nn, node_block(d)), node_block(d), 0, st>>>(d);
+    launch_node_update_split(d, st);
     cudaEventRecord(ev[3], st);
     k_elem_kinematics_split<<<blocks_for(d.ne, kin_block(d)), kin_block(d), 0, st>>>(d);
     cudaEventRecord(ev[4], st);
