@@ -2,6 +2,7 @@
 // the captured run-loop graph and the step entry points.
 #include "lulesh_internal.h"
 #include "kernels.h"
+#include "common.cuh"
 
 #include <cuda_runtime.h>
 
@@ -41,6 +42,8 @@ struct lulesh_ctx {
 namespace {
 
 constexpr int kChunkCycles = 16;     // cycles per graph in the host-driven fallback
+constexpr int kUnroll = 4;           // cycles per pass of the while node, on meshes of up to
+constexpr long kSmallElems = 150000; // so many elements
 thread_local std::string g_err;
 
 }  // namespace
@@ -217,10 +220,10 @@ void nodal(lulesh_ctx *ctx, const Dom &d)
     else launch_lagrange_nodal(d, ctx->stream);
 }
 
-void elements(lulesh_ctx *ctx, const Dom &d, bool with_constraints)
+void elements(lulesh_ctx *ctx, const Dom &d, const CycleEnd *end)
 {
-    if (is_split(ctx)) launch_lagrange_elements_split(d, ctx->stream, with_constraints);
-    else launch_lagrange_elements(d, ctx->stream, with_constraints);
+    if (is_split(ctx)) launch_lagrange_elements_split(d, ctx->stream, end);
+    else launch_lagrange_elements(d, ctx->stream, end);
 }
 
 void run_body(lulesh_ctx *ctx, const Dom &d, cudaGraphConditionalHandle h)
@@ -229,7 +232,14 @@ void run_body(lulesh_ctx *ctx, const Dom &d, cudaGraphConditionalHandle h)
     else launch_run_body(d, ctx->stream, h, ctx->d_active);
 }
 
-// Build the run-loop graph: prologue -> while(cond) { one cycle }.  Falls
+// Cycles per pass of the while node.  A pass costs the node's own turn-round,
+// 3-4 us, which on a small mesh is a noticeable part of a cycle (s=10 39.6 ->
+// 36.5 us with four cycles, 36.1 with eight); the cycles after the
+// first return at once when the run has ended, which is cheap there.  On a
+// large mesh neither is worth having: one cycle per pass.
+int body_cycles(const lulesh_ctx *ctx) { return ctx->ne <= kSmallElems ? kUnroll : 1; }
+
+// Build the run-loop graph: prologue -> while(cond) { a few cycles }.  Falls
 // back to a host-driven graph of kChunkCycles gated cycles when conditional
 // nodes are not available.
 int build_run_graph(lulesh_ctx *ctx)
@@ -263,8 +273,10 @@ int build_run_graph(lulesh_ctx *ctx)
                                                cudaStreamCaptureModeThreadLocal) == cudaSuccess;
             if (ok) {
                 Dom d = ctx->dom;
-                d.gate = nullptr;
-                run_body(ctx, d, h);
+                for (int i = 0; i < body_cycles(ctx); ++i) {
+                    d.gate = i ? ctx->d_active : nullptr;
+                    run_body(ctx, d, h);
+                }
                 cudaGraph_t out = nullptr;
                 ok = cudaStreamEndCapture(ctx->stream, &out) == cudaSuccess;
             }
@@ -773,7 +785,7 @@ int lulesh_lagrange_elements(lulesh_ctx *ctx)
 {
     if (!ctx) return LULESH_ERR_ARG;
     if (ctx->status) return ctx->status;
-    elements(ctx, ctx->dom, false);
+    elements(ctx, ctx->dom, nullptr);
     ctx->launches += 2;
     int rc = check_launch(ctx);
     return rc ? rc : read_status(ctx);
@@ -794,8 +806,8 @@ int lulesh_lagrange_leapfrog(lulesh_ctx *ctx)
     if (!ctx) return LULESH_ERR_ARG;
     if (ctx->status) return ctx->status;
     nodal(ctx, ctx->dom);
-    elements(ctx, ctx->dom, true);
-    launch_finalize(ctx->dom, ctx->stream);
+    const CycleEnd end{};
+    elements(ctx, ctx->dom, &end);
     ctx->launches += 5;
     int rc = check_launch(ctx);
     return rc ? rc : read_status(ctx);

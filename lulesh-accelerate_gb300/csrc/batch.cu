@@ -249,8 +249,9 @@ long long staged_tiles(const lulesh_batch *b, int cls, int rows)
 
 int max_blocks(lulesh_batch *b, int kernel, int block)
 {
-    return b->precision == LULESH_PRECISION_SPLIT ? batch_max_blocks_split(kernel, block)
-                                                  : batch_max_blocks_fp64(kernel, block, b->dom.df);
+    const bool early = b->dom.nn < kEarlyNodes;
+    return b->precision == LULESH_PRECISION_SPLIT ? batch_max_blocks_split(kernel, block, early)
+                                                  : batch_max_blocks_fp64(kernel, block, b->dom.df, early);
 }
 
 unsigned compact_blocks(const lulesh_batch *b)

@@ -42,27 +42,38 @@ __device__ __forceinline__ bool skip_step(const Dom &d)
 // ---------------------------------------------------------------------
 // TimeIncrement (LULESH-OMP.cc:557-604)
 // ---------------------------------------------------------------------
+// x / 3, correctly rounded: the remainder of the product with the rounded
+// reciprocal is exact and corrects it (Markstein 1990).  The step is one
+// thread's chain of FP64 operations, and a division is a dozen of them; the
+// halving is exact as a product.
+__device__ __forceinline__ double third(double x)
+{
+    const double q = x * (1.0 / 3.0), r = fma(-3.0, q, x);
+    return fma(r, 1.0 / 3.0, q);
+}
 __device__ __forceinline__ void time_increment(DevScalars *sc, const lulesh_params &P)
 {
-    double targetdt = P.stoptime - sc->time;
-    if ((P.dtfixed <= 0.0) && (sc->cycle != 0)) {
-        const double olddt = sc->deltatime;
+    const double time = sc->time, courant = sc->dtcourant, hydro = sc->dthydro;
+    const int cycle = sc->cycle;
+    double dt = sc->deltatime, targetdt = P.stoptime - time;
+    if ((P.dtfixed <= 0.0) && (cycle != 0)) {
+        const double olddt = dt;
         double newdt = 1.0e+20;
-        if (sc->dtcourant < newdt) newdt = sc->dtcourant / 2.0;
-        if (sc->dthydro < newdt) newdt = sc->dthydro * 2.0 / 3.0;
+        if (courant < newdt) newdt = courant * 0.5;
+        if (hydro < newdt) newdt = third(hydro * 2.0);
         const double ratio = newdt / olddt;
         if (ratio >= 1.0) {
             if (ratio < P.deltatimemultlb) newdt = olddt;
             else if (ratio > P.deltatimemultub) newdt = olddt * P.deltatimemultub;
         }
         if (newdt > P.dtmax) newdt = P.dtmax;
-        sc->deltatime = newdt;
+        dt = newdt;
     }
-    if ((targetdt > sc->deltatime) && (targetdt < (4.0 * sc->deltatime / 3.0)))
-        targetdt = 2.0 * sc->deltatime / 3.0;
-    if (targetdt < sc->deltatime) sc->deltatime = targetdt;
-    sc->time += sc->deltatime;
-    ++sc->cycle;
+    if ((targetdt > dt) && (targetdt < third(4.0 * dt))) targetdt = third(2.0 * dt);
+    if (targetdt < dt) dt = targetdt;
+    sc->deltatime = dt;
+    sc->time = time + dt;
+    sc->cycle = cycle + 1;
 }
 
 // Comparisons of doubles on the integer pipes.  The FP64 unit of this part
@@ -273,6 +284,61 @@ __device__ __forceinline__ void for_node_corners(const Dom &d, const DevScalars 
     }
     for_listed_corners(d, n, f);
 }
+
+// A node's first eight corner slots in that order, for loading all of them
+// before any is used (for_node_corners takes each in a branch of its own, one
+// memory latency after the other, which is most of the update on a mesh that
+// does not fill the SMs): present tells which exist; the others are slot 0.
+// A listed node with more corners has the rest at list entries rest..end.
+struct CornerSlots {
+    int slot[8];
+    unsigned present;
+    int rest, end;
+};
+__device__ __forceinline__ CornerSlots corner_slots(const Dom &d, const DevScalars *sc, int n)
+{
+    CornerSlots c;
+    c.present = 0;
+    c.rest = c.end = 0;
+    const int s = d.s > 0 ? d.s : sc->edge;
+    if (s > 0) {
+        const NodePlace at = node_place(d, sc, s, n);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int dp = !(i & 4), dr = !(i & 2), dc = !(i & 1);
+            const bool in = at.inside(s, dp, dr, dc);
+            c.slot[i] = in ? (int)(corner_of(dp, dr, dc) * (size_t)d.ne + at.element(s, dp, dr, dc)) : 0;
+            c.present |= (in ? 1u : 0u) << i;
+        }
+    } else {
+        const int st = __ldg(d.corner_start + n), en = __ldg(d.corner_start + n + 1);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const bool in = st + i < en;
+            c.slot[i] = in ? __ldg(d.corner_list + st + i) : 0;
+            c.present |= (in ? 1u : 0u) << i;
+        }
+        c.rest = st + 8;
+        c.end = en;
+    }
+    return c;
+}
+// The three components of those corners, zero where there is none.
+template <typename T>
+__device__ __forceinline__ void load_corners(const CornerSlots &c, const T *fx, const T *fy, const T *fz, T f[3][8])
+{
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const bool in = (c.present >> i) & 1;
+        f[0][i] = fx[c.slot[i]];
+        f[1][i] = fy[c.slot[i]];
+        f[2][i] = fz[c.slot[i]];
+        if (!in) f[0][i] = f[1][i] = f[2][i] = T{};
+    }
+}
+// Meshes that take the early gathers: below four 128-thread blocks per SM,
+// where choose_blocks has cut the blocks (a batch: as many nodes in all).
+constexpr int kEarlyNodes = 80000;
 
 // One direction of the monotonic limiter (:2198-2228).
 template <typename T>
@@ -553,8 +619,9 @@ __device__ __forceinline__ void constraint_keys_df(df64 ss, df64 vdov, df64 area
 __device__ __forceinline__ void finalize_constraints(DevScalars *sc)
 {
     const unsigned long long limit = order_key(1.0e+20);
-    if (sc->courant_key < limit) sc->dtcourant = key_value(sc->courant_key);
-    if (sc->hydro_key < limit) sc->dthydro = key_value(sc->hydro_key);
+    const unsigned long long courant = sc->courant_key, hydro = sc->hydro_key;
+    if (courant < limit) sc->dtcourant = key_value(courant);
+    if (hydro < limit) sc->dthydro = key_value(hydro);
     sc->courant_key = ~0ULL;
     sc->hydro_key = ~0ULL;
 }
@@ -568,6 +635,29 @@ __device__ __forceinline__ unsigned run_continue(const DevScalars *sc, const lul
     const int cap = (sc->run_max > 0 && sc->run_max < kRunCycleLimit) ? sc->run_max : kRunCycleLimit;
     return (sc->err_any == 0) && (sc->time < P.stoptime) && (sc->deltatime > 0.0) &&
            (sc->run_cycles < cap);
+}
+
+// The end of a cycle, one thread's work: the constraint minima are published,
+// and in the run loop (active not null) the cycle is counted, the loop
+// condition set and the next cycle's TimeIncrement done, which as a kernel of
+// its own cost another launch per cycle.  (Having the material kernel's last
+// block do all this instead was slower: s=10 32.9 against 31.8 us a cycle, and
+// every block's fence and count cost the split material kernel 4 % at s=192.)
+struct CycleEnd {
+    cudaGraphConditionalHandle handle;
+    int *active;
+};
+__device__ __forceinline__ void end_cycle(const Dom &d, const CycleEnd &end)
+{
+    DevScalars *sc = d.sc;
+    if (end.active && !*end.active) return;
+    finalize_constraints(sc);
+    if (!end.active) return;
+    sc->run_cycles++;
+    const unsigned go = run_continue(sc, d.prm);
+    *end.active = (int)go;
+    if (end.handle) cudaGraphSetConditional(end.handle, go);
+    if (go) time_increment(sc, d.prm);
 }
 
 }  // namespace lulesh

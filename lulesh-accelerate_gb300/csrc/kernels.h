@@ -39,19 +39,22 @@ inline void choose_blocks(Dom &d, int sms)
     d.nblock = nb;
 }
 
+struct CycleEnd;   // common.cuh
+void launch_end_cycle(const Dom &d, cudaStream_t st, const CycleEnd &end);
+
 // Plain FP64 path (step_fp64.cu).
 void launch_time_increment(const Dom &d, cudaStream_t st);
 void launch_lagrange_nodal(const Dom &d, cudaStream_t st);
-void launch_lagrange_elements(const Dom &d, cudaStream_t st, bool with_constraints);
+// end null: without the time constraints
+void launch_lagrange_elements(const Dom &d, cudaStream_t st, const CycleEnd *end);
 void launch_time_constraints(const Dom &d, cudaStream_t st);
-void launch_finalize(const Dom &d, cudaStream_t st);
 void launch_run_prologue(const Dom &d, cudaStream_t st, const int *max_cycles,
                          cudaGraphConditionalHandle h, int *active);
 void launch_run_body(const Dom &d, cudaStream_t st, cudaGraphConditionalHandle h, int *active);
-void launch_run_epilogue(const Dom &d, cudaStream_t st, cudaGraphConditionalHandle h, int *active);
 int kernels_per_cycle();
 constexpr int kRunCycleLimit = LULESH_RUN_CYCLE_BUDGET;
-constexpr int kTimedKernels = 6;   // time increment, force, node, kinematics, material, finalize
+// time increment, force, node, kinematics, material, constraint publication
+constexpr int kTimedKernels = 6;
 void launch_cycle_timed(const Dom &d, cudaStream_t st, cudaEvent_t ev[kTimedKernels + 1]);
 void launch_fp64_probe(double *out, int blocks, int threads, int iters, cudaStream_t st);
 void launch_rate_probe(int which, float *out, int blocks, int threads, int iters, cudaStream_t st);
@@ -64,14 +67,14 @@ void launch_math_probe(unsigned long long *keys, int n, cudaStream_t st);
 void launch_elem_force_df(const Dom &d, cudaStream_t st);
 void launch_node_update_df(const Dom &d, cudaStream_t st);
 void launch_elem_kinematics_df(const Dom &d, cudaStream_t st);
-void launch_elem_material_df(const Dom &d, cudaStream_t st, bool with_constraints);
+void launch_elem_material_df(const Dom &d, cudaStream_t st, const CycleEnd *end);
 void launch_batch_kernel_df(const Dom &d, const BatchView &b, cudaStream_t st, int kernel, int cls, LaunchCfg cfg);
-int batch_max_blocks_df(int kernel, int block);
+int batch_max_blocks_df(int kernel, int block, bool early);
 
 // Split-precision path (step_split.cu).
 void launch_split_sync(const Dom &d, cudaStream_t st);
 void launch_lagrange_nodal_split(const Dom &d, cudaStream_t st);
-void launch_lagrange_elements_split(const Dom &d, cudaStream_t st, bool with_constraints);
+void launch_lagrange_elements_split(const Dom &d, cudaStream_t st, const CycleEnd *end);
 void launch_run_body_split(const Dom &d, cudaStream_t st, cudaGraphConditionalHandle h, int *active);
 void launch_cycle_timed_split(const Dom &d, cudaStream_t st, cudaEvent_t ev[kTimedKernels + 1]);
 
@@ -81,8 +84,8 @@ void launch_batch_kernel_fp64(const Dom &d, const BatchView &b, cudaStream_t st,
                               LaunchCfg cfg);
 void launch_batch_kernel_split(const Dom &d, const BatchView &b, cudaStream_t st, int kernel, int cls,
                                LaunchCfg cfg);
-int batch_max_blocks_fp64(int kernel, int block, int arith);
-int batch_max_blocks_split(int kernel, int block);
+int batch_max_blocks_fp64(int kernel, int block, int arith, bool early);
+int batch_max_blocks_split(int kernel, int block, bool early);
 void launch_batch_force_split_staged(const Dom &d, const BatchView &b, const StagedClass &sc, int rows,
                                      LaunchCfg cfg, cudaStream_t st);
 int batch_max_blocks_split_staged(int rows);

@@ -114,7 +114,7 @@ __device__ __forceinline__ Crosses crosses_of(const Modes &m)
 // times the normal generators in F_1..F_3.  60 products per component
 // instead of 64 and the 96 that the shape vectors take, and the transforms
 // are additions.  Everything runs on pairs of modes (dfpack.cuh).
-__device__ __forceinline__ void elem_force_df(const Dom &d, int k, DevScalars *sc)
+__device__ __forceinline__ void elem_force_components(const Dom &d, int k, DevScalars *sc, int dim0, int dim1)
 {
     const size_t ne = (size_t)d.ne;
     // the element scalars first: their loads are in flight with the geometry's
@@ -136,7 +136,7 @@ __device__ __forceinline__ void elem_force_df(const Dom &d, int k, DevScalars *s
     }
     // the first velocity component's corners, in flight during the geometry
     double un[8];
-    gather8(d.xd, nl, un);
+    gather8(dim0 == 0 ? d.xd : (dim0 == 1 ? d.yd : d.zd), nl, un);
 
     V2x3 W12, W56, W34;
     V1x3 n1, n2, n3;   // normal generators, times (p + q)/64
@@ -184,7 +184,7 @@ __device__ __forceinline__ void elem_force_df(const Dom &d, int k, DevScalars *s
     // is most of the kernel's instructions); each iteration issues the next
     // component's corner gather before its own arithmetic.
 #pragma unroll 1
-    for (int dim = 0; dim < 3; ++dim) {
+    for (int dim = dim0; dim < dim1; ++dim) {
         // (the component is selected, not indexed, so that it stays in
         // registers)
         auto comp = [&](const V1x3 &v) {
@@ -195,7 +195,7 @@ __device__ __forceinline__ void elem_force_df(const Dom &d, int k, DevScalars *s
         df64 F3, F4, F7;
         if (hourglass) {
             const ModePacks u = walsh_packs(corners_of(un));
-            if (dim < 2) gather8(dim == 0 ? d.yd : d.zd, nl, un);
+            if (dim + 1 < dim1) gather8(dim == 0 ? d.yd : d.zd, nl, un);
             const df2n u12 = df2_both(u.m12), u56 = df2_both(u.m56), u34 = df2_both(df2_pack(df2_y(u.m73), u.m4));
             auto modes_dot = [&](df2 a, df2 b, df2 c) {
                 return df2_both(df2_dup(joined(Dot2(a, u12).add(b, u56)).plus(joined(Dot2(c, u34))).value()));
@@ -239,12 +239,26 @@ __device__ __forceinline__ void elem_force_df(const Dom &d, int k, DevScalars *s
     }
 }
 
+__device__ __forceinline__ void elem_force_df(const Dom &d, int k, DevScalars *sc) { elem_force_components(d, k, sc, 0, 3); }
+
 __global__ void __launch_bounds__(kBlockElem) k_elem_force_df(const __grid_constant__ Dom d)
 {
     if (skip_step(d)) return;
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= d.ne) return;
     elem_force_df(d, k, d.sc);
+}
+
+// Meshes that leave most of the SMs' warp slots empty run one thread per
+// element and component (blockIdx.y): the geometry is formed three times, but
+// a thread's chain is 2,200 instructions instead of 4,200, and its length is
+// what the kernel takes there (the kinematics kernel likewise, below).
+__global__ void __launch_bounds__(kBlockElem) k_elem_force_df_by_component(const __grid_constant__ Dom d)
+{
+    if (skip_step(d)) return;
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= d.ne) return;
+    elem_force_components(d, k, d.sc, blockIdx.y, blockIdx.y + 1);
 }
 
 // ---------------------------------------------------------------------
@@ -255,6 +269,12 @@ __global__ void __launch_bounds__(kBlockElem) k_elem_force_df(const __grid_const
 // two on the diagonal and the two off it, so that exchanging rows and columns
 // exchanges operands only and the mirror symmetry that the element kernels
 // keep (dfpack.cuh) is not lost here.
+__device__ __forceinline__ df64 corner_tree(const df64 f[8])
+{
+    // list order: (1,1,1) (1,1,0) (1,0,1) (1,0,0) (0,1,1) ... of (dp, dr, dc)
+    return ((f[0] + f[3]) + (f[1] + f[2])) + ((f[4] + f[7]) + (f[5] + f[6]));
+}
+template <bool kEarly>
 __device__ __forceinline__ void node_update_df(const Dom &d, int n, const DevScalars *sc)
 {
     const float2 *const fc[3] = {reinterpret_cast<const float2 *>(d.fcx), reinterpret_cast<const float2 *>(d.fcy),
@@ -262,7 +282,26 @@ __device__ __forceinline__ void node_update_df(const Dom &d, int n, const DevSca
     const NodeState state = load_node(d, n);
     df64 f[3] = {df64(0.f, 0.f), df64(0.f, 0.f), df64(0.f, 0.f)};
     const int s = d.s > 0 ? d.s : sc->edge;
-    if (s > 0) {
+    if (kEarly) {
+        const CornerSlots at = corner_slots(d, sc, n);
+        float2 c[3][8];
+        load_corners(at, fc[0], fc[1], fc[2], c);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            df64 v[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) v[j] = as_df(c[i][j]);
+            if (s > 0) {
+                f[i] = corner_tree(v);
+            } else {
+                f[i] = v[0];
+#pragma unroll
+                for (int j = 1; j < 8; ++j)
+                    if ((at.present >> j) & 1) f[i] = f[i] + v[j];
+                for (int j = at.rest; j < at.end; ++j) f[i] = f[i] + as_df(fc[i][__ldg(d.corner_list + j)]);
+            }
+        }
+    } else if (s > 0) {
         const NodePlace at = node_place(d, sc, s, n);
         const size_t ne = (size_t)d.ne;
 #pragma unroll
@@ -287,13 +326,14 @@ __device__ __forceinline__ void node_update_df(const Dom &d, int n, const DevSca
 // memory, and the early loads of load_node (0.387 -> 0.379 ms at s=192) cost
 // registers that the compiler would otherwise take 54 of; 0.355 ms at the
 // cap, 0.380 at 32 registers.
-__global__ void __launch_bounds__(kBlockNode, 12) k_node_update_df(const __grid_constant__ Dom d)
+template <bool kEarly>
+__global__ void __launch_bounds__(kBlockNode, kEarly ? 4 : 12) k_node_update_df(const __grid_constant__ Dom d)
 {
     if (skip_step(d)) return;
     const int n = blockIdx.x * blockDim.x + threadIdx.x;
     if (n >= d.nn) return;
     if (n == 0 && d.geo) d.sc->geo_valid = 0;   // the positions move: the geometry cache goes stale
-    node_update_df(d, n, d.sc);
+    node_update_df<kEarly>(d, n, d.sc);
 }
 
 // ---------------------------------------------------------------------
@@ -315,7 +355,11 @@ __device__ __forceinline__ df64 face_pair_max(const V1x3 &X, const V1x3 &Y)
     return fmax(df2_x(n), df2_y(n));
 }
 
-__device__ __forceinline__ void elem_kinematics_df(const Dom &d, int k, DevScalars *sc)
+// kParts: kVolume the volume, the length and the geometry cache, kGradients
+// the Q gradients, kStrain the strain rate.
+enum : int { kVolume = 1, kGradients = 2, kStrain = 4, kAllParts = 7 };
+template <int kParts>
+__device__ __forceinline__ void elem_kinematics_parts(const Dom &d, int k, DevScalars *sc)
 {
     const size_t ne = (size_t)d.ne;
     int nl[8];
@@ -323,10 +367,12 @@ __device__ __forceinline__ void elem_kinematics_df(const Dom &d, int k, DevScala
     const ModePacks mx = field_modes(d.x, nl), my = field_modes(d.y, nl), mz = field_modes(d.z, nl);
     // the next cycle's force kernel works on these same positions; every
     // context that runs this kernel keeps the cache
-    store_geometry_df(d.geo, ne, k, 0, mx);
-    store_geometry_df(d.geo, ne, k, 1, my);
-    store_geometry_df(d.geo, ne, k, 2, mz);
-    if (k == sc->elem_begin) sc->geo_valid = 1;
+    if constexpr (kParts & kVolume) {
+        store_geometry_df(d.geo, ne, k, 0, mx);
+        store_geometry_df(d.geo, ne, k, 1, my);
+        store_geometry_df(d.geo, ne, k, 2, mz);
+        if (k == sc->elem_begin) sc->geo_valid = 1;
+    }
 
     const Modes M = modes_of(mx, my, mz);
     const Crosses X = crosses_of(M);
@@ -341,13 +387,13 @@ __device__ __forceinline__ void elem_kinematics_df(const Dom &d, int k, DevScala
     }();
     // volume / volo, as a product with the reciprocal taken at set-up, in
     // FP64: it is state, and one product costs less than its two conversions
+    if constexpr (kParts & kVolume) {
     const double rel = to_double(df_scale(vol64, 1.f / 64.f)) * __ldg(d.inv_volo + k);
     d.vnew[k] = rel;
     d.delv[k] = rel - d.v[k];
     if (rel <= 0.0) flag_error(sc, ERR_K3_VNEW, k);
 
     // CalcElemCharacteristicLength (:1821-1862): 4V / sqrt(max AreaFace)
-    {
         // a = M3xM4, -b = M5xM2, c = M6xM1; Y1 = b - a, Y2 = c + a, Y3 = c + b
         const V2x3 bc = cross2(d56, swapped(M.m12));
         const V1x3 a = cross1(M.m3, M.m4), nb = half_x(bc), c = half_y(bc);
@@ -355,6 +401,7 @@ __device__ __forceinline__ void elem_kinematics_df(const Dom &d, int k, DevScala
                             face_pair_max(X.n3, sum1(c, minus(nb))));
         reinterpret_cast<float2 *>(d.arealg)[k] = as_float2(df_scale(vol64, 0.25f) * df_rsqrt(f));
     }
+    if constexpr (!(kParts & (kGradients | kStrain))) return;
 
     V2x3 V12;   // velocity modes (V1, V2) and V3
     V1x3 V3v;
@@ -380,7 +427,7 @@ __device__ __forceinline__ void elem_kinematics_df(const Dom &d, int k, DevScala
     // are M/4, so each cross product is (M x M')/16 and each velocity
     // difference Mv/4; volo vnew is the volume.  eta and xi in the halves of
     // a pair (M3xM1, M3xM2), zeta beside them.  Kept as pairs (Dom::delv_xi).
-    {
+    if constexpr (kParts & kGradients) {
         const df64 ptiny(1.e-36);
         const df64 vol = df_scale(vol64, 1.f / 64.f);
         // (1/16) (1/4) / (vol + ptiny)
@@ -401,7 +448,7 @@ __device__ __forceinline__ void elem_kinematics_df(const Dom &d, int k, DevScala
     // CalcKinematicsForElems, strain-rate part (:1975-2020): the half-step
     // Jacobian's columns (M - dt/2 V)/8, the rate their cofactors . V over
     // their determinant (strain_rate, hexmodes.cuh); cof = (CxA, CxB)
-    {
+    if constexpr (kParts & kStrain) {
         const df64 dt2 = to_df(0.5 * sc->deltatime);
         const df2n nd = df2_both(df2_dup(dt2));
         auto back2 = [&](df2 m, df2 v) { return Dot2(v, nd).minus(m).negative(); };
@@ -413,6 +460,23 @@ __device__ __forceinline__ void elem_kinematics_df(const Dom &d, int k, DevScala
         const df64 num = dot1(cze, V3v).plus(difference(dot2(cof, V21))).value();
         reinterpret_cast<float2 *>(d.vdov)[k] = as_float2(df_div(num, dot1(C, cze).value()));
     }
+}
+
+__device__ __forceinline__ void elem_kinematics_df(const Dom &d, int k, DevScalars *sc)
+{
+    elem_kinematics_parts<kAllParts>(d, k, sc);
+}
+
+// One thread per element and part (blockIdx.y), for the meshes of
+// k_elem_force_df_by_component.
+__global__ void __launch_bounds__(kKinBlockFactor * kBlockElem, 2) k_elem_kinematics_df_by_part(const __grid_constant__ Dom d)
+{
+    if (skip_step(d)) return;
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= d.ne) return;
+    if (blockIdx.y == 0) elem_kinematics_parts<kGradients>(d, k, d.sc);
+    else if (blockIdx.y == 1) elem_kinematics_parts<kVolume>(d, k, d.sc);
+    else elem_kinematics_parts<kStrain>(d, k, d.sc);
 }
 
 __global__ void __launch_bounds__(kKinBlockFactor * kBlockElem, 2) k_elem_kinematics_df(const __grid_constant__ Dom d)
@@ -437,15 +501,14 @@ __global__ void __launch_bounds__(kKinBlockFactor * kBlockElem, 2) k_elem_kinema
 // taken as +-2^100.  That changes no outcome: a ratio beyond it is never the
 // minimum unless both are, and then the result is max_slope either way; a
 // negative one makes the result 0 either way.
-__device__ __forceinline__ df64 limiter_phi_df(const float2 *__restrict__ delv, df64 own, int bm, int bp,
-                                               int m_symm, int p_symm, int lm, int lp, df64 limiter, df64 max_slope)
+// dm, dp: the neighbours' slopes (of any element where the face has a flag).
+__device__ __forceinline__ df64 limiter_phi_df(df64 own, df64 dm, df64 dp, int bm, int bp, int m_symm, int p_symm,
+                                               df64 limiter, df64 max_slope)
 {
     const df64 norm = df_rcp(own + df64(1.e-36));
-    df64 dm(0.f, 0.f), dp(0.f, 0.f);   // 0 beyond a free face
-    if (bm == 0) dm = as_df(delv[lm]);
-    else if (bm == m_symm) dm = own;
-    if (bp == 0) dp = as_df(delv[lp]);
-    else if (bp == p_symm) dp = own;
+    const df64 zero(0.f, 0.f);   // beyond a free face
+    if (bm != 0) dm = bm == m_symm ? own : zero;
+    if (bp != 0) dp = bp == p_symm ? own : zero;
     const float big = 1.2676506e30f;   // 2^100
     auto ratio = [&](df64 a) {
         if (fabsf(a.hi) * fabsf(norm.hi) > big)   // may be inf: still > big
@@ -480,12 +543,15 @@ __device__ __forceinline__ void elem_material_df(const Dom &d, int k, DevScalars
     const df64 lim = to_df(P.monoq_limiter_mult), maxs = to_df(P.monoq_max_slope);
     const float2 *dv_xi = pairs(d.delv_xi), *dv_eta = pairs(d.delv_eta), *dv_zeta = pairs(d.delv_zeta);
     const df64 own_xi = as_df(dv_xi[k]), own_eta = as_df(dv_eta[k]), own_zeta = as_df(dv_zeta[k]);
-    const df64 phixi = limiter_phi_df(dv_xi, own_xi, bc & BC_XI_M, bc & BC_XI_P, BC_XI_M_SYMM, BC_XI_P_SYMM, nb.xim,
-                                      nb.xip, lim, maxs);
-    const df64 phieta = limiter_phi_df(dv_eta, own_eta, bc & BC_ETA_M, bc & BC_ETA_P, BC_ETA_M_SYMM, BC_ETA_P_SYMM,
-                                       nb.etam, nb.etap, lim, maxs);
-    const df64 phizeta = limiter_phi_df(dv_zeta, own_zeta, bc & BC_ZETA_M, bc & BC_ZETA_P, BC_ZETA_M_SYMM,
-                                        BC_ZETA_P_SYMM, nb.zetam, nb.zetap, lim, maxs);
+    // the neighbours' slopes without waiting for the face flags: where a flag
+    // replaces one, whatever element its clamped index names is loaded
+    auto near_k = [&](const float2 *f, int i) { return as_df(f[min(max(i, 0), d.ne - 1)]); };
+    const df64 xm = near_k(dv_xi, nb.xim), xp = near_k(dv_xi, nb.xip), em = near_k(dv_eta, nb.etam);
+    const df64 ep = near_k(dv_eta, nb.etap), zm = near_k(dv_zeta, nb.zetam), zp = near_k(dv_zeta, nb.zetap);
+    const df64 phixi = limiter_phi_df(own_xi, xm, xp, bc & BC_XI_M, bc & BC_XI_P, BC_XI_M_SYMM, BC_XI_P_SYMM, lim, maxs);
+    const df64 phieta = limiter_phi_df(own_eta, em, ep, bc & BC_ETA_M, bc & BC_ETA_P, BC_ETA_M_SYMM, BC_ETA_P_SYMM, lim, maxs);
+    const df64 phizeta = limiter_phi_df(own_zeta, zm, zp, bc & BC_ZETA_M, bc & BC_ZETA_P, BC_ZETA_M_SYMM, BC_ZETA_P_SYMM,
+                                        lim, maxs);
     df64 qlin(0.f, 0.f), qquad(0.f, 0.f);
     if (!(vdov.hi > 0.f)) {
         // the products delv * delx; a positive one contributes nothing
@@ -533,29 +599,34 @@ __global__ void __launch_bounds__(kBlockElem, 8) k_elem_material_df(const __grid
 // ---------------------------------------------------------------------
 // Launchers
 // ---------------------------------------------------------------------
+constexpr int kByPartElems = 7000;
 static inline unsigned blocks_for(long n, int bs) { return (unsigned)((n + bs - 1) / bs); }
 
 void launch_elem_force_df(const Dom &d, cudaStream_t st)
 {
-    k_elem_force_df<<<blocks_for(d.ne, elem_block(d)), elem_block(d), 0, st>>>(d);
+    const unsigned grid = blocks_for(d.ne, elem_block(d));
+    if (d.ne < kByPartElems) k_elem_force_df_by_component<<<dim3(grid, 3), elem_block(d), 0, st>>>(d);
+    else k_elem_force_df<<<grid, elem_block(d), 0, st>>>(d);
 }
 
 void launch_node_update_df(const Dom &d, cudaStream_t st)
 {
-    k_node_update_df<<<blocks_for(d.nn, node_block(d)), node_block(d), 0, st>>>(d);
+    const unsigned grid = blocks_for(d.nn, node_block(d));
+    if (d.nn < kEarlyNodes) k_node_update_df<true><<<grid, node_block(d), 0, st>>>(d);
+    else k_node_update_df<false><<<grid, node_block(d), 0, st>>>(d);
 }
 
 void launch_elem_kinematics_df(const Dom &d, cudaStream_t st)
 {
-    k_elem_kinematics_df<<<blocks_for(d.ne, kin_block(d)), kin_block(d), 0, st>>>(d);
+    const unsigned grid = blocks_for(d.ne, kin_block(d));
+    if (d.ne < kByPartElems) k_elem_kinematics_df_by_part<<<dim3(grid, 3), kin_block(d), 0, st>>>(d);
+    else k_elem_kinematics_df<<<grid, kin_block(d), 0, st>>>(d);
 }
 
-void launch_elem_material_df(const Dom &d, cudaStream_t st, bool with_constraints)
+void launch_elem_material_df(const Dom &d, cudaStream_t st, const CycleEnd *end)
 {
-    if (with_constraints)
-        k_elem_material_df<true><<<blocks_for(d.ne, elem_block(d)), elem_block(d), 0, st>>>(d);
-    else
-        k_elem_material_df<false><<<blocks_for(d.ne, elem_block(d)), elem_block(d), 0, st>>>(d);
+    if (end) k_elem_material_df<true><<<blocks_for(d.ne, elem_block(d)), elem_block(d), 0, st>>>(d);
+    else k_elem_material_df<false><<<blocks_for(d.ne, elem_block(d)), elem_block(d), 0, st>>>(d);
 }
 
 // Batched ensembles: kernels 0..3 (force, node update, kinematics, material)
@@ -564,19 +635,25 @@ void launch_batch_kernel_df(const Dom &d, const BatchView &b, cudaStream_t st, i
 {
     switch (kernel) {
     case 0: kb_elem<elem_force_df><<<cfg.grid, cfg.block, 0, st>>>(d, b, cls); break;
-    case 1: kb_node<node_update_df><<<cfg.grid, cfg.block, 0, st>>>(d, b, cls); break;
+    case 1:
+        if (d.nn < kEarlyNodes) kb_node<node_update_df<true>><<<cfg.grid, cfg.block, 0, st>>>(d, b, cls);
+        else kb_node<node_update_df<false>><<<cfg.grid, cfg.block, 0, st>>>(d, b, cls);
+        break;
     case 2: kb_elem<elem_kinematics_df><<<cfg.grid, cfg.block, 0, st>>>(d, b, cls); break;
     default: kb_material_capped<elem_material_df<true>, 4><<<cfg.grid, cfg.block, 0, st>>>(d, b, cls); break;
     }
 }
 
-int batch_max_blocks_df(int kernel, int block)
+int batch_max_blocks_df(int kernel, int block, bool early)
 {
     int n = 0;
     cudaError_t e;
     switch (kernel) {
     case 0: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kb_elem<elem_force_df>, block, 0); break;
-    case 1: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kb_node<node_update_df>, block, 0); break;
+    case 1:
+        e = early ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kb_node<node_update_df<true>>, block, 0)
+                  : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kb_node<node_update_df<false>>, block, 0);
+        break;
     case 2: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kb_elem<elem_kinematics_df>, block, 0); break;
     default: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kb_material_capped<elem_material_df<true>, 4>, block, 0); break;
     }

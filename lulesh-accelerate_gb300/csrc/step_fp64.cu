@@ -230,35 +230,44 @@ __global__ void __launch_bounds__(kBlockElem, 4) k_elem_force(const __grid_const
 // Node update: fixed-order corner gather + acceleration, BC, velocity,
 // position
 // ---------------------------------------------------------------------
+template <bool kEarly>
 __device__ __forceinline__ void node_update_fp64(const Dom &d, int n, const DevScalars *sc)
 {
-
     // the sums start from the first corner rather than from 0.0 (the same
     // value: x + 0.0 == x, up to the sign of a zero sum), one FP64 add fewer
     // per component; every node belongs to at least one element
     const NodeState state = load_node(d, n);
     double fx = 0.0, fy = 0.0, fz = 0.0;
-    for_node_corners(d, sc, n, [&](int c, bool first) {
-        if (first) {
-            fx = d.fcx[c];
-            fy = d.fcy[c];
-            fz = d.fcz[c];
-        } else {
-            fx += d.fcx[c];
-            fy += d.fcy[c];
-            fz += d.fcz[c];
+    auto take = [&](double cx, double cy, double cz, bool first) {
+        fx = first ? cx : fx + cx;
+        fy = first ? cy : fy + cy;
+        fz = first ? cz : fz + cz;
+    };
+    if (kEarly) {
+        const CornerSlots at = corner_slots(d, sc, n);
+        double c[3][8];
+        load_corners<double>(at, d.fcx, d.fcy, d.fcz, c);
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+            if ((at.present >> j) & 1) take(c[0][j], c[1][j], c[2][j], (at.present & ((1u << j) - 1)) == 0);
+        for (int j = at.rest; j < at.end; ++j) {
+            const int i = __ldg(d.corner_list + j);
+            take(d.fcx[i], d.fcy[i], d.fcz[i], false);
         }
-    });
+    } else {
+        for_node_corners(d, sc, n, [&](int c, bool first) { take(d.fcx[c], d.fcy[c], d.fcz[c], first); });
+    }
     node_integrate(d, n, sc, state, fx, fy, fz);
 }
 
+template <bool kEarly>
 __global__ void __launch_bounds__(kBlockNode) k_node_update(const __grid_constant__ Dom d)
 {
     if (skip_step(d)) return;
     const int n = blockIdx.x * blockDim.x + threadIdx.x;
     if (n >= d.nn) return;
     if (n == 0 && d.geo) d.sc->geo_valid = 0;   // the positions move: the geometry cache goes stale
-    node_update_fp64(d, n, d.sc);
+    node_update_fp64<kEarly>(d, n, d.sc);
 }
 
 // ---------------------------------------------------------------------
@@ -429,11 +438,10 @@ __global__ void __launch_bounds__(kBlockElem) k_time_constraints(const __grid_co
     block_min_publish(kc, kh, d.sc);
 }
 
-__global__ void k_finalize(const __grid_constant__ Dom d)
-{
-    finalize_constraints(d.sc);
-}
+__global__ void k_end_cycle(const __grid_constant__ Dom d, const __grid_constant__ CycleEnd end) { end_cycle(d, end); }
 
+// The start of a run: may a cycle start at all?  The first cycle's
+// TimeIncrement (every later one is its predecessor's end_cycle).
 __global__ void k_run_prologue(const __grid_constant__ Dom d, const int *max_cycles,
                                cudaGraphConditionalHandle handle, int *active)
 {
@@ -442,19 +450,8 @@ __global__ void k_run_prologue(const __grid_constant__ Dom d, const int *max_cyc
     const unsigned go = run_continue(d.sc, d.prm);
     *active = (int)go;
     if (handle) cudaGraphSetConditional(handle, go);
+    if (go) time_increment(d.sc, d.prm);
 }
-
-__global__ void k_run_epilogue(const __grid_constant__ Dom d, cudaGraphConditionalHandle handle,
-                               int *active)
-{
-    if (!*active) return;
-    finalize_constraints(d.sc);
-    d.sc->run_cycles++;
-    const unsigned go = run_continue(d.sc, d.prm);
-    *active = (int)go;
-    if (handle) cudaGraphSetConditional(handle, go);
-}
-
 
 // ---------------------------------------------------------------------
 // Launchers
@@ -477,7 +474,8 @@ static void launch_elem_force(const Dom &d, cudaStream_t st)
 static void launch_node_update(const Dom &d, cudaStream_t st)
 {
     if (d.df == kArithDF64) launch_node_update_df(d, st);
-    else k_node_update<<<blocks_for(d.nn, node_block(d)), node_block(d), 0, st>>>(d);
+    else if (d.nn < kEarlyNodes) k_node_update<true><<<blocks_for(d.nn, node_block(d)), node_block(d), 0, st>>>(d);
+    else k_node_update<false><<<blocks_for(d.nn, node_block(d)), node_block(d), 0, st>>>(d);
 }
 
 static void launch_elem_kinematics(const Dom &d, cudaStream_t st)
@@ -492,31 +490,30 @@ void launch_lagrange_nodal(const Dom &d, cudaStream_t st)
     launch_node_update(d, st);
 }
 
-void launch_lagrange_elements(const Dom &d, cudaStream_t st, bool with_constraints)
+// end null: without the constraints
+static void launch_elem_material(const Dom &d, cudaStream_t st, const CycleEnd *end)
+{
+    if (d.df == kArithDF64) launch_elem_material_df(d, st, end);
+    else if (end) k_elem_material<true><<<blocks_for(d.ne, elem_block(d)), elem_block(d), 0, st>>>(d);
+    else k_elem_material<false><<<blocks_for(d.ne, elem_block(d)), elem_block(d), 0, st>>>(d);
+}
+
+void launch_end_cycle(const Dom &d, cudaStream_t st, const CycleEnd &end)
+{
+    k_end_cycle<<<1, 1, 0, st>>>(d, end);
+}
+
+void launch_lagrange_elements(const Dom &d, cudaStream_t st, const CycleEnd *end)
 {
     launch_elem_kinematics(d, st);
-    if (d.df == kArithDF64)
-        launch_elem_material_df(d, st, with_constraints);
-    else if (with_constraints)
-        k_elem_material<true><<<blocks_for(d.ne, elem_block(d)), elem_block(d), 0, st>>>(d);
-    else
-        k_elem_material<false><<<blocks_for(d.ne, elem_block(d)), elem_block(d), 0, st>>>(d);
+    launch_elem_material(d, st, end);
+    if (end) launch_end_cycle(d, st, *end);
 }
 
 void launch_time_constraints(const Dom &d, cudaStream_t st)
 {
     k_time_constraints<<<blocks_for(d.ne, elem_block(d)), elem_block(d), 0, st>>>(d);
-    k_finalize<<<1, 1, 0, st>>>(d);
-}
-
-void launch_finalize(const Dom &d, cudaStream_t st)
-{
-    k_finalize<<<1, 1, 0, st>>>(d);
-}
-
-void launch_run_epilogue(const Dom &d, cudaStream_t st, cudaGraphConditionalHandle h, int *active)
-{
-    k_run_epilogue<<<1, 1, 0, st>>>(d, h, active);
+    launch_end_cycle(d, st, CycleEnd{});
 }
 
 void launch_run_prologue(const Dom &d, cudaStream_t st, const int *max_cycles,
@@ -525,23 +522,22 @@ void launch_run_prologue(const Dom &d, cudaStream_t st, const int *max_cycles,
     k_run_prologue<<<1, 1, 0, st>>>(d, max_cycles, h, active);
 }
 
-// One cycle of the run loop.  In the graph with a conditional while node
-// d.gate is null and the node stops the loop; in the host-driven fallback
-// d.gate == active and the cycles after the last one return at once.
+// One cycle of the run loop.  d.gate null: it runs; d.gate == active: it
+// returns at once when the run has ended.
 void launch_run_body(const Dom &d, cudaStream_t st, cudaGraphConditionalHandle h, int *active)
 {
-    k_time_increment<<<1, 1, 0, st>>>(d);
+    const CycleEnd end{h, active};
     launch_lagrange_nodal(d, st);
-    launch_lagrange_elements(d, st, true);
-    k_run_epilogue<<<1, 1, 0, st>>>(d, h, active);
+    launch_lagrange_elements(d, st, &end);
 }
 
-int kernels_per_cycle() { return 6; }
+int kernels_per_cycle() { return 5; }
 
 // Kernels of one cycle launched one by one, with an event recorded before
-// each (ev[0..6]); for per-kernel timing.
-void launch_cycle_timed(const Dom &d, cudaStream_t st, cudaEvent_t ev[7])
+// each (ev[0..5]); for per-kernel timing.
+void launch_cycle_timed(const Dom &d, cudaStream_t st, cudaEvent_t ev[kTimedKernels + 1])
 {
+    const CycleEnd end{};
     cudaEventRecord(ev[0], st);
     k_time_increment<<<1, 1, 0, st>>>(d);
     cudaEventRecord(ev[1], st);
@@ -551,10 +547,9 @@ void launch_cycle_timed(const Dom &d, cudaStream_t st, cudaEvent_t ev[7])
     cudaEventRecord(ev[3], st);
     launch_elem_kinematics(d, st);
     cudaEventRecord(ev[4], st);
-    if (d.df == kArithDF64) launch_elem_material_df(d, st, true);
-    else k_elem_material<true><<<blocks_for(d.ne, elem_block(d)), elem_block(d), 0, st>>>(d);
+    launch_elem_material(d, st, &end);
     cudaEventRecord(ev[5], st);
-    k_finalize<<<1, 1, 0, st>>>(d);
+    launch_end_cycle(d, st, end);
     cudaEventRecord(ev[6], st);
 }
 
@@ -674,21 +669,27 @@ void launch_batch_kernel_fp64(const Dom &d, const BatchView &b, cudaStream_t st,
     }
     switch (kernel) {
     case 0: kb_elem<elem_force_fp64><<<cfg.grid, cfg.block, 0, st>>>(d, b, cls); break;
-    case 1: kb_node<node_update_fp64><<<cfg.grid, cfg.block, 0, st>>>(d, b, cls); break;
+    case 1:
+        if (d.nn < kEarlyNodes) kb_node<node_update_fp64<true>><<<cfg.grid, cfg.block, 0, st>>>(d, b, cls);
+        else kb_node<node_update_fp64<false>><<<cfg.grid, cfg.block, 0, st>>>(d, b, cls);
+        break;
     case 2: kb_elem<elem_kinematics_fp64><<<cfg.grid, cfg.block, 0, st>>>(d, b, cls); break;
     default: kb_material<elem_material_fp64<true>><<<cfg.grid, cfg.block, 0, st>>>(d, b, cls); break;
     }
 }
 
 // Resident blocks per SM of a batched kernel at a block size.
-int batch_max_blocks_fp64(int kernel, int block, int arith)
+int batch_max_blocks_fp64(int kernel, int block, int arith, bool early)
 {
-    if (arith == kArithDF64) return batch_max_blocks_df(kernel, block);
+    if (arith == kArithDF64) return batch_max_blocks_df(kernel, block, early);
     int n = 0;
     cudaError_t e;
     switch (kernel) {
     case 0: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kb_elem<elem_force_fp64>, block, 0); break;
-    case 1: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kb_node<node_update_fp64>, block, 0); break;
+    case 1:
+        e = early ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kb_node<node_update_fp64<true>>, block, 0)
+                  : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kb_node<node_update_fp64<false>>, block, 0);
+        break;
     case 2: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kb_elem<elem_kinematics_fp64>, block, 0); break;
     default: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kb_material<elem_material_fp64<true>>, block, 0); break;
     }

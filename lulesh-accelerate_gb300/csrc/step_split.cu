@@ -375,9 +375,9 @@ __device__ __forceinline__ void kahan_add(float &s, float &c, float v)
     s = t;
 }
 
-// kEarly loads the node's state before its corners (load_node): on meshes
-// that leave most of an SM idle the update is its chain of memory latencies,
-// and this shortens it (a cycle of s=30 37.7 -> 36.9 us).  On large ones the
+// kEarly loads the node's state and all its corners before it uses any: on
+// meshes that leave most of an SM idle the update is its chain of memory
+// latencies, and this shortens it (a cycle of s=30 37.7 -> @C@ us).  On large ones the
 // registers that it holds through the gather cost more (s=192 0.31 -> 0.40
 // ms: 56 registers, or 40 with spills, instead of 32), and each component is
 // loaded where it is used.
@@ -387,11 +387,25 @@ __device__ __forceinline__ void node_update_split_from(const Dom &d, int n, cons
     NodeState s{};
     if (kEarly) s = load_node(d, n);
     float sx = 0.f, sy = 0.f, sz = 0.f, cx = 0.f, cy = 0.f, cz = 0.f;
-    for_node_corners(d, sc, n, [&](int c, bool) {
-        kahan_add(sx, cx, d.f32x[c]);
-        kahan_add(sy, cy, d.f32y[c]);
-        kahan_add(sz, cz, d.f32z[c]);
-    });
+    auto take = [&](float x, float y, float z) {
+        kahan_add(sx, cx, x);
+        kahan_add(sy, cy, y);
+        kahan_add(sz, cz, z);
+    };
+    if (kEarly) {
+        const CornerSlots at = corner_slots(d, sc, n);
+        float c[3][8];
+        load_corners<float>(at, d.f32x, d.f32y, d.f32z, c);
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+            if ((at.present >> j) & 1) take(c[0][j], c[1][j], c[2][j]);
+        for (int j = at.rest; j < at.end; ++j) {
+            const int i = __ldg(d.corner_list + j);
+            take(d.f32x[i], d.f32y[i], d.f32z[i]);
+        }
+    } else {
+        for_node_corners(d, sc, n, [&](int c, bool) { take(d.f32x[c], d.f32y[c], d.f32z[c]); });
+    }
     const double fx = f2d(sx) - f2d(cx);
     const double fy = f2d(sy) - f2d(cy);
     const double fz = f2d(sz) - f2d(cz);
@@ -416,11 +430,6 @@ __device__ __forceinline__ void node_update_split_from(const Dom &d, int n, cons
     move(fy, 2, d.yd, d.y, d.yds, d.ys, s.yd, s.y);
     move(fz, 4, d.zd, d.z, d.zds, d.zs, s.zd, s.z);
 }
-__device__ __forceinline__ void node_update_split(const Dom &d, int n, const DevScalars *sc)
-{
-    node_update_split_from<false>(d, n, sc);
-}
-
 template <bool kEarly>
 __global__ void __launch_bounds__(kBlockNode) k_node_update_split(const __grid_constant__ Dom d)
 {
@@ -600,12 +609,10 @@ void launch_split_sync(const Dom &d, cudaStream_t st)
     k_split_sync<<<blocks_for(d.nn, node_block(d)), node_block(d), 0, st>>>(d);
 }
 
-// (a mesh whose blocks choose_blocks has cut is one that does not fill the
-// SMs)
 static void launch_node_update_split(const Dom &d, cudaStream_t st)
 {
     const unsigned grid = blocks_for(d.nn, node_block(d));
-    if (node_block(d) < kBlockNode) k_node_update_split<true><<<grid, node_block(d), 0, st>>>(d);
+    if (d.nn < kEarlyNodes) k_node_update_split<true><<<grid, node_block(d), 0, st>>>(d);
     else k_node_update_split<false><<<grid, node_block(d), 0, st>>>(d);
 }
 
@@ -615,25 +622,29 @@ void launch_lagrange_nodal_split(const Dom &d, cudaStream_t st)
     launch_node_update_split(d, st);
 }
 
-void launch_lagrange_elements_split(const Dom &d, cudaStream_t st, bool with_constraints)
+static void launch_elem_material_split(const Dom &d, cudaStream_t st, const CycleEnd *end)
+{
+    if (end) k_elem_material_split<true><<<blocks_for(d.ne, elem_block(d)), elem_block(d), 0, st>>>(d);
+    else k_elem_material_split<false><<<blocks_for(d.ne, elem_block(d)), elem_block(d), 0, st>>>(d);
+}
+
+void launch_lagrange_elements_split(const Dom &d, cudaStream_t st, const CycleEnd *end)
 {
     k_elem_kinematics_split<<<blocks_for(d.ne, kin_block(d)), kin_block(d), 0, st>>>(d);
-    if (with_constraints)
-        k_elem_material_split<true><<<blocks_for(d.ne, elem_block(d)), elem_block(d), 0, st>>>(d);
-    else
-        k_elem_material_split<false><<<blocks_for(d.ne, elem_block(d)), elem_block(d), 0, st>>>(d);
+    launch_elem_material_split(d, st, end);
+    if (end) launch_end_cycle(d, st, *end);
 }
 
 void launch_run_body_split(const Dom &d, cudaStream_t st, cudaGraphConditionalHandle h, int *active)
 {
-    launch_time_increment(d, st);
+    const CycleEnd end{h, active};
     launch_lagrange_nodal_split(d, st);
-    launch_lagrange_elements_split(d, st, true);
-    launch_run_epilogue(d, st, h, active);
+    launch_lagrange_elements_split(d, st, &end);
 }
 
 void launch_cycle_timed_split(const Dom &d, cudaStream_t st, cudaEvent_t ev[kTimedKernels + 1])
 {
+    const CycleEnd end{};
     cudaEventRecord(ev[0], st);
     launch_time_increment(d, st);
     cudaEventRecord(ev[1], st);
@@ -643,9 +654,9 @@ void launch_cycle_timed_split(const Dom &d, cudaStream_t st, cudaEvent_t ev[kTim
     cudaEventRecord(ev[3], st);
     k_elem_kinematics_split<<<blocks_for(d.ne, kin_block(d)), kin_block(d), 0, st>>>(d);
     cudaEventRecord(ev[4], st);
-    k_elem_material_split<true><<<blocks_for(d.ne, elem_block(d)), elem_block(d), 0, st>>>(d);
+    launch_elem_material_split(d, st, &end);
     cudaEventRecord(ev[5], st);
-    launch_finalize(d, st);
+    launch_end_cycle(d, st, end);
     cudaEventRecord(ev[6], st);
 }
 
@@ -657,7 +668,10 @@ void launch_batch_kernel_split(const Dom &d, const BatchView &b, cudaStream_t st
 {
     switch (kernel) {
     case 0: kb_elem<elem_force_split><<<cfg.grid, cfg.block, 0, st>>>(d, b, cls); break;
-    case 1: kb_node<node_update_split><<<cfg.grid, cfg.block, 0, st>>>(d, b, cls); break;
+    case 1:
+        if (d.nn < kEarlyNodes) kb_node<node_update_split_from<true>><<<cfg.grid, cfg.block, 0, st>>>(d, b, cls);
+        else kb_node<node_update_split_from<false>><<<cfg.grid, cfg.block, 0, st>>>(d, b, cls);
+        break;
     case 2: kb_elem_capped<elem_kinematics_split, 2><<<cfg.grid, cfg.block, 0, st>>>(d, b, cls); break;
     default: kb_material_capped<elem_material_split<true>, 4><<<cfg.grid, cfg.block, 0, st>>>(d, b, cls); break;
     }
@@ -682,13 +696,16 @@ int batch_max_blocks_split_staged(int rows)
 }
 
 // Resident blocks per SM of a batched kernel at a block size.
-int batch_max_blocks_split(int kernel, int block)
+int batch_max_blocks_split(int kernel, int block, bool early)
 {
     int n = 0;
     cudaError_t e;
     switch (kernel) {
     case 0: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kb_elem<elem_force_split>, block, 0); break;
-    case 1: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kb_node<node_update_split>, block, 0); break;
+    case 1:
+        e = early ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kb_node<node_update_split_from<true>>, block, 0)
+                  : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kb_node<node_update_split_from<false>>, block, 0);
+        break;
     case 2: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kb_elem_capped<elem_kinematics_split, 2>, block, 0); break;
     default: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kb_material_capped<elem_material_split<true>, 4>, block, 0); break;
     }
