@@ -384,10 +384,11 @@ int lulesh_batch_get_field(lulesh_batch *b, int i, const char *name, double *hos
  * or lulesh_batch_run_retuned call. */
 int lulesh_batch_zone_cycles(lulesh_batch *b, double *zone_cycles);
 
-/* Choose threads per block (64/128/256, i.e. 4/2/1 elements per thread of a
- * 256-element tile) and resident blocks per SM (1/2/4/8 and the most that
- * fit) of each step kernel per size class by timing the candidates on this
- * batch, whose state is restored afterwards; in split precision, for a
+/* Choose threads per block (64/128/256; a 256-element tile is dealt out that
+ * many elements at a time, one per thread) and blocks per SM (1/2/4/8, the
+ * most that fit, and four waves of those) of each step kernel per size class
+ * by timing the candidates on this batch, whose state is restored
+ * afterwards; in split precision, for a
  * class whose instances are all cubes with s >= 64, also the staging depth
  * of the force kernel: its corners gathered from global memory (0), or
  * tiles of 2 or 4 element rows x 64 columns staged in shared memory (blocks

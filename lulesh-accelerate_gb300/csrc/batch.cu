@@ -10,17 +10,16 @@
 // block they read and write (time step, error words, constraint minima) is
 // the instance's own.
 //
-// Execution.  One cycle is: a per-instance TimeIncrement; the four step
-// kernels, each a persistent kernel per size class walking that class's list
-// of active tiles (each class's chain of four is one parallel graph branch);
-// a per-instance epilogue that publishes the constraint minima, counts the
-// cycle and retires instances that reached their stop time; and a compaction
-// of the active-tile lists when an instance retired.  The whole run is one
+// Execution.  One cycle is: the four step kernels, each a persistent kernel
+// per size class walking that class's list of active tiles (each class's
+// chain of four is one parallel graph branch); and a per-instance epilogue
+// that publishes the constraint minima, counts the cycle, does the next
+// TimeIncrement or retires an instance that reached its stop time, and
+// rebuilds the active-tile lists when one retired.  The whole run is one
 // CUDA graph with a conditional WHILE node that loops while any instance is
 // active -- no host synchronisation per cycle.
 //
-// Launch shapes (threads per block = kTile / elements per thread, resident
-// blocks per SM of the persistent grid, and for the split force kernel of a
+// Launch shapes (threads per block, blocks per SM, and for the split force kernel of a
 // class of structured cubes the staging depth: gathered corners, or tiles of
 // two or four element rows staged in shared memory) are chosen per size
 // class and kernel by lulesh_batch_autotune, which times the candidates on
@@ -132,17 +131,33 @@ __global__ void kb_geo_invalidate(DevScalars *sc, int n)
     if (i < n) sc[i].geo_valid = 0;
 }
 
-__global__ void kb_time_increment(const __grid_constant__ Dom d, const __grid_constant__ BatchView b)
+// Rebuild the active-tile lists, by one block.  The order inside a list does
+// not matter: every tile's work is independent and the constraint reduction
+// is an order-free minimum.
+__device__ void rebuild_lists(const BatchView &b)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= b.n_inst || !b.inst_active[i]) return;
-    DevScalars *sc = d.sc + i;
-    if (sc->err_any) return;
-    time_increment(sc, d.prm);
+    __shared__ int n[2 * kMaxClasses];
+    __syncthreads();   // inst_active is complete, and the previous use of n over
+    if (threadIdx.x < 2 * kMaxClasses) n[threadIdx.x] = 0;
+    __syncthreads();
+    for (int t = threadIdx.x; t < b.n_etiles; t += blockDim.x) {
+        const int i = b.etile_inst[t];
+        if (!b.inst_active[i]) continue;
+        const int c = b.etile_class[t], slot = atomicAdd(&n[c], 1);
+        b.active_etiles[b.eclass_off[c] + slot] = {t * kTile, min(b.inst_elem_end[i], (t + 1) * kTile), i, t};
+    }
+    for (int t = threadIdx.x; t < b.n_ntiles; t += blockDim.x) {
+        const int i = b.ntile_inst[t];
+        if (!b.inst_active[i]) continue;
+        const int c = b.ntile_class[t], slot = atomicAdd(&n[kMaxClasses + c], 1);
+        b.active_ntiles[b.nclass_off[c] + slot] = {t * kTile, min(b.inst_node_end[i], (t + 1) * kTile), i, t};
+    }
+    __syncthreads();
+    if (threadIdx.x < 2 * kMaxClasses) b.counts[threadIdx.x] = n[threadIdx.x];
 }
 
 // One block: reset the per-instance run counters, decide which instances
-// run at all, ask for a full rebuild of the active-tile lists.
+// run at all and do their first TimeIncrement, and list their tiles.
 __global__ void kb_prologue(const __grid_constant__ Dom d, const __grid_constant__ BatchView b,
                             const int *max_cycles, cudaGraphConditionalHandle h)
 {
@@ -155,20 +170,21 @@ __global__ void kb_prologue(const __grid_constant__ Dom d, const __grid_constant
         sc->run_max = *max_cycles;
         const unsigned go = run_continue(sc, d.prm);
         b.inst_active[i] = (unsigned char)go;
-        if (go) any = 1;
+        if (go) {
+            any = 1;
+            time_increment(sc, d.prm);
+        }
     }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int c = 0; c < 2 * kMaxClasses; ++c) b.counts[c] = 0;
-        b.counts[2 * kMaxClasses] = 1;
-        b.counts[2 * kMaxClasses + 1] = any;
-        if (h) cudaGraphSetConditional(h, any);
-    }
+    rebuild_lists(b);
+    if (threadIdx.x == 0 && h) cudaGraphSetConditional(h, any);
 }
 
-// One block: publish each running instance's constraint minima, count its
-// cycle, retire it when it reached its stop time (or failed), and set the
-// loop condition.
+// One block, at the end of a cycle: publish each running instance's
+// constraint minima, count its cycle and do its next TimeIncrement, or retire
+// it when it reached its stop time (or failed); rebuild the tile lists when
+// one retired; set the loop condition.  As four kernels (the time increment
+// and the compaction, over all tiles, their own) this was more than a third
+// of a small ensemble's launches.
 __global__ void kb_epilogue(const __grid_constant__ Dom d, const __grid_constant__ BatchView b,
                             cudaGraphConditionalHandle h)
 {
@@ -185,38 +201,15 @@ __global__ void kb_epilogue(const __grid_constant__ Dom d, const __grid_constant
         sc->run_cycles++;
         if (run_continue(sc, d.prm)) {
             any = 1;
+            time_increment(sc, d.prm);
         } else {
             b.inst_active[i] = 0;
             changed = 1;
         }
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        if (changed)
-            for (int c = 0; c < 2 * kMaxClasses; ++c) b.counts[c] = 0;
-        b.counts[2 * kMaxClasses] = changed;
-        b.counts[2 * kMaxClasses + 1] = any;
-        if (h) cudaGraphSetConditional(h, any);
-    }
-}
-
-// Rebuild the active-tile lists (only after an instance retired).  The
-// order inside a list does not matter: every tile's work is independent and
-// the constraint reduction is an order-free minimum.
-__global__ void kb_compact(const __grid_constant__ BatchView b)
-{
-    if (!b.counts[2 * kMaxClasses]) return;
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t < b.n_etiles && b.inst_active[b.etile_inst[t]]) {
-        const int c = b.etile_class[t];
-        const int slot = atomicAdd(&b.counts[c], 1);
-        b.active_etiles[b.eclass_off[c] + slot] = t;
-    }
-    if (t < b.n_ntiles && b.inst_active[b.ntile_inst[t]]) {
-        const int c = b.ntile_class[t];
-        const int slot = atomicAdd(&b.counts[kMaxClasses + c], 1);
-        b.active_ntiles[b.nclass_off[c] + slot] = t;
-    }
+    if (changed) rebuild_lists(b);
+    if (threadIdx.x == 0 && h) cudaGraphSetConditional(h, any);
 }
 
 // ---- host helpers ------------------------------------------------------
@@ -254,11 +247,9 @@ int max_blocks(lulesh_batch *b, int kernel, int block)
                                                   : batch_max_blocks_fp64(kernel, block, b->dom.df, early);
 }
 
-unsigned compact_blocks(const lulesh_batch *b)
-{
-    const long t = std::max(b->bv.n_etiles, b->bv.n_ntiles);
-    return (unsigned)((t + 255) / 256);
-}
+// Threads of the control kernels' one block: the instances and, when one
+// retires, the tiles are walked with this stride.
+unsigned control_threads(const lulesh_batch *b) { return b->n <= 32 && b->bv.n_etiles <= 1024 ? 256 : 1024; }
 
 // One cycle on b->stream; each size class runs its four kernels as one
 // parallel branch (fork/join through events, which stream capture turns into
@@ -266,7 +257,6 @@ unsigned compact_blocks(const lulesh_batch *b)
 void launch_cycle(lulesh_batch *b, cudaGraphConditionalHandle h)
 {
     cudaStream_t st = b->stream;
-    kb_time_increment<<<(b->n + 127) / 128, 128, 0, st>>>(b->dom, b->bv);
     // Instances never interact, so each size class runs its whole chain of
     // four phases on its own branch: a class that finishes a phase goes on
     // to its next one while the others are still busy, instead of waiting
@@ -289,13 +279,17 @@ void launch_cycle(lulesh_batch *b, cudaGraphConditionalHandle h)
             cudaStreamWaitEvent(st, b->ev_join[c], 0);
         }
     }
-    kb_epilogue<<<1, 1024, 0, st>>>(b->dom, b->bv, h);
-    kb_compact<<<compact_blocks(b), 256, 0, st>>>(b->bv);
+    kb_epilogue<<<1, control_threads(b), 0, st>>>(b->dom, b->bv, h);
 }
+
+// Cycles per pass of the while node: several where a cycle is short of the
+// node's own turn-round (lulesh_run's rule); after the last instance has
+// retired the lists are empty and a cycle's kernels return at once.
+int body_cycles(const lulesh_batch *b) { return b->ne_tot <= 150000 ? 4 : 1; }
 
 int count_kernels_per_cycle(const lulesh_batch *b)
 {
-    int n = 3;   // time increment, epilogue, compaction
+    int n = 1;   // epilogue
     for (int k = 0; k < kBatchKernels; ++k)
         for (int c = 0; c < kMaxClasses; ++c) n += (k == 1 ? b->class_ntiles[c] : b->class_etiles[c]) > 0;
     return n;
@@ -317,11 +311,10 @@ int build_graph(lulesh_batch *b)
     if (e == cudaSuccess) e = cudaStreamBeginCaptureToGraph(b->stream, g, nullptr, nullptr, 0,
                                                              cudaStreamCaptureModeThreadLocal);
     if (e == cudaSuccess) {
-        kb_prologue<<<1, 1024, 0, b->stream>>>(b->dom, b->bv, b->d_max, h);
-        kb_compact<<<compact_blocks(b), 256, 0, b->stream>>>(b->bv);
+        kb_prologue<<<1, control_threads(b), 0, b->stream>>>(b->dom, b->bv, b->d_max, h);
         e = cudaStreamEndCapture(b->stream, &g);
     }
-    // the last node of the prologue part is the compaction
+    // the prologue's node
     cudaGraphNode_t tail = nullptr;
     if (e == cudaSuccess) {
         size_t nn = 0;
@@ -344,7 +337,7 @@ int build_graph(lulesh_batch *b)
         cudaGraph_t body = cp.conditional.phGraph_out[0];
         e = cudaStreamBeginCaptureToGraph(b->stream, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
         if (e == cudaSuccess) {
-            launch_cycle(b, h);
+            for (int i = 0; i < body_cycles(b); ++i) launch_cycle(b, h);
             cudaGraph_t out = nullptr;
             e = cudaStreamEndCapture(b->stream, &out);
         }
@@ -359,13 +352,27 @@ int build_graph(lulesh_batch *b)
     return LULESH_OK;
 }
 
+// Blocks of a kernel that walks a class's tiles: one per share of a tile, at
+// most per_sm on every SM.
+int grid_for(const lulesh_batch *b, int cls, int kernel, int block, int per_sm)
+{
+    const long tiles = kernel == 1 ? b->class_ntiles[cls] : b->class_etiles[cls];
+    return (int)std::max(1L, std::min(tiles * ((kTile + block - 1) / block), (long)b->sms * per_sm));
+}
+
+// Waves of resident blocks in a default launch: more than one, so that the
+// blocks balance over the SMs as they finish, but not a block for every share,
+// most of which would find nothing once instances have retired (eight FP64
+// instances of 16..56: 289 us a cycle with two waves, 280 with four, 283 with
+// eight).
+constexpr int kDefaultWaves = 4;
+
 void default_cfg(lulesh_batch *b)
 {
     for (int c = 0; c < kMaxClasses; ++c)
         for (int k = 0; k < kBatchKernels; ++k) {
-            const int tiles = k == 1 ? b->class_ntiles[c] : b->class_etiles[c];
             const int per_sm = std::max(1, max_blocks(b, k, 128));
-            b->cfg[c][k] = {128, std::max(1, std::min(tiles, b->sms * per_sm))};
+            b->cfg[c][k] = {128, grid_for(b, c, k, 128, kDefaultWaves * per_sm)};
         }
 }
 
@@ -562,10 +569,10 @@ int lulesh_batch_create(int n, const int *sizes, const double *e0_scale, int ini
     }
     A(d.inv_mass, nn); A(d.inv_volo, ne);
     A(d.sc, (size_t)n); A(b->d_max, 1);
-    int *etile_inst_d, *ntile_inst_d, *etile_class_d, *ntile_class_d, *iee, *ine, *eco, *nco;
+    int *etile_inst_d, *ntile_inst_d, *etile_class_d, *ntile_class_d, *iee, *ine;
     A(etile_inst_d, net); A(ntile_inst_d, nnt); A(etile_class_d, net); A(ntile_class_d, nnt);
-    A(iee, n); A(ine, n); A(eco, kMaxClasses); A(nco, kMaxClasses);
-    A(b->bv.active_etiles, net); A(b->bv.active_ntiles, nnt); A(b->bv.counts, 2 * kMaxClasses + 2);
+    A(iee, n); A(ine, n);
+    A(b->bv.active_etiles, net); A(b->bv.active_ntiles, nnt); A(b->bv.counts, 2 * kMaxClasses);
     A(b->bv.inst_active, n);
     d.nodelist = nodelist; d.corner_start = cstart; d.corner_list = clist; d.node_bc = nbc;
     d.lxim = lxim; d.lxip = lxip; d.letam = letam; d.letap = letap; d.lzetam = lzetam; d.lzetap = lzetap;
@@ -581,7 +588,10 @@ int lulesh_batch_create(int n, const int *sizes, const double *e0_scale, int ini
     bv.etile_inst = etile_inst_d; bv.ntile_inst = ntile_inst_d;
     bv.etile_class = etile_class_d; bv.ntile_class = ntile_class_d;
     bv.inst_elem_end = iee; bv.inst_node_end = ine;
-    bv.eclass_off = eco; bv.nclass_off = nco;
+    for (int c = 0; c < kMaxClasses; ++c) {
+        bv.eclass_off[c] = eclass_off[c];
+        bv.nclass_off[c] = nclass_off[c];
+    }
 
     // host images of the flat arrays, instance by instance
     cudaStream_t st = b->stream;
@@ -657,8 +667,6 @@ int lulesh_batch_create(int n, const int *sizes, const double *e0_scale, int ini
     up(ntile_class_d, ntile_class.data(), nnt * 4);
     up(iee, iee_h.data(), n * 4);
     up(ine, ine_h.data(), n * 4);
-    up(eco, eclass_off, sizeof eclass_off);
-    up(nco, nclass_off, sizeof nclass_off);
     // padding entries of the mass arrays are read by whole-array kernels
     // (the split path's reciprocal masses): give them unit values
     {
@@ -681,7 +689,7 @@ int lulesh_batch_create(int n, const int *sizes, const double *e0_scale, int ini
     for (double *f : {d.p, d.q, d.ss, d.vnew, d.delv, d.vdov, d.arealg, d.delv_xi, d.delv_eta, d.delv_zeta,
                       d.delx_xi, d.delx_eta, d.delx_zeta})
         ok = ok && cudaMemsetAsync(f, 0, ne * 8, st) == cudaSuccess;
-    ok = ok && cudaMemsetAsync(b->bv.counts, 0, (2 * kMaxClasses + 2) * 4, st) == cudaSuccess;
+    ok = ok && cudaMemsetAsync(b->bv.counts, 0, 2 * kMaxClasses * 4, st) == cudaSuccess;
     if (ok && precision == LULESH_PRECISION_SPLIT) {
         launch_split_sync(d, st);
         ok = cudaGetLastError() == cudaSuccess;
@@ -754,9 +762,8 @@ int lulesh_batch_run(lulesh_batch *b, int max_cycles, int *cycles_done)
         b->last_zc += (double)b->ne_i[i] * b->h_sc[i].run_cycles;
     }
     if (cycles_done) *cycles_done = most;
-    // time increment, epilogue and compaction run every cycle; each step
-    // kernel once per class per cycle
-    b->launches += 2 + (long long)most * b->kernels_per_cycle;
+    // the epilogue and each class's step kernels run every cycle
+    b->launches += 1 + (long long)most * b->kernels_per_cycle;
     (void)total;
     // an instance that stopped short of its stop time without an error and
     // without reaching the caller's cap ran out of cycle budget (or of
@@ -911,7 +918,6 @@ int lulesh_batch_set_tuning(lulesh_batch *b, int cls, int kernel, int block, int
 {
     if (!b || cls < 0 || cls >= kMaxClasses || kernel < 0 || kernel >= kBatchKernels || blocks_per_sm < 1)
         return bfail(b, LULESH_ERR_ARG, "lulesh_batch_set_tuning: bad arguments");
-    const int tiles = kernel == 1 ? b->class_ntiles[cls] : b->class_etiles[cls];
     if (rows != 0) {
         if (kernel != 0 || (rows != 2 && rows != 4) || !can_stage(b, cls))
             return bfail(b, LULESH_ERR_ARG, "lulesh_batch_set_tuning: this class's kernel cannot be staged that deep");
@@ -924,7 +930,7 @@ int lulesh_batch_set_tuning(lulesh_batch *b, int cls, int kernel, int block, int
         const int fit = max_blocks(b, kernel, block);
         if (fit < 1) return bfail(b, LULESH_ERR_ARG, "lulesh_batch_set_tuning: no block of that size fits on an SM");
         const int per_sm = std::min(blocks_per_sm, fit);
-        b->cfg[cls][kernel] = {block, std::max(1, std::min(std::max(tiles, 1), b->sms * per_sm))};
+        b->cfg[cls][kernel] = {block, grid_for(b, cls, kernel, block, per_sm)};
     }
     destroy_graph(b);   // the run graph bakes in the launch shapes
     return LULESH_OK;
@@ -949,8 +955,8 @@ int lulesh_batch_autotune(lulesh_batch *b, const char *cache_path, int retune)
                                 (int)std::max(1LL, std::min(staged_tiles(b, c, te.stage), (long long)b->sms * per_sm)),
                                 te.stage};
             } else {
-                const int per_sm = std::max(1, std::min(te.per_sm, max_blocks(b, k, te.block)));
-                b->cfg[c][k] = {te.block, std::max(1, std::min(tiles, b->sms * per_sm))};
+                const int per_sm = std::max(1, std::min(te.per_sm, kDefaultWaves * max_blocks(b, k, te.block)));
+                b->cfg[c][k] = {te.block, grid_for(b, c, k, te.block, per_sm)};
             }
         }
     if (need) {
@@ -973,11 +979,24 @@ int lulesh_batch_autotune(lulesh_batch *b, const char *cache_path, int retune)
         snap.push_back(ssnap);
         cudaMemcpyAsync(ssnap, d.sc, sizeof(DevScalars) * b->n, cudaMemcpyDeviceToDevice, b->stream);
 
+        // Every candidate runs the real kernel on the batch's own state; the
+        // state comes back before each kernel's candidates, since a node
+        // update repeated with the same forces would carry the mesh away (and
+        // a failed instance's elements are skipped: nothing left to time).
+        auto restore = [&]() {
+            for (int j = 0; j < 11; ++j)
+                cudaMemcpyAsync(j < 6 ? node_f[j] : elem_f[j - 6], snap[j], (j < 6 ? nn : ne) * sizeof(double),
+                                cudaMemcpyDeviceToDevice, b->stream);
+            cudaMemcpyAsync(d.sc, ssnap, sizeof(DevScalars) * b->n, cudaMemcpyDeviceToDevice, b->stream);
+            // the tuning runs rewrote the geometry cache from positions that
+            // are now restored: mark it stale
+            kb_geo_invalidate<<<(b->n + 127) / 128, 128, 0, b->stream>>>(d.sc, b->n);
+            if (b->precision == LULESH_PRECISION_SPLIT) launch_split_sync(b->dom, b->stream);
+        };
         // active lists for the current state
         b->h_stage[0] = 0;
         cudaMemcpyAsync(b->d_max, b->h_stage, sizeof(int), cudaMemcpyHostToDevice, b->stream);
-        kb_prologue<<<1, 1024, 0, b->stream>>>(b->dom, b->bv, b->d_max, 0);
-        kb_compact<<<compact_blocks(b), 256, 0, b->stream>>>(b->bv);
+        kb_prologue<<<1, control_threads(b), 0, b->stream>>>(b->dom, b->bv, b->d_max, 0);
         cudaEvent_t e0, e1;
         cudaEventCreate(&e0);
         cudaEventCreate(&e1);
@@ -987,6 +1006,7 @@ int lulesh_batch_autotune(lulesh_batch *b, const char *cache_path, int retune)
             for (int k = 0; k < kBatchKernels; ++k) {
                 const int tiles = k == 1 ? b->class_ntiles[c] : b->class_etiles[c];
                 if (!tiles) continue;
+                restore();
                 float best = 1e30f;
                 LaunchCfg best_cfg = b->cfg[c][k];
                 int best_depth = 1;
@@ -1008,25 +1028,27 @@ int lulesh_batch_autotune(lulesh_batch *b, const char *cache_path, int retune)
                         best_depth = dp;
                     }
                 };
-                // resident blocks per SM: 1, 2, 4, 8 and the most that fit
-                // (three 128-thread blocks of the 168-register force body,
-                // for instance, which no power of two reaches)
-                auto per_sm_candidates = [&](int cap) {
+                // blocks per SM: 1, 2, 4, 8 and the most that fit (three
+                // 128-thread blocks of the 168-register force body, for
+                // instance, which no power of two reaches), resident
+                // throughout, or a few waves of the most that fit
+                auto per_sm_candidates = [&](int cap, int waves) {
                     std::vector<int> v;
                     for (int dp : depths)
                         if (dp <= cap) v.push_back(dp);
                     if (cap >= 1 && std::find(v.begin(), v.end(), cap) == v.end()) v.push_back(cap);
+                    if (cap >= 1 && waves > 1) v.push_back(waves * cap);
                     return v;
                 };
                 for (int bs : blocks)
-                    for (int dp : per_sm_candidates(max_blocks(b, k, bs)))
-                        try_cfg({bs, std::max(1, std::min(tiles, b->sms * dp))}, dp);
+                    for (int dp : per_sm_candidates(max_blocks(b, k, bs), kDefaultWaves))
+                        try_cfg({bs, grid_for(b, c, k, bs, dp)}, dp);
                 // the split force kernel of a class of structured cubes: the
                 // staged tiles, two or four element rows deep
                 if (k == 0 && can_stage(b, c))
                     for (int rows : kStageRows) {
                         const long long st_tiles = staged_tiles(b, c, rows);
-                        for (int dp : per_sm_candidates(batch_max_blocks_split_staged(rows)))
+                        for (int dp : per_sm_candidates(batch_max_blocks_split_staged(rows), 1))
                             try_cfg({rows * kTileCols, (int)std::max(1LL, std::min(st_tiles, (long long)b->sms * dp)), rows},
                                     dp);
                     }
@@ -1035,15 +1057,7 @@ int lulesh_batch_autotune(lulesh_batch *b, const char *cache_path, int retune)
             }
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);
-        // restore
-        for (int j = 0; j < 11; ++j)
-            cudaMemcpyAsync(j < 6 ? node_f[j] : elem_f[j - 6], snap[j], (j < 6 ? nn : ne) * sizeof(double),
-                            cudaMemcpyDeviceToDevice, b->stream);
-        cudaMemcpyAsync(d.sc, ssnap, sizeof(DevScalars) * b->n, cudaMemcpyDeviceToDevice, b->stream);
-        // the tuning runs rewrote the geometry cache from positions that are
-        // now restored: mark it stale
-        kb_geo_invalidate<<<(b->n + 127) / 128, 128, 0, b->stream>>>(d.sc, b->n);
-        if (b->precision == LULESH_PRECISION_SPLIT) launch_split_sync(b->dom, b->stream);
+        restore();
         cudaError_t e = cudaStreamSynchronize(b->stream);
         cleanup();
         if (e != cudaSuccess) return bfail(b, LULESH_ERR_CUDA, std::string("autotune: ") + cudaGetErrorString(e));

@@ -184,16 +184,20 @@ constexpr int kTile = 256;
 constexpr int kMaxClasses = 3;
 constexpr int kBatchKernels = 4;   // force, node update, kinematics, material
 
+// A tile that a running instance still needs: its first element (or node),
+// one past the last of them, the instance.
+struct ActiveTile {
+    int begin, end, inst, tile;
+};
 struct BatchView {
     int n_inst, n_classes, n_etiles, n_ntiles;
     const int *etile_inst, *ntile_inst;          // instance of each tile
     const int *etile_class, *ntile_class;        // size class of each tile
     const int *inst_elem_end, *inst_node_end;    // one past the instance's last element / node
-    const int *eclass_off, *nclass_off;          // start of each class's active list
-    int *active_etiles, *active_ntiles;          // active tiles, grouped by class
+    int eclass_off[kMaxClasses], nclass_off[kMaxClasses];   // start of each class's active list
+    ActiveTile *active_etiles, *active_ntiles;   // active tiles, grouped by class
     // counts[c] / counts[kMaxClasses + c]: active element / node tiles of
-    // class c; counts[2*kMaxClasses]: rebuild the lists; [2*kMaxClasses+1]:
-    // instances still running
+    // class c
     int *counts;
     unsigned char *inst_active;
 };

@@ -634,12 +634,12 @@ void launch_elem_material_df(const Dom &d, cudaStream_t st, const CycleEnd *end)
 void launch_batch_kernel_df(const Dom &d, const BatchView &b, cudaStream_t st, int kernel, int cls, LaunchCfg cfg)
 {
     switch (kernel) {
-    case 0: kb_elem<elem_force_df><<<cfg.grid, cfg.block, 0, st>>>(d, b, cls); break;
+    case 0: kb_elem<elem_force_df, 168><<<cfg.grid, cfg.block, 0, st>>>(d, b, cls); break;
     case 1:
-        if (d.nn < kEarlyNodes) kb_node<node_update_df<true>><<<cfg.grid, cfg.block, 0, st>>>(d, b, cls);
-        else kb_node<node_update_df<false>><<<cfg.grid, cfg.block, 0, st>>>(d, b, cls);
+        if (d.nn < kEarlyNodes) kb_node<node_update_df<true>, 128><<<cfg.grid, cfg.block, 0, st>>>(d, b, cls);
+        else kb_node<node_update_df<false>, 64><<<cfg.grid, cfg.block, 0, st>>>(d, b, cls);
         break;
-    case 2: kb_elem<elem_kinematics_df><<<cfg.grid, cfg.block, 0, st>>>(d, b, cls); break;
+    case 2: kb_elem<elem_kinematics_df, 128><<<cfg.grid, cfg.block, 0, st>>>(d, b, cls); break;
     default: kb_material_capped<elem_material_df<true>, 4><<<cfg.grid, cfg.block, 0, st>>>(d, b, cls); break;
     }
 }
@@ -649,12 +649,12 @@ int batch_max_blocks_df(int kernel, int block, bool early)
     int n = 0;
     cudaError_t e;
     switch (kernel) {
-    case 0: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kb_elem<elem_force_df>, block, 0); break;
+    case 0: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kb_elem<elem_force_df, 168>, block, 0); break;
     case 1:
-        e = early ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kb_node<node_update_df<true>>, block, 0)
-                  : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kb_node<node_update_df<false>>, block, 0);
+        e = early ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kb_node<node_update_df<true>, 128>, block, 0)
+                  : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kb_node<node_update_df<false>, 64>, block, 0);
         break;
-    case 2: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kb_elem<elem_kinematics_df>, block, 0); break;
+    case 2: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kb_elem<elem_kinematics_df, 128>, block, 0); break;
     default: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kb_material_capped<elem_material_df<true>, 4>, block, 0); break;
     }
     return e == cudaSuccess ? n : 0;

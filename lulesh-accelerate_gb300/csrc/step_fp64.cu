@@ -668,12 +668,12 @@ void launch_batch_kernel_fp64(const Dom &d, const BatchView &b, cudaStream_t st,
         return;
     }
     switch (kernel) {
-    case 0: kb_elem<elem_force_fp64><<<cfg.grid, cfg.block, 0, st>>>(d, b, cls); break;
+    case 0: kb_elem<elem_force_fp64, 128><<<cfg.grid, cfg.block, 0, st>>>(d, b, cls); break;
     case 1:
-        if (d.nn < kEarlyNodes) kb_node<node_update_fp64<true>><<<cfg.grid, cfg.block, 0, st>>>(d, b, cls);
-        else kb_node<node_update_fp64<false>><<<cfg.grid, cfg.block, 0, st>>>(d, b, cls);
+        if (d.nn < kEarlyNodes) kb_node<node_update_fp64<true>, 128><<<cfg.grid, cfg.block, 0, st>>>(d, b, cls);
+        else kb_node<node_update_fp64<false>, 56><<<cfg.grid, cfg.block, 0, st>>>(d, b, cls);
         break;
-    case 2: kb_elem<elem_kinematics_fp64><<<cfg.grid, cfg.block, 0, st>>>(d, b, cls); break;
+    case 2: kb_elem<elem_kinematics_fp64, 128><<<cfg.grid, cfg.block, 0, st>>>(d, b, cls); break;
     default: kb_material<elem_material_fp64<true>><<<cfg.grid, cfg.block, 0, st>>>(d, b, cls); break;
     }
 }
@@ -685,12 +685,12 @@ int batch_max_blocks_fp64(int kernel, int block, int arith, bool early)
     int n = 0;
     cudaError_t e;
     switch (kernel) {
-    case 0: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kb_elem<elem_force_fp64>, block, 0); break;
+    case 0: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kb_elem<elem_force_fp64, 128>, block, 0); break;
     case 1:
-        e = early ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kb_node<node_update_fp64<true>>, block, 0)
-                  : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kb_node<node_update_fp64<false>>, block, 0);
+        e = early ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kb_node<node_update_fp64<true>, 128>, block, 0)
+                  : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kb_node<node_update_fp64<false>, 56>, block, 0);
         break;
-    case 2: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kb_elem<elem_kinematics_fp64>, block, 0); break;
+    case 2: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kb_elem<elem_kinematics_fp64, 128>, block, 0); break;
     default: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kb_material<elem_material_fp64<true>>, block, 0); break;
     }
     return e == cudaSuccess ? n : 0;

@@ -377,7 +377,8 @@ __device__ __forceinline__ void kahan_add(float &s, float &c, float v)
 
 // kEarly loads the node's state and all its corners before it uses any: on
 // meshes that leave most of an SM idle the update is its chain of memory
-// latencies, and this shortens it (a cycle of s=30 37.7 -> @C@ us).  On large ones the
+// latencies, and this shortens it (a cycle of s=30 36.2 -> 31.2 us, with the
+// merged control kernels).  On large ones the
 // registers that it holds through the gather cost more (s=192 0.31 -> 0.40
 // ms: 56 registers, or 40 with spills, instead of 32), and each component is
 // loaded where it is used.
@@ -667,10 +668,10 @@ void launch_batch_kernel_split(const Dom &d, const BatchView &b, cudaStream_t st
                               LaunchCfg cfg)
 {
     switch (kernel) {
-    case 0: kb_elem<elem_force_split><<<cfg.grid, cfg.block, 0, st>>>(d, b, cls); break;
+    case 0: kb_elem<elem_force_split, 96><<<cfg.grid, cfg.block, 0, st>>>(d, b, cls); break;
     case 1:
-        if (d.nn < kEarlyNodes) kb_node<node_update_split_from<true>><<<cfg.grid, cfg.block, 0, st>>>(d, b, cls);
-        else kb_node<node_update_split_from<false>><<<cfg.grid, cfg.block, 0, st>>>(d, b, cls);
+        if (d.nn < kEarlyNodes) kb_node<node_update_split_from<true>, 64><<<cfg.grid, cfg.block, 0, st>>>(d, b, cls);
+        else kb_node<node_update_split_from<false>, 40><<<cfg.grid, cfg.block, 0, st>>>(d, b, cls);
         break;
     case 2: kb_elem_capped<elem_kinematics_split, 2><<<cfg.grid, cfg.block, 0, st>>>(d, b, cls); break;
     default: kb_material_capped<elem_material_split<true>, 4><<<cfg.grid, cfg.block, 0, st>>>(d, b, cls); break;
@@ -701,10 +702,10 @@ int batch_max_blocks_split(int kernel, int block, bool early)
     int n = 0;
     cudaError_t e;
     switch (kernel) {
-    case 0: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kb_elem<elem_force_split>, block, 0); break;
+    case 0: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kb_elem<elem_force_split, 96>, block, 0); break;
     case 1:
-        e = early ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kb_node<node_update_split_from<true>>, block, 0)
-                  : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kb_node<node_update_split_from<false>>, block, 0);
+        e = early ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kb_node<node_update_split_from<true>, 64>, block, 0)
+                  : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kb_node<node_update_split_from<false>, 40>, block, 0);
         break;
     case 2: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kb_elem_capped<elem_kinematics_split, 2>, block, 0); break;
     default: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kb_material_capped<elem_material_split<true>, 4>, block, 0); break;
