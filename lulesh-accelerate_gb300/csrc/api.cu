@@ -735,9 +735,14 @@ int lulesh_get_field(lulesh_ctx *ctx, const char *name, double *host, long n)
                 return LULESH_OK;
             }
     }
+    if (ctx->dom.df == kArithDF64 && pair_field_name(name)) {
+        // through the corner forces' array, which holds nothing between calls
+        launch_pairs_to_doubles(f, ctx->dom.fcx, n, ctx->stream);
+        if (int rc = check_launch(ctx)) return rc;
+        f = ctx->dom.fcx;
+    }
     CK(cudaMemcpyAsync(host, f, n * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
-    if (ctx->dom.df == kArithDF64 && pair_field_name(name)) pairs_to_doubles(host, n);
     return LULESH_OK;
 }
 
@@ -748,13 +753,12 @@ int lulesh_set_field(lulesh_ctx *ctx, const char *name, const double *host, long
     double *f = find_field(ctx, name, &node, &writable);
     if (!f) return fail(ctx, LULESH_ERR_ARG, std::string("unknown field ") + name);
     if (n != (node ? ctx->nn : ctx->ne)) return fail(ctx, LULESH_ERR_ARG, std::string("wrong length for field ") + name);
-    std::vector<double> pairs;
-    if (ctx->dom.df == kArithDF64 && pair_field_name(name)) {
-        pairs.resize((size_t)n);
-        doubles_to_pairs(host, n, pairs.data());
-        host = pairs.data();
+    const bool pairs = ctx->dom.df == kArithDF64 && pair_field_name(name);
+    CK(cudaMemcpyAsync(pairs ? ctx->dom.fcx : f, host, n * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
+    if (pairs) {
+        launch_doubles_to_pairs(ctx->dom.fcx, f, n, ctx->stream);
+        if (int rc = check_launch(ctx)) return rc;
     }
-    CK(cudaMemcpyAsync(f, host, n * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
     int rc = clear_errors(ctx);
     return rc ? rc : refresh_split(ctx);

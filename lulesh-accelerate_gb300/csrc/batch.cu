@@ -880,9 +880,15 @@ int lulesh_batch_get_field(lulesh_batch *b, int i, const char *name, double *hos
             const long len = f.node ? b->nn_i[i] : b->ne_i[i];
             if (n != len) return bfail(b, LULESH_ERR_ARG, std::string("wrong length for field ") + name);
             const long off = f.node ? b->noff[i] : b->eoff[i];
-            BCK(cudaMemcpyAsync(host, f.p + off, n * sizeof(double), cudaMemcpyDeviceToHost, b->stream));
+            const double *from = f.p + off;
+            if (d.df == kArithDF64 && pair_field_name(name)) {
+                // through the corner forces' array, which holds nothing between calls
+                launch_pairs_to_doubles(from, d.fcx, n, b->stream);
+                BCK(cudaGetLastError());
+                from = d.fcx;
+            }
+            BCK(cudaMemcpyAsync(host, from, n * sizeof(double), cudaMemcpyDeviceToHost, b->stream));
             BCK(cudaStreamSynchronize(b->stream));
-            if (d.df == kArithDF64 && pair_field_name(name)) pairs_to_doubles(host, n);
             return LULESH_OK;
         }
     return bfail(b, LULESH_ERR_ARG, std::string("unknown field ") + name);

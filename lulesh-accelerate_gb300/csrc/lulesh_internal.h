@@ -93,12 +93,8 @@ int region_reps(int r, int nr, int cost);
 // order x y z xd yd zd e p v q; LULESH_OK or LULESH_ERR_ARG with *err set.
 int write_domain_file(const char *basename, int s, long ne, long nn, const int *nodelist, int step,
                       double time, const double *const fields[10], std::string *err);
-// Fields that the double-float kernels keep as pairs of floats, by name, and
-// the conversions of their accessors: a pair is its exact sum, a double its
-// FP32 rounding and the remainder's.
+// Fields that the double-float kernels keep as pairs of floats, by name.
 bool pair_field_name(const char *name);
-void pairs_to_doubles(double *a, long n);          // in place
-void doubles_to_pairs(const double *a, long n, double *out);
 // The message lulesh_last_error(NULL) returns.
 void set_last_error(const std::string &msg);
 void default_params(lulesh_params *p);

@@ -83,24 +83,6 @@ bool pair_field_name(const char *name)
     return false;
 }
 
-void pairs_to_doubles(double *a, long n)
-{
-    for (long i = 0; i < n; ++i) {
-        float w[2];
-        std::memcpy(w, a + i, sizeof w);
-        a[i] = (double)w[0] + (double)w[1];
-    }
-}
-
-void doubles_to_pairs(const double *a, long n, double *out)
-{
-    for (long i = 0; i < n; ++i) {
-        const float hi = (float)a[i];
-        const float w[2] = {hi, std::isfinite(hi) ? (float)(a[i] - (double)hi) : 0.f};
-        std::memcpy(out + i, w, sizeof w);
-    }
-}
-
 void HostMesh::reciprocals(bool even, std::vector<double> &inv_volo, std::vector<double> &inv_mass) const
 {
     inv_volo.resize(ne);
