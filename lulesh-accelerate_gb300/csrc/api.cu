@@ -337,19 +337,19 @@ void lulesh_destroy(lulesh_ctx *ctx)
 
 namespace {
 
-// A context for a built host mesh: device arrays, initial state, stream.
-int create_from_mesh(const HostMesh &m, int precision, const lulesh_params *params, lulesh_ctx **out)
+// A context: stream, device arrays, initial state.  m null: the s^3 cube of
+// a Sedov problem, set up on the device (mesh_gpu.cu); else that host mesh.
+int create_context(const HostMesh *m, int s, int init_mode, int precision, const lulesh_params *params, lulesh_ctx **out)
 {
-    const int s = m.s;
     *out = nullptr;
     lulesh_ctx *ctx = new lulesh_ctx;
     int rc = LULESH_OK;
     auto bail = [&](int code) { g_err = ctx->err; lulesh_destroy(ctx); return code; };
 
     ctx->s = s;
-    ctx->origin = m.origin;
-    ctx->ne = m.ne;
-    ctx->nn = m.nn;
+    ctx->origin = m ? m->origin : 0;
+    ctx->ne = m ? m->ne : (long)s * s * s;
+    ctx->nn = m ? m->nn : (long)(s + 1) * (s + 1) * (s + 1);
     ctx->precision = precision;
     if (cudaGetDevice(&ctx->device) != cudaSuccess ||
         cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking) != cudaSuccess) {
@@ -364,8 +364,8 @@ int create_from_mesh(const HostMesh &m, int precision, const lulesh_params *para
 
     Dom &d = ctx->dom;
     d.s = s;
-    d.ne = (int)m.ne;
-    d.nn = (int)m.nn;
+    d.ne = (int)ctx->ne;
+    d.nn = (int)ctx->nn;
     d.keep = 0;
     if (params) d.prm = *params;
     else default_params(&d.prm);
@@ -375,80 +375,103 @@ int create_from_mesh(const HostMesh &m, int precision, const lulesh_params *para
             sms = 1;
         choose_blocks(d, sms);
     }
-    const size_t ne = m.ne, nn = m.nn;
+    const size_t ne = ctx->ne, nn = ctx->nn;
+    d.df = arith_of(precision);
+    d.gate = nullptr;
 
-    int *nodelist, *cstart, *clist, *lxim, *lxip, *letam, *letap, *lzetam, *lzetap, *ebc;
+    // All arrays in one allocation.  The lists that a cube's kernels form
+    // from the indices exist only for a mesh given by its lists.
+    int *nodelist, *cstart = nullptr, *clist = nullptr, *ebc, *nb[6] = {};
     unsigned char *nbc;
     double *volo, *emass, *nmass;
-#define A(p, n) if ((rc = dalloc(ctx, &(p), (n))) != LULESH_OK) return bail(rc)
-    A(nodelist, 8 * ne); A(cstart, nn + 1); A(clist, 8 * ne); A(nbc, nn);
-    A(lxim, ne); A(lxip, ne); A(letam, ne); A(letap, ne); A(lzetam, ne); A(lzetap, ne); A(ebc, ne);
-    A(volo, ne); A(emass, ne); A(nmass, nn);
-    A(d.x, nn); A(d.y, nn); A(d.z, nn); A(d.xd, nn); A(d.yd, nn); A(d.zd, nn);
-    A(d.fx, nn); A(d.fy, nn); A(d.fz, nn);
-    A(d.e, ne); A(d.p, ne); A(d.q, ne); A(d.v, ne); A(d.ss, ne);
-    A(d.vnew, ne); A(d.delv, ne); A(d.vdov, ne); A(d.arealg, ne); A(d.ql, ne); A(d.qq, ne);
-    A(d.delv_xi, ne); A(d.delv_eta, ne); A(d.delv_zeta, ne);
-    A(d.delx_xi, ne); A(d.delx_eta, ne); A(d.delx_zeta, ne);
-    d.df = arith_of(precision);
-    if (precision != LULESH_PRECISION_SPLIT) {
-        A(d.fcx, 8 * ne); A(d.fcy, 8 * ne); A(d.fcz, 8 * ne);
-        A(d.geo, geo_words(d.df) * ne);
-    } else {
-        A(d.f32x, 8 * ne); A(d.f32y, 8 * ne); A(d.f32z, 8 * ne);
-        A(d.xs, nn); A(d.ys, nn); A(d.zs, nn); A(d.xds, nn); A(d.yds, nn); A(d.zds, nn);
-        A(d.gq, 6 * ne);
-    }
-    A(d.inv_mass, nn); A(d.inv_volo, ne);
-    A(d.sc, 1); A(ctx->d_active, 1); A(ctx->d_max_cycles, 1);
-#undef A
+    auto layout = [&](Slab &b) {
+        b.take(nodelist, 8 * ne);
+        if (m) {
+            b.take(cstart, nn + 1);
+            b.take(clist, 8 * ne);
+            for (int *&l : nb) b.take(l, ne);
+        }
+        b.take(nbc, nn);
+        b.take(ebc, ne);
+        b.take(volo, ne);
+        b.take(emass, ne);
+        b.take(nmass, nn);
+        for (double **f : {&d.x, &d.y, &d.z, &d.xd, &d.yd, &d.zd, &d.fx, &d.fy, &d.fz, &d.inv_mass}) b.take(*f, nn);
+        for (double **f : {&d.e, &d.p, &d.q, &d.v, &d.ss, &d.vnew, &d.delv, &d.vdov, &d.arealg, &d.ql, &d.qq, &d.delv_xi,
+                           &d.delv_eta, &d.delv_zeta, &d.delx_xi, &d.delx_eta, &d.delx_zeta, &d.inv_volo})
+            b.take(*f, ne);
+        if (precision != LULESH_PRECISION_SPLIT) {
+            for (double **f : {&d.fcx, &d.fcy, &d.fcz}) b.take(*f, 8 * ne);
+            b.take(d.geo, geo_words(d.df) * ne);
+        } else {
+            for (float **f : {&d.f32x, &d.f32y, &d.f32z}) b.take(*f, 8 * ne);
+            for (float2 **f : {&d.xs, &d.ys, &d.zs, &d.xds, &d.yds, &d.zds}) b.take(*f, nn);
+            b.take(d.gq, 6 * ne);
+        }
+        b.take(d.sc, 1);
+        b.take(ctx->d_active, 1);
+        b.take(ctx->d_max_cycles, 1);
+    };
+    Slab slab;
+    layout(slab);
+    if ((rc = dalloc(ctx, &slab.base, slab.used)) != LULESH_OK) return bail(rc);
+    const size_t bytes = slab.used;
+    slab.used = 0;
+    layout(slab);
     d.nodelist = nodelist;
     d.corner_start = cstart;
     d.corner_list = clist;
     d.node_bc = nbc;
-    d.lxim = lxim; d.lxip = lxip; d.letam = letam; d.letap = letap; d.lzetam = lzetam; d.lzetap = lzetap;
+    d.lxim = nb[0]; d.lxip = nb[1]; d.letam = nb[2]; d.letap = nb[3]; d.lzetam = nb[4]; d.lzetap = nb[5];
     d.elem_bc = ebc;
     d.volo = volo; d.elem_mass = emass; d.nodal_mass = nmass;
-    d.gate = nullptr;
 
-    // node -> corner slots, translated from the reference's 8*elem+corner
-    // numbering to the corner-major slot corner*ne + elem
-    std::vector<int> start(nn + 1), slots(8 * ne);
-    for (size_t i = 0; i < nn; ++i) start[i] = m.node_elem_start[i];
-    start[nn] = (int)(8 * ne);
-    for (size_t i = 0; i < 8 * ne; ++i) {
-        const int k = m.node_elem_corner_list[i];
-        slots[i] = (k & 7) * (int)ne + (k >> 3);
-    }
-    std::vector<double> ones(ne, 1.0), e(ne, 0.0), inv_mass, inv_volo;
-    m.reciprocals(d.df == kArithDF64, inv_volo, inv_mass);
-    e[m.origin] = m.e0;
     cudaStream_t st = ctx->stream;
-    auto up = [&](void *dst, const void *src, size_t bytes) {
-        return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st) == cudaSuccess;
+    auto up = [&](void *dst, const void *src, size_t n) {
+        return cudaMemcpyAsync(dst, src, n, cudaMemcpyHostToDevice, st) == cudaSuccess;
     };
-    bool ok = up(nodelist, m.nodelist.data(), 8 * ne * 4) && up(cstart, start.data(), (nn + 1) * 4) &&
-              up(clist, slots.data(), 8 * ne * 4) && up(nbc, m.node_bc.data(), nn) &&
-              up(lxim, m.lxim.data(), ne * 4) && up(lxip, m.lxip.data(), ne * 4) &&
-              up(letam, m.letam.data(), ne * 4) && up(letap, m.letap.data(), ne * 4) &&
-              up(lzetam, m.lzetam.data(), ne * 4) && up(lzetap, m.lzetap.data(), ne * 4) &&
-              up(ebc, m.elem_bc.data(), ne * 4) && up(volo, m.volo.data(), ne * 8) &&
-              up(emass, m.elem_mass.data(), ne * 8) && up(nmass, m.nodal_mass.data(), nn * 8) && up(d.inv_mass, inv_mass.data(), nn * 8) && up(d.inv_volo, inv_volo.data(), ne * 8) &&
-              up(d.x, m.x.data(), nn * 8) && up(d.y, m.y.data(), nn * 8) && up(d.z, m.z.data(), nn * 8) &&
-              up(d.e, e.data(), ne * 8) && up(d.v, ones.data(), ne * 8);
-    ok = ok && cudaMemsetAsync(d.xd, 0, nn * 8, st) == cudaSuccess &&
-         cudaMemsetAsync(d.yd, 0, nn * 8, st) == cudaSuccess &&
-         cudaMemsetAsync(d.zd, 0, nn * 8, st) == cudaSuccess &&
-         cudaMemsetAsync(d.fx, 0, nn * 8, st) == cudaSuccess &&
-         cudaMemsetAsync(d.fy, 0, nn * 8, st) == cudaSuccess &&
-         cudaMemsetAsync(d.fz, 0, nn * 8, st) == cudaSuccess;
-    for (double *f : {d.p, d.q, d.ss, d.vnew, d.delv, d.vdov, d.arealg, d.ql, d.qq, d.delv_xi, d.delv_eta,
-                      d.delv_zeta, d.delx_xi, d.delx_eta, d.delx_zeta})
-        ok = ok && cudaMemsetAsync(f, 0, ne * 8, st) == cudaSuccess;
+    double e0, dt0;
+    bool ok = cudaMemsetAsync(slab.base, 0, bytes, st) == cudaSuccess;
+    std::vector<double> e, ones, inv_volo, inv_mass;
+    std::vector<int> start, slots;
+    if (m) {
+        e0 = m->e0;
+        dt0 = m->dt0;
+        // node -> corner slots, translated from the reference's 8*elem+corner
+        // numbering to the corner-major slot corner*ne + elem
+        start.assign(m->node_elem_start.begin(), m->node_elem_start.end());
+        start.push_back((int)(8 * ne));
+        slots.resize(8 * ne);
+        for (size_t i = 0; i < 8 * ne; ++i) {
+            const int k = m->node_elem_corner_list[i];
+            slots[i] = (k & 7) * (int)ne + (k >> 3);
+        }
+        ones.assign(ne, 1.0);
+        e.assign(ne, 0.0);
+        e[m->origin] = e0;
+        inv_volo.resize(ne);
+        inv_mass.resize(nn);
+        for (size_t i = 0; i < ne; ++i) inv_volo[i] = 1.0 / m->volo[i];
+        for (size_t i = 0; i < nn; ++i) inv_mass[i] = 1.0 / m->nodal_mass[i];
+        ok = ok && up(nodelist, m->nodelist.data(), 8 * ne * 4) && up(cstart, start.data(), (nn + 1) * 4) &&
+             up(clist, slots.data(), 8 * ne * 4) && up(nbc, m->node_bc.data(), nn) && up(ebc, m->elem_bc.data(), ne * 4) &&
+             up(volo, m->volo.data(), ne * 8) && up(emass, m->elem_mass.data(), ne * 8) &&
+             up(nmass, m->nodal_mass.data(), nn * 8) && up(d.inv_mass, inv_mass.data(), nn * 8) &&
+             up(d.inv_volo, inv_volo.data(), ne * 8) && up(d.x, m->x.data(), nn * 8) && up(d.y, m->y.data(), nn * 8) &&
+             up(d.z, m->z.data(), nn * 8) && up(d.e, e.data(), ne * 8) && up(d.v, ones.data(), ne * 8);
+        const std::vector<int> *lists[6] = {&m->lxim, &m->lxip, &m->letam, &m->letap, &m->lzetam, &m->lzetap};
+        for (int i = 0; i < 6; ++i) ok = ok && up(nb[i], lists[i]->data(), ne * 4);
+    } else {
+        sedov_start(s, init_mode, cube_corner_volume(s), &e0, &dt0);
+        if (ok) {
+            launch_build_cube(d, CubeDesc{s, 0, 0, e0}, st);
+            ok = cudaGetLastError() == cudaSuccess;
+        }
+    }
     DevScalars *h = ctx->h_sc;
     memset(h, 0, sizeof *h);
     h->time = 0.0;
-    h->deltatime = m.dt0;
+    h->deltatime = dt0;
     h->dtcourant = 1.0e+20;
     h->dthydro = 1.0e+20;
     h->cycle = 0;
@@ -486,9 +509,7 @@ int lulesh_create(int s, int init_mode, int precision, const lulesh_params *para
     if (init_mode != LULESH_INIT_V1 && init_mode != LULESH_INIT_V2)
         return fail(nullptr, LULESH_ERR_ARG, "lulesh_create: init_mode must be LULESH_INIT_V1 or LULESH_INIT_V2");
     if (int rc = check_precision(precision, "lulesh_create")) return rc;
-    HostMesh m;
-    m.build(s, init_mode);
-    return create_from_mesh(m, precision, params, out);
+    return create_context(nullptr, s, init_mode, precision, params, out);
 }
 
 int lulesh_create_unstructured(const lulesh_unstructured_mesh *mesh, int precision, const lulesh_params *params,
@@ -500,7 +521,7 @@ int lulesh_create_unstructured(const lulesh_unstructured_mesh *mesh, int precisi
     HostMesh m;
     std::string err;
     if (m.build_unstructured(*mesh, &err) != LULESH_OK) return fail(nullptr, LULESH_ERR_ARG, err);
-    return create_from_mesh(m, precision, params, out);
+    return create_context(&m, m.s, 0, precision, params, out);
 }
 
 int lulesh_create_lmesh(const char *path, int precision, const lulesh_params *params, lulesh_ctx **out)

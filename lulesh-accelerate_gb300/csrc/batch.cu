@@ -546,36 +546,54 @@ int lulesh_batch_create(int n, const int *sizes, const double *e0_scale, int ini
     else default_params(&d.prm);
     const size_t ne = b->ne_tot, nn = b->nn_tot;
     int rc;
-    int *nodelist, *cstart, *clist, *lxim, *lxip, *letam, *letap, *lzetam, *lzetap, *ebc;
+    d.df = arith_of(precision);
+    // All arrays in one allocation.  The corner and neighbour lists stay null:
+    // the kernels form them from a cube's indices.
+    int *nodelist, *ebc;
     unsigned char *nbc;
     double *volo, *emass, *nmass;
-#define A(p, cnt) if ((rc = balloc(b, &(p), (cnt))) != LULESH_OK) return bail(rc)
-    A(nodelist, 8 * ne); A(cstart, nn + 1); A(clist, 8 * ne); A(nbc, nn);
-    A(lxim, ne); A(lxip, ne); A(letam, ne); A(letap, ne); A(lzetam, ne); A(lzetap, ne); A(ebc, ne);
-    A(volo, ne); A(emass, ne); A(nmass, nn);
-    A(d.x, nn); A(d.y, nn); A(d.z, nn); A(d.xd, nn); A(d.yd, nn); A(d.zd, nn);
-    A(d.e, ne); A(d.p, ne); A(d.q, ne); A(d.v, ne); A(d.ss, ne);
-    A(d.vnew, ne); A(d.delv, ne); A(d.vdov, ne); A(d.arealg, ne);
-    A(d.delv_xi, ne); A(d.delv_eta, ne); A(d.delv_zeta, ne);
-    A(d.delx_xi, ne); A(d.delx_eta, ne); A(d.delx_zeta, ne);
-    d.df = arith_of(precision);
-    if (precision != LULESH_PRECISION_SPLIT) {
-        A(d.fcx, 8 * ne); A(d.fcy, 8 * ne); A(d.fcz, 8 * ne);
-        A(d.geo, geo_words(d.df) * ne);
-    } else {
-        A(d.f32x, 8 * ne); A(d.f32y, 8 * ne); A(d.f32z, 8 * ne);
-        A(d.xs, nn); A(d.ys, nn); A(d.zs, nn); A(d.xds, nn); A(d.yds, nn); A(d.zds, nn);
-        A(d.gq, 6 * ne);
-    }
-    A(d.inv_mass, nn); A(d.inv_volo, ne);
-    A(d.sc, (size_t)n); A(b->d_max, 1);
     int *etile_inst_d, *ntile_inst_d, *etile_class_d, *ntile_class_d, *iee, *ine;
-    A(etile_inst_d, net); A(ntile_inst_d, nnt); A(etile_class_d, net); A(ntile_class_d, nnt);
-    A(iee, n); A(ine, n);
-    A(b->bv.active_etiles, net); A(b->bv.active_ntiles, nnt); A(b->bv.counts, 2 * kMaxClasses);
-    A(b->bv.inst_active, n);
-    d.nodelist = nodelist; d.corner_start = cstart; d.corner_list = clist; d.node_bc = nbc;
-    d.lxim = lxim; d.lxip = lxip; d.letam = letam; d.letap = letap; d.lzetam = lzetam; d.lzetap = lzetap;
+    CubeDesc *cubes_d;
+    auto layout = [&](Slab &sl) {
+        sl.take(nodelist, 8 * ne);
+        sl.take(nbc, nn);
+        sl.take(ebc, ne);
+        sl.take(volo, ne);
+        sl.take(emass, ne);
+        sl.take(nmass, nn);
+        for (double **f : {&d.x, &d.y, &d.z, &d.xd, &d.yd, &d.zd, &d.inv_mass}) sl.take(*f, nn);
+        for (double **f : {&d.e, &d.p, &d.q, &d.v, &d.ss, &d.vnew, &d.delv, &d.vdov, &d.arealg, &d.delv_xi, &d.delv_eta,
+                           &d.delv_zeta, &d.delx_xi, &d.delx_eta, &d.delx_zeta, &d.inv_volo})
+            sl.take(*f, ne);
+        if (precision != LULESH_PRECISION_SPLIT) {
+            for (double **f : {&d.fcx, &d.fcy, &d.fcz}) sl.take(*f, 8 * ne);
+            sl.take(d.geo, geo_words(d.df) * ne);
+        } else {
+            for (float **f : {&d.f32x, &d.f32y, &d.f32z}) sl.take(*f, 8 * ne);
+            for (float2 **f : {&d.xs, &d.ys, &d.zs, &d.xds, &d.yds, &d.zds}) sl.take(*f, nn);
+            sl.take(d.gq, 6 * ne);
+        }
+        sl.take(d.sc, n);
+        sl.take(b->d_max, 1);
+        sl.take(etile_inst_d, net);
+        sl.take(ntile_inst_d, nnt);
+        sl.take(etile_class_d, net);
+        sl.take(ntile_class_d, nnt);
+        sl.take(iee, n);
+        sl.take(ine, n);
+        sl.take(cubes_d, n);
+        sl.take(b->bv.active_etiles, net);
+        sl.take(b->bv.active_ntiles, nnt);
+        sl.take(b->bv.counts, 2 * kMaxClasses);
+        sl.take(b->bv.inst_active, n);
+    };
+    Slab slab;
+    layout(slab);
+    if ((rc = balloc(b, &slab.base, slab.used)) != LULESH_OK) return bail(rc);
+    const size_t bytes = slab.used;
+    slab.used = 0;
+    layout(slab);
+    d.nodelist = nodelist; d.node_bc = nbc;
     d.elem_bc = ebc; d.volo = volo; d.elem_mass = emass; d.nodal_mass = nmass;
     d.ql = nullptr; d.qq = nullptr; d.fx = nullptr; d.fy = nullptr; d.fz = nullptr;
     d.gate = nullptr;
@@ -593,56 +611,21 @@ int lulesh_batch_create(int n, const int *sizes, const double *e0_scale, int ini
         bv.nclass_off[c] = nclass_off[c];
     }
 
-    // host images of the flat arrays, instance by instance
+    // the tables of tiles and instances from the host, the cubes themselves
+    // set up on the device (mesh_gpu.cu)
     cudaStream_t st = b->stream;
-    bool ok = true;
-    auto up = [&](void *dst, const void *src, size_t bytes) {
-        ok = ok && cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st) == cudaSuccess;
+    bool ok = cudaMemsetAsync(slab.base, 0, bytes, st) == cudaSuccess;
+    auto up = [&](void *dst, const void *src, size_t len) {
+        ok = ok && cudaMemcpyAsync(dst, src, len, cudaMemcpyHostToDevice, st) == cudaSuccess;
     };
-    std::vector<int> start(nn + 1, 0), iee_h(n), ine_h(n);
-    std::vector<double> fill_one;
-    long cpos = 0;   // corner-list position: instances contiguous, no padding
+    std::vector<int> iee_h(n), ine_h(n);
+    std::vector<CubeDesc> cubes(n);
     for (int i = 0; i < n; ++i) {
-        HostMesh m;
-        m.build(sizes[i], init_mode);
-        const double f = e0_scale ? e0_scale[i] : 1.0;
-        const double e0 = m.e0 * f;
-        const double dt0 = init_mode == LULESH_INIT_V2 ? (.5 * std::cbrt(m.volo[0])) / std::sqrt(2.0 * e0) : m.dt0;
-        const long eo_i = b->eoff[i], no_i = b->noff[i], nei = b->ne_i[i], nni = b->nn_i[i];
-        std::vector<int> nl(8 * nei), slots(8 * nei), lx[6];
-        for (long k = 0; k < 8 * nei; ++k) {
-            nl[k] = (int)(m.nodelist[k] + no_i);
-            const int c = m.node_elem_corner_list[k];
-            slots[k] = (int)((c & 7) * (long)ne + eo_i + (c >> 3));
-        }
-        const std::vector<int> *src[6] = {&m.lxim, &m.lxip, &m.letam, &m.letap, &m.lzetam, &m.lzetap};
-        int *dst[6] = {lxim, lxip, letam, letap, lzetam, lzetap};
-        for (int j = 0; j < 6; ++j) {
-            lx[j].resize(nei);
-            for (long k = 0; k < nei; ++k) lx[j][k] = (int)((*src[j])[k] + eo_i);
-            up(dst[j] + eo_i, lx[j].data(), nei * 4);
-        }
-        for (long k = 0; k < nni; ++k) start[no_i + k] = (int)(cpos + m.node_elem_start[k]);
-        for (long k = nni; k < round_tile(nni); ++k) start[no_i + k] = (int)(cpos + 8 * nei);
-        std::vector<double> e(nei, 0.0), one(nei, 1.0);
-        e[0] = e0;
-        up(nodelist + 8 * eo_i, nl.data(), 8 * nei * 4);
-        up(clist + cpos, slots.data(), 8 * nei * 4);
-        up(nbc + no_i, m.node_bc.data(), nni);
-        up(ebc + eo_i, m.elem_bc.data(), nei * 4);
-        up(volo + eo_i, m.volo.data(), nei * 8);
-        up(emass + eo_i, m.elem_mass.data(), nei * 8);
-        up(nmass + no_i, m.nodal_mass.data(), nni * 8);
-        std::vector<double> im, iv;
-        m.reciprocals(d.df == kArithDF64, iv, im);
-        up(d.inv_mass + no_i, im.data(), nni * 8);
-        up(d.inv_volo + eo_i, iv.data(), nei * 8);
-        up(d.x + no_i, m.x.data(), nni * 8);
-        up(d.y + no_i, m.y.data(), nni * 8);
-        up(d.z + no_i, m.z.data(), nni * 8);
-        up(d.e + eo_i, e.data(), nei * 8);
-        up(d.v + eo_i, one.data(), nei * 8);
-        cudaStreamSynchronize(st);   // the host vectors above go out of scope
+        double e0, dt0;
+        sedov_start(sizes[i], init_mode, cube_corner_volume(sizes[i]), &e0, &dt0);
+        const double scaled = e0 * (e0_scale ? e0_scale[i] : 1.0);
+        if (init_mode == LULESH_INIT_V2) dt0 = (.5 * std::cbrt(cube_corner_volume(sizes[i]))) / std::sqrt(2.0 * scaled);
+        cubes[i] = {sizes[i], (int)b->eoff[i], (int)b->noff[i], scaled};
         DevScalars &h = b->h_sc[i];
         memset(&h, 0, sizeof h);
         h.deltatime = dt0;
@@ -650,16 +633,12 @@ int lulesh_batch_create(int n, const int *sizes, const double *e0_scale, int ini
         h.dthydro = 1.0e+20;
         h.courant_key = ~0ULL;
         h.hydro_key = ~0ULL;
-        h.elem_begin = (int)eo_i;
+        h.elem_begin = (int)b->eoff[i];
         h.edge = sizes[i];
-        h.node_begin = (int)no_i;
-        iee_h[i] = (int)(eo_i + nei);
-        ine_h[i] = (int)(no_i + nni);
-        cpos += 8 * nei;
+        h.node_begin = (int)b->noff[i];
+        iee_h[i] = (int)(b->eoff[i] + b->ne_i[i]);
+        ine_h[i] = (int)(b->noff[i] + b->nn_i[i]);
     }
-    start[nn] = (int)cpos;
-    // padded node tails after the last instance keep empty corner ranges
-    up(cstart, start.data(), (nn + 1) * 4);
     up(d.sc, b->h_sc, sizeof(DevScalars) * n);
     up(etile_inst_d, etile_inst.data(), net * 4);
     up(ntile_inst_d, ntile_inst.data(), nnt * 4);
@@ -667,29 +646,11 @@ int lulesh_batch_create(int n, const int *sizes, const double *e0_scale, int ini
     up(ntile_class_d, ntile_class.data(), nnt * 4);
     up(iee, iee_h.data(), n * 4);
     up(ine, ine_h.data(), n * 4);
-    // padding entries of the mass arrays are read by whole-array kernels
-    // (the split path's reciprocal masses): give them unit values
-    {
-        std::vector<double> ones(std::max(ne, nn), 1.0);
-        for (int i = 0; i < n; ++i) {
-            const long etail = round_tile(b->ne_i[i]) - b->ne_i[i], ntail = round_tile(b->nn_i[i]) - b->nn_i[i];
-            if (etail) {
-                up(volo + b->eoff[i] + b->ne_i[i], ones.data(), etail * 8);
-                up(emass + b->eoff[i] + b->ne_i[i], ones.data(), etail * 8);
-                up(d.inv_volo + b->eoff[i] + b->ne_i[i], ones.data(), etail * 8);
-            }
-            if (ntail) {
-                up(nmass + b->noff[i] + b->nn_i[i], ones.data(), ntail * 8);
-                up(d.inv_mass + b->noff[i] + b->nn_i[i], ones.data(), ntail * 8);
-            }
-        }
-        cudaStreamSynchronize(st);
+    up(cubes_d, cubes.data(), n * sizeof(CubeDesc));
+    if (ok) {
+        launch_build_cubes(d, cubes_d, etile_inst_d, ntile_inst_d, st);
+        ok = cudaGetLastError() == cudaSuccess;
     }
-    for (double *f : {d.xd, d.yd, d.zd}) ok = ok && cudaMemsetAsync(f, 0, nn * 8, st) == cudaSuccess;
-    for (double *f : {d.p, d.q, d.ss, d.vnew, d.delv, d.vdov, d.arealg, d.delv_xi, d.delv_eta, d.delv_zeta,
-                      d.delx_xi, d.delx_eta, d.delx_zeta})
-        ok = ok && cudaMemsetAsync(f, 0, ne * 8, st) == cudaSuccess;
-    ok = ok && cudaMemsetAsync(b->bv.counts, 0, 2 * kMaxClasses * 4, st) == cudaSuccess;
     if (ok && precision == LULESH_PRECISION_SPLIT) {
         launch_split_sync(d, st);
         ok = cudaGetLastError() == cudaSuccess;
@@ -716,7 +677,9 @@ int lulesh_batch_create(int n, const int *sizes, const double *e0_scale, int ini
             if (inst.empty() || !all) continue;
             const int m = (int)inst.size();
             int *d_inst, *d_s, *d_eb, *d_nb;
-            A(d_inst, m); A(d_s, m); A(d_eb, m); A(d_nb, m);
+            if ((rc = balloc(b, &d_inst, m)) || (rc = balloc(b, &d_s, m)) || (rc = balloc(b, &d_eb, m)) ||
+                (rc = balloc(b, &d_nb, m)))
+                return bail(rc);
             ok = cudaMemcpy(d_inst, inst.data(), m * 4, cudaMemcpyHostToDevice) == cudaSuccess &&
                  cudaMemcpy(d_s, sz.data(), m * 4, cudaMemcpyHostToDevice) == cudaSuccess &&
                  cudaMemcpy(d_eb, eb.data(), m * 4, cudaMemcpyHostToDevice) == cudaSuccess &&
@@ -726,7 +689,7 @@ int lulesh_batch_create(int n, const int *sizes, const double *e0_scale, int ini
                 for (int j = 0; j < m; ++j)
                     begin[j + 1] = begin[j] + (kStageRows[r] == 4 ? TileShape<4>::tiles(sz[j]) : TileShape<2>::tiles(sz[j]));
                 long long *d_begin;
-                A(d_begin, m + 1);
+                if ((rc = balloc(b, &d_begin, m + 1))) return bail(rc);
                 ok = cudaMemcpy(d_begin, begin.data(), (m + 1) * sizeof(long long), cudaMemcpyHostToDevice) == cudaSuccess;
                 b->staged[c][r] = {m, d_inst, d_s, d_eb, d_nb, d_begin};
             }
@@ -736,7 +699,6 @@ int lulesh_batch_create(int n, const int *sizes, const double *e0_scale, int ini
             }
         }
     }
-#undef A
     default_cfg(b);
     *out = b;
     return LULESH_OK;

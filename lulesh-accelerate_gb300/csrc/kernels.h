@@ -42,6 +42,11 @@ inline void choose_blocks(Dom &d, int sms)
 struct CycleEnd;   // common.cuh
 void launch_end_cycle(const Dom &d, cudaStream_t st, const CycleEnd &end);
 
+// The initial state and mesh data of one cube, or of a batch's cubes with
+// their tiles' numbers (mesh_gpu.cu), into arrays that hold zeros.
+void launch_build_cube(const Dom &d, const CubeDesc &cube, cudaStream_t st);
+void launch_build_cubes(const Dom &d, const CubeDesc *cubes, const int *etile_cube, const int *ntile_cube, cudaStream_t st);
+
 // Plain FP64 path (step_fp64.cu).
 void launch_time_increment(const Dom &d, cudaStream_t st);
 void launch_lagrange_nodal(const Dom &d, cudaStream_t st);

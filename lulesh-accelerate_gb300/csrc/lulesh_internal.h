@@ -64,13 +64,6 @@ struct HostMesh {
     void build(int s, int init_mode);
     // LULESH_OK, or LULESH_ERR_ARG with a message in *err
     int build_unstructured(const lulesh_unstructured_mesh &u, std::string *err);
-    // Reciprocal reference volumes and nodal masses for the kernels.  With
-    // even set, on the cube, each is taken of the mean of the entity's value
-    // and its mirror image's (rows and columns exchanged), which the set-up's
-    // sums leave an ulp apart: the double-float kernels keep a mirror-
-    // symmetric state exactly symmetric (dfpack.cuh), and these are the only
-    // data that would disturb it.
-    void reciprocals(bool even, std::vector<double> &inv_volo, std::vector<double> &inv_mass) const;
 
   private:
     void derive();                       // corner lists, volumes, masses
@@ -85,6 +78,23 @@ struct LmeshFile {
 };
 
 double host_elem_volume(const double x[8], const double y[8], const double z[8]);
+// The Sedov problem's initial energy and time step on the s^3 cube, whose
+// corner element has volume volo0 (cube_corner_volume).
+void sedov_start(int s, int init_mode, double volo0, double *e0, double *dt0);
+double cube_corner_volume(int s);
+
+// Carves device arrays out of one allocation, each on a 256-byte boundary:
+// the same sequence of take() calls first on a null base, for the size.
+struct Slab {
+    char *base = nullptr;
+    size_t used = 0;
+    template <typename T>
+    void take(T *&p, size_t n)
+    {
+        p = base ? reinterpret_cast<T *>(base + used) : nullptr;
+        used += ((n ? n : 1) * sizeof(T) + 255) / 256 * 256;
+    }
+};
 // LULESH 2.0 region numbers (1..nr) of ne elements and the EOS repetitions
 // of region r (0-based)
 void region_numbers(long ne, int nr, int balance, std::vector<int> &reg);
@@ -177,6 +187,13 @@ struct Dom {
 // tile of kTile elements (or nodes) belongs to exactly one instance.  Tiles
 // are grouped into size classes, each with its own launch shape.
 constexpr int kTile = 256;
+// One cube of a set-up on the device (launch_build_cubes): its edge, the
+// first of its elements and nodes in the flat arrays, the energy of its
+// first element.
+struct CubeDesc {
+    int s, elem_begin, node_begin;
+    double e0;
+};
 constexpr int kMaxClasses = 3;
 constexpr int kBatchKernels = 4;   // force, node update, kinematics, material
 

@@ -10,6 +10,7 @@
 // -ffp-contract=off so that the floating-point results are the reference's
 // on every host architecture.
 #include "lulesh_internal.h"
+#include "elem_volume.h"
 
 #include <cerrno>
 #include <cmath>
@@ -20,32 +21,7 @@
 
 namespace lulesh {
 
-// CalcElemVolume (LULESH-OMP.cc:1706-1790), same association as the
-// reference, for the host set-up.
-double host_elem_volume(const double x[8], const double y[8], const double z[8])
-{
-    const double twelveth = 1.0 / 12.0;
-    const double dx61 = x[6] - x[1], dy61 = y[6] - y[1], dz61 = z[6] - z[1];
-    const double dx70 = x[7] - x[0], dy70 = y[7] - y[0], dz70 = z[7] - z[0];
-    const double dx63 = x[6] - x[3], dy63 = y[6] - y[3], dz63 = z[6] - z[3];
-    const double dx20 = x[2] - x[0], dy20 = y[2] - y[0], dz20 = z[2] - z[0];
-    const double dx50 = x[5] - x[0], dy50 = y[5] - y[0], dz50 = z[5] - z[0];
-    const double dx64 = x[6] - x[4], dy64 = y[6] - y[4], dz64 = z[6] - z[4];
-    const double dx31 = x[3] - x[1], dy31 = y[3] - y[1], dz31 = z[3] - z[1];
-    const double dx72 = x[7] - x[2], dy72 = y[7] - y[2], dz72 = z[7] - z[2];
-    const double dx43 = x[4] - x[3], dy43 = y[4] - y[3], dz43 = z[4] - z[3];
-    const double dx57 = x[5] - x[7], dy57 = y[5] - y[7], dz57 = z[5] - z[7];
-    const double dx14 = x[1] - x[4], dy14 = y[1] - y[4], dz14 = z[1] - z[4];
-    const double dx25 = x[2] - x[5], dy25 = y[2] - y[5], dz25 = z[2] - z[5];
-    auto triple = [](double x1, double y1, double z1, double x2, double y2, double z2,
-                     double x3, double y3, double z3) {
-        return x1 * (y2 * z3 - z2 * y3) + x2 * (z1 * y3 - y1 * z3) + x3 * (y1 * z2 - z1 * y2);
-    };
-    double vol = triple(dx31 + dx72, dx63, dx20, dy31 + dy72, dy63, dy20, dz31 + dz72, dz63, dz20) +
-                 triple(dx43 + dx57, dx64, dx70, dy43 + dy57, dy64, dy70, dz43 + dz57, dz64, dz70) +
-                 triple(dx14 + dx25, dx61, dx50, dy14 + dy25, dy61, dy50, dz14 + dz25, dz61, dz50);
-    return vol * twelveth;
-}
+double host_elem_volume(const double x[8], const double y[8], const double z[8]) { return elem_volume<double>(x, y, z); }
 
 void default_params(lulesh_params *p)
 {
@@ -83,25 +59,6 @@ bool pair_field_name(const char *name)
     return false;
 }
 
-void HostMesh::reciprocals(bool even, std::vector<double> &inv_volo, std::vector<double> &inv_mass) const
-{
-    inv_volo.resize(ne);
-    inv_mass.resize(nn);
-    if (!even || s <= 0) {
-        for (long i = 0; i < ne; ++i) inv_volo[i] = 1.0 / volo[i];
-        for (long i = 0; i < nn; ++i) inv_mass[i] = 1.0 / nodal_mass[i];
-        return;
-    }
-    auto fill = [](const std::vector<double> &a, long n, std::vector<double> &out) {
-        for (long p = 0; p < n; ++p)
-            for (long r = 0; r < n; ++r)
-                for (long c = 0; c < n; ++c)
-                    out[(p * n + r) * n + c] = 1.0 / (0.5 * (a[(p * n + r) * n + c] + a[(p * n + c) * n + r]));
-    };
-    fill(volo, s, inv_volo);
-    fill(nodal_mass, s + 1, inv_mass);
-}
-
 // Node-to-corner lists in (element, corner) order, reference volumes and the
 // element and nodal masses of a filled-in nodelist.
 void HostMesh::derive()
@@ -137,6 +94,30 @@ void HostMesh::derive()
     }
 }
 
+// The coordinate of the cube's i-th of s + 1 planes, LULESH-OMP.cc:3001-3014.
+static double plane_coord(int i, int s) { return i ? 1.125 * double(i) / double(s) : 0.0; }
+
+void sedov_start(int s, int init_mode, double volo0, double *e0, double *dt0)
+{
+    if (init_mode == LULESH_INIT_V2) {
+        // lulesh-2.0.3/lulesh-init.cc:171-182
+        const double ebase = 3.948746e+7;
+        const double scale = double(s) / 45.0;
+        *e0 = ebase * scale * scale * scale;
+        *dt0 = (.5 * std::cbrt(volo0)) / std::sqrt(2.0 * *e0);
+    } else {
+        *e0 = 3.948746e+7;   // LULESH-OMP.cc:3112
+        *dt0 = 1.0e-7;       // LULESH-OMP.cc:3053
+    }
+}
+
+double cube_corner_volume(int s)
+{
+    const double h = plane_coord(1, s);
+    const double x[8] = {0, h, h, 0, 0, h, h, 0}, y[8] = {0, 0, h, h, 0, 0, h, h}, z[8] = {0, 0, 0, 0, h, h, h, h};
+    return host_elem_volume(x, y, z);
+}
+
 void HostMesh::build(int s_, int init_mode)
 {
     s = s_;
@@ -151,10 +132,9 @@ void HostMesh::build(int s_, int init_mode)
     for (int pl = 0; pl < en; ++pl)
         for (int row = 0; row < en; ++row)
             for (int col = 0; col < en; ++col, ++n) {
-                // LULESH-OMP.cc:3001-3014: 1.125*(i)/s, exactly 0 on the first plane
-                x[n] = col ? 1.125 * double(col) / double(s) : 0.0;
-                y[n] = row ? 1.125 * double(row) / double(s) : 0.0;
-                z[n] = pl ? 1.125 * double(pl) / double(s) : 0.0;
+                x[n] = plane_coord(col, s);
+                y[n] = plane_coord(row, s);
+                z[n] = plane_coord(pl, s);
             }
 
     nodelist.assign(8 * ne, 0);
@@ -177,16 +157,7 @@ void HostMesh::build(int s_, int init_mode)
     derive();
 
     origin = 0;
-    if (init_mode == LULESH_INIT_V2) {
-        // lulesh-2.0.3/lulesh-init.cc:171-182
-        const double ebase = 3.948746e+7;
-        const double scale = double(s) / 45.0;
-        e0 = ebase * scale * scale * scale;
-        dt0 = (.5 * std::cbrt(volo[0])) / std::sqrt(2.0 * e0);
-    } else {
-        e0 = 3.948746e+7;   // LULESH-OMP.cc:3112
-        dt0 = 1.0e-7;       // LULESH-OMP.cc:3053
-    }
+    sedov_start(s, init_mode, volo[0], &e0, &dt0);
 
     // symmetry-plane node sets (LULESH-OMP.cc:3114-3125) as a per-node mask
     node_bc.assign(nn, 0);
