@@ -205,6 +205,17 @@ def _ptr(a: np.ndarray | None, ctype=C.c_double):
     return a.ctypes.data_as(C.POINTER(ctype))
 
 
+def _arg(a: np.ndarray):
+    """The array's data for a ``double *`` argument of a call: a quarter of the
+    time of ``_ptr`` (0.3 us, 1.4), which a call with eleven arrays notices.
+    A view over the array's own buffer; read-only, empty and strided arrays
+    have none and go the general way."""
+    try:
+        return C.byref(C.c_double.from_buffer(a))
+    except (TypeError, ValueError, BufferError):
+        return _ptr(a)
+
+
 def _check(rc: int, handle=None):
     if rc == OK:
         return
@@ -447,7 +458,7 @@ class Lulesh:
 
     def get_field(self, name: str) -> np.ndarray:
         out = np.empty(self._len(name))
-        _check(load_library().lulesh_get_field(self._h, name.encode(), _ptr(out), out.size), self._h)
+        _check(load_library().lulesh_get_field(self._h, name.encode(), _arg(out), out.size), self._h)
         return out
 
     def set_field(self, name: str, values) -> None:
@@ -479,13 +490,13 @@ class Lulesh:
 
     def upload(self, dom: Domain):
         a = [np.ascontiguousarray(v, dtype=np.float64) for v in dom.arrays()]
-        _check(load_library().lulesh_upload_domain(self._h, *[_ptr(v) for v in a],
+        _check(load_library().lulesh_upload_domain(self._h, *[_arg(v) for v in a],
                                                    float(dom.time), float(dom.deltatime)), self._h)
 
     def download(self, into: Domain | None = None) -> Domain:
         dom = into or Domain.empty(self.num_elem, self.num_node)
         t, dt = C.c_double(), C.c_double()
-        _check(load_library().lulesh_download_domain(self._h, *[_ptr(v) for v in dom.arrays()],
+        _check(load_library().lulesh_download_domain(self._h, *[_arg(v) for v in dom.arrays()],
                                                      C.byref(t), C.byref(dt)), self._h)
         dom.time, dom.deltatime = t.value, dt.value
         return dom
@@ -575,7 +586,7 @@ class Batch:
         s = int(self.sizes[i])
         n = (s + 1) ** 3 if name in NODE_FIELDS else s ** 3
         out = np.empty(n)
-        _check_batch(load_library().lulesh_batch_get_field(self._h, i, name.encode(), _ptr(out), n), self._h)
+        _check_batch(load_library().lulesh_batch_get_field(self._h, i, name.encode(), _arg(out), n), self._h)
         return out
 
     def zone_cycles(self) -> float:

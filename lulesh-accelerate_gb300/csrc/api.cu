@@ -27,6 +27,7 @@ struct lulesh_ctx {
     int *d_active = nullptr;         // run-loop gate
     int *d_max_cycles = nullptr;
     int *h_stage = nullptr;          // pinned staging ints
+    double *h_state = nullptr;       // mapped pinned buffer for the state of a small mesh, else null
     // run loop
     cudaGraphExec_t run_exec = nullptr;
     int run_mode = 0;                // 0 not built, 1 conditional while node, 2 host-driven chunks
@@ -41,6 +42,13 @@ struct lulesh_ctx {
 
 namespace {
 
+// States of up to so many bytes pass through the pinned buffer, if the host's
+// arrays are pinned themselves (s <= 17), or if any is pageable (s <= 25).
+// The copy into the buffer takes ~35 us per MB, eleven copies from or to
+// pinned arrays 27 us together and pageable ones 90-110: with 0.5 MB either
+// way is as fast for the former (s=18 staged 39 us, copied 38-44), with 2.5
+// MB for the latter (s=30).
+constexpr size_t kStagedPinned = 512 << 10, kStagedPageable = 1536 << 10;
 constexpr int kChunkCycles = 16;     // cycles per graph in the host-driven fallback
 constexpr int kUnroll = 4;           // cycles per pass of the while node, on meshes of up to
 constexpr long kSmallElems = 150000; // so many elements
@@ -172,16 +180,14 @@ int check_launch(lulesh_ctx *ctx)
     return LULESH_OK;
 }
 
+// Clears the errors after the host replaced a field.
 int clear_errors(lulesh_ctx *ctx)
 {
-    DevScalars *h = ctx->h_sc;
-    CK(cudaMemcpyAsync(h, ctx->dom.sc, sizeof(DevScalars), cudaMemcpyDeviceToHost, ctx->stream));
-    CK(cudaStreamSynchronize(ctx->stream));
-    h->err_any = 0;
-    for (int i = 0; i < ERR_NUM; ++i) h->err[i] = 0;
-    h->geo_valid = 0;   // the host may have replaced positions
-    CK(cudaMemcpyAsync(ctx->dom.sc, h, sizeof(DevScalars), cudaMemcpyHostToDevice, ctx->stream));
-    CK(cudaStreamSynchronize(ctx->stream));
+    ScalarSet set{};
+    set.moved = true;   // it may have been positions
+    launch_set_scalars(ctx->dom.sc, set, ctx->stream);
+    int rc = check_launch(ctx);
+    if (rc) return rc;
     ctx->status = LULESH_OK;
     return LULESH_OK;
 }
@@ -203,15 +209,42 @@ int download(lulesh_ctx *ctx, double *dst, const double *src, long n)
 bool is_split(const lulesh_ctx *ctx) { return ctx->precision == LULESH_PRECISION_SPLIT; }
 
 // After the host replaced FP64 node state, refresh the split path's hi/lo
-// copies (a no-op for the FP64 path).
+// copies (nothing to do on the FP64 paths), and wait for all of it.
 int refresh_split(lulesh_ctx *ctx)
 {
-    if (!is_split(ctx)) return LULESH_OK;
-    launch_split_sync(ctx->dom, ctx->stream);
-    int rc = check_launch(ctx);
-    if (rc) return rc;
+    if (is_split(ctx)) {
+        launch_split_sync(ctx->dom, ctx->stream);
+        int rc = check_launch(ctx);
+        if (rc) return rc;
+    }
     CK(cudaStreamSynchronize(ctx->stream));
     return LULESH_OK;
+}
+
+// The fields of the Domain record in the order of the ABI's arguments.
+StateView state_view(const Dom &d, const double *const host[11])
+{
+    StateView v{{d.x, d.y, d.z, d.xd, d.yd, d.zd, d.e, d.p, d.q, d.v, d.ss}, d.nn, d.ne, 0};
+    for (int f = 0; f < 11; ++f) v.present |= (host[f] ? 1u : 0u) << f;
+    return v;
+}
+size_t field_len(const StateView &v, int f) { return f < 6 ? v.nn : v.ne; }
+
+// Does the state pass through the pinned buffer?
+bool staged(const lulesh_ctx *ctx, const double *const host[11])
+{
+    if (!ctx->h_state) return false;
+    if ((6 * (size_t)ctx->nn + 5 * (size_t)ctx->ne) * sizeof(double) <= kStagedPinned) return true;
+    for (int f = 0; f < 11; ++f) {
+        cudaPointerAttributes at{};
+        if (!host[f]) continue;
+        if (cudaPointerGetAttributes(&at, host[f]) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        if (at.type == cudaMemoryTypeUnregistered) return true;
+    }
+    return false;
 }
 
 void nodal(lulesh_ctx *ctx, const Dom &d)
@@ -329,6 +362,7 @@ void lulesh_destroy(lulesh_ctx *ctx)
     for (void *p : ctx->allocs) cudaFree(p);
     if (ctx->h_sc) cudaFreeHost(ctx->h_sc);
     if (ctx->h_stage) cudaFreeHost(ctx->h_stage);
+    if (ctx->h_state) cudaFreeHost(ctx->h_state);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
 }
@@ -356,8 +390,10 @@ int create_context(const HostMesh *m, int s, int init_mode, int precision, const
         ctx->err = std::string("no usable CUDA device: ") + cudaGetErrorString(cudaGetLastError());
         return bail(LULESH_ERR_CUDA);
     }
+    const size_t state = (6 * (size_t)ctx->nn + 5 * (size_t)ctx->ne) * sizeof(double);
     if (cudaMallocHost(&ctx->h_sc, sizeof(DevScalars)) != cudaSuccess ||
-        cudaMallocHost(&ctx->h_stage, 16 * sizeof(int)) != cudaSuccess) {
+        cudaMallocHost(&ctx->h_stage, 16 * sizeof(int)) != cudaSuccess ||
+        (state <= kStagedPageable && cudaMallocHost(&ctx->h_state, state) != cudaSuccess)) {
         ctx->err = "cudaMallocHost failed";
         return bail(LULESH_ERR_CUDA);
     }
@@ -660,23 +696,25 @@ int lulesh_upload_domain(lulesh_ctx *ctx, const double *x, const double *y, cons
                          double time, double deltatime)
 {
     if (!ctx) return LULESH_ERR_ARG;
-    Dom &d = ctx->dom;
+    const Dom &d = ctx->dom;
+    const double *const host[11] = {x, y, z, xd, yd, zd, e, p, q, v, ss};
+    const StateView view = state_view(d, host);
+    ScalarSet set{};
+    set.time = time;
+    set.deltatime = deltatime;
+    set.clock = set.moved = true;
     int rc;
-    const long nn = ctx->nn, ne = ctx->ne;
-    if ((rc = upload(ctx, d.x, x, nn)) || (rc = upload(ctx, d.y, y, nn)) || (rc = upload(ctx, d.z, z, nn)) ||
-        (rc = upload(ctx, d.xd, xd, nn)) || (rc = upload(ctx, d.yd, yd, nn)) || (rc = upload(ctx, d.zd, zd, nn)) ||
-        (rc = upload(ctx, d.e, e, ne)) || (rc = upload(ctx, d.p, p, ne)) || (rc = upload(ctx, d.q, q, ne)) ||
-        (rc = upload(ctx, d.v, v, ne)) || (rc = upload(ctx, d.ss, ss, ne)))
-        return rc;
-    CK(cudaMemcpyAsync(ctx->h_sc, d.sc, sizeof(DevScalars), cudaMemcpyDeviceToHost, ctx->stream));
-    CK(cudaStreamSynchronize(ctx->stream));
-    ctx->h_sc->time = time;
-    ctx->h_sc->deltatime = deltatime;
-    ctx->h_sc->err_any = 0;
-    for (int i = 0; i < ERR_NUM; ++i) ctx->h_sc->err[i] = 0;
-    ctx->h_sc->geo_valid = 0;   // new positions: the geometry cache is stale
-    CK(cudaMemcpyAsync(d.sc, ctx->h_sc, sizeof(DevScalars), cudaMemcpyHostToDevice, ctx->stream));
-    CK(cudaStreamSynchronize(ctx->stream));
+    if (staged(ctx, host)) {
+        double *at = ctx->h_state;
+        for (int f = 0; f < 11; at += field_len(view, f++))
+            if (host[f]) memcpy(at, host[f], field_len(view, f) * sizeof(double));
+        launch_state_in(view, ctx->h_state, d.sc, set, ctx->stream);
+    } else {
+        for (int f = 0; f < 11; ++f)
+            if ((rc = upload(ctx, view.field[f], host[f], field_len(view, f)))) return rc;
+        launch_set_scalars(d.sc, set, ctx->stream);
+    }
+    if ((rc = check_launch(ctx))) return rc;
     ctx->status = LULESH_OK;
     return refresh_split(ctx);
 }
@@ -686,17 +724,25 @@ int lulesh_download_domain(lulesh_ctx *ctx, double *x, double *y, double *z, dou
                            double *time, double *deltatime)
 {
     if (!ctx) return LULESH_ERR_ARG;
-    Dom &d = ctx->dom;
+    const Dom &d = ctx->dom;
+    double *const host[11] = {x, y, z, xd, yd, zd, e, p, q, v, ss};
+    const StateView view = state_view(d, host);
     int rc;
-    const long nn = ctx->nn, ne = ctx->ne;
-    if ((rc = download(ctx, x, d.x, nn)) || (rc = download(ctx, y, d.y, nn)) || (rc = download(ctx, z, d.z, nn)) ||
-        (rc = download(ctx, xd, d.xd, nn)) || (rc = download(ctx, yd, d.yd, nn)) ||
-        (rc = download(ctx, zd, d.zd, nn)) || (rc = download(ctx, e, d.e, ne)) ||
-        (rc = download(ctx, p, d.p, ne)) || (rc = download(ctx, q, d.q, ne)) ||
-        (rc = download(ctx, v, d.v, ne)) || (rc = download(ctx, ss, d.ss, ne)))
-        return rc;
-    CK(cudaMemcpyAsync(ctx->h_sc, d.sc, sizeof(DevScalars), cudaMemcpyDeviceToHost, ctx->stream));
+    const bool through = staged(ctx, host);
+    if (through) {
+        launch_state_out(view, ctx->h_state, d.sc, ctx->h_sc, ctx->stream);
+        if ((rc = check_launch(ctx))) return rc;
+    } else {
+        for (int f = 0; f < 11; ++f)
+            if ((rc = download(ctx, host[f], view.field[f], field_len(view, f)))) return rc;
+        CK(cudaMemcpyAsync(ctx->h_sc, d.sc, sizeof(DevScalars), cudaMemcpyDeviceToHost, ctx->stream));
+    }
     CK(cudaStreamSynchronize(ctx->stream));
+    if (through) {
+        const double *at = ctx->h_state;
+        for (int f = 0; f < 11; at += field_len(view, f++))
+            if (host[f]) memcpy(host[f], at, field_len(view, f) * sizeof(double));
+    }
     if (time) *time = ctx->h_sc->time;
     if (deltatime) *deltatime = ctx->h_sc->deltatime;
     return LULESH_OK;
@@ -718,19 +764,9 @@ int lulesh_get_scalars(lulesh_ctx *ctx, lulesh_scalars *out)
 int lulesh_set_scalars(lulesh_ctx *ctx, const lulesh_scalars *in)
 {
     if (!ctx || !in) return LULESH_ERR_ARG;
-    CK(cudaMemcpyAsync(ctx->h_sc, ctx->dom.sc, sizeof(DevScalars), cudaMemcpyDeviceToHost, ctx->stream));
-    CK(cudaStreamSynchronize(ctx->stream));
-    DevScalars *h = ctx->h_sc;
-    h->time = in->time;
-    h->deltatime = in->deltatime;
-    h->dtcourant = in->dtcourant;
-    h->dthydro = in->dthydro;
-    h->cycle = in->cycle;
-    h->err_any = 0;
-    for (int i = 0; i < ERR_NUM; ++i) h->err[i] = 0;
-    h->courant_key = ~0ULL;
-    h->hydro_key = ~0ULL;
-    CK(cudaMemcpyAsync(ctx->dom.sc, h, sizeof(DevScalars), cudaMemcpyHostToDevice, ctx->stream));
+    launch_set_scalars(ctx->dom.sc, ScalarSet{in->time, in->deltatime, in->dtcourant, in->dthydro, in->cycle, true, true, false},
+                       ctx->stream);
+    if (int rc = check_launch(ctx)) return rc;
     CK(cudaStreamSynchronize(ctx->stream));
     ctx->status = LULESH_OK;
     return LULESH_OK;
@@ -780,7 +816,6 @@ int lulesh_set_field(lulesh_ctx *ctx, const char *name, const double *host, long
         launch_doubles_to_pairs(ctx->dom.fcx, f, n, ctx->stream);
         if (int rc = check_launch(ctx)) return rc;
     }
-    CK(cudaStreamSynchronize(ctx->stream));
     int rc = clear_errors(ctx);
     return rc ? rc : refresh_split(ctx);
 }

@@ -3,12 +3,13 @@
 //
 // Layout.  The instances' nodes and elements are concatenated into flat
 // arrays; every instance's range starts on a multiple of kTile, so a tile of
-// kTile elements (or nodes) belongs to one instance.  Connectivity is
-// rewritten to global indices at upload (nodelist, face neighbours, the
-// node-to-corner slots corner*E_total + element), so the per-element and
-// per-node bodies of the single-instance step run unchanged; only the scalar
-// block they read and write (time step, error words, constraint minima) is
-// the instance's own.
+// kTile elements (or nodes) belongs to one instance.  The node lists
+// hold global indices, and face neighbours and corner slots (corner*E_total +
+// element) are formed from an instance's first element and edge, so the
+// per-element and per-node bodies of the single-instance step run unchanged;
+// only the scalar block they read and write (time step, error words,
+// constraint minima) is the instance's own.  The cubes are set up on the
+// device (mesh_gpu.cu).
 //
 // Execution.  One cycle is: the four step kernels, each a persistent kernel
 // per size class walking that class's list of active tiles (each class's

@@ -47,6 +47,27 @@ void launch_end_cycle(const Dom &d, cudaStream_t st, const CycleEnd &end);
 void launch_build_cube(const Dom &d, const CubeDesc &cube, cudaStream_t st);
 void launch_build_cubes(const Dom &d, const CubeDesc *cubes, const int *etile_cube, const int *ntile_cube, cudaStream_t st);
 
+// The scalars that a call sets, beside clearing the error words.
+struct ScalarSet {
+    double time, deltatime, dtcourant, dthydro;
+    int cycle;
+    bool clock;         // time and deltatime
+    bool constraints;   // dtcourant, dthydro and the cycle count; the minima start afresh
+    bool moved;         // new positions: the geometry cache is stale
+};
+// The fields of the Domain record in the order of lulesh_upload_domain, and
+// which of them a call transfers (bit f).
+struct StateView {
+    double *field[11];
+    int nn, ne;
+    unsigned present;
+};
+void launch_set_scalars(DevScalars *sc, const ScalarSet &set, cudaStream_t st);
+// A whole state between its fields and a mapped host buffer that holds them
+// one after the other (state_io.cu)
+void launch_state_in(const StateView &v, const double *stage, DevScalars *sc, const ScalarSet &set, cudaStream_t st);
+void launch_state_out(const StateView &v, double *stage, const DevScalars *sc, DevScalars *host_sc, cudaStream_t st);
+
 // Plain FP64 path (step_fp64.cu).
 void launch_time_increment(const Dom &d, cudaStream_t st);
 void launch_lagrange_nodal(const Dom &d, cudaStream_t st);
