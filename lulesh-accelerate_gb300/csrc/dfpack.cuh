@@ -353,21 +353,6 @@ __device__ __forceinline__ ModePacks walsh_packs(const CornerPacks &r)
     return {df2_renorm(df2_add(f.u, f.w)), df2_renorm(df2_sub(f.w, f.u)), df2_renorm(df2_sub(f.s, f.t)),
             df_renorm(df_sum(df2_x(f.t), df2_x(f.s)))};
 }
-// The linear modes alone: (M1, M2) and M3.
-struct LinearPacks {
-    df2 m12;
-    df64 m3;
-};
-__device__ __forceinline__ LinearPacks walsh_linear_packs(const CornerPacks &r)
-{
-    const df2 ag = minus_plus(df2_x(r.r15), df2_x(r.r37));
-    const df2 bh = minus_plus(df2_y(r.r15), df2_y(r.r37));
-    const df2 dk = minus_plus(df2_y(r.r26), r.r4);
-    const df64 c = df2_x(r.r26);
-    const df2 z = df2_add(df2_pack(df2_y(dk), c), df2_pack(df2_y(bh), df2_y(ag)));   // k + h, c + g
-    return {df2_renorm(df2_add(plus_minus(c, df2_x(ag)), plus_minus(df2_x(dk), df2_x(bh)))),
-            df_renorm(df_diff(df2_x(z), df2_y(z)))};
-}
 
 // The corner values sum_i s_i(c) F_i of modes F1..F7 in the pairs (F1, F2),
 // (F5, F6), F3, F4 and F7, not renormalised: v[0] = corners 2 and 1, v[1] =

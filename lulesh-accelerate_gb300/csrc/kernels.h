@@ -53,7 +53,7 @@ struct ScalarSet {
     int cycle;
     bool clock;         // time and deltatime
     bool constraints;   // dtcourant, dthydro and the cycle count; the minima start afresh
-    bool moved;         // new positions: the geometry cache is stale
+    bool moved;         // new positions or velocities: the geometry cache is stale
 };
 // The fields of the Domain record in the order of lulesh_upload_domain, and
 // which of them a call transfers (bit f).

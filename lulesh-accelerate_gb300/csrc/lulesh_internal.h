@@ -43,7 +43,7 @@ struct DevScalars {
     int err[ERR_NUM];                    // first offending element + 1, 0 = none
     int run_cycles;                      // cycles done by the current lulesh_run
     int run_max;                         // its cap (<= 0: none)
-    int geo_valid;                       // Dom::geo holds the current positions' geometry
+    int geo_valid;                       // Dom::geo holds what belongs to the current positions and velocities
     int elem_begin;                      // first element of the instance (batches)
     int edge;                            // its edge length s, a structured cube (batches; 0 otherwise)
     int node_begin;                      // its first node (batches)
@@ -122,8 +122,9 @@ inline int arith_of(int precision)
 }
 
 // Words per element of the geometry cache (Dom::geo): in IEEE FP64 the modes
-// and the cross products, in pairs the modes alone.
-inline int geo_words(int df) { return df == kArithDF64 ? 21 : 39; }
+// and the cross products of the positions, in pairs the modes of the positions
+// and velocities.
+inline int geo_words(int df) { return df == kArithDF64 ? 42 : 39; }
 
 // Everything one kernel launch needs, passed by value.
 struct Dom {
@@ -170,7 +171,8 @@ struct Dom {
     // do not change between the two); valid while DevScalars::geo_valid is
     // set.  Null: not kept.  In IEEE FP64 the Walsh modes M1..M7 (21 words)
     // and the six shared cross products (18 words), [39][ne]; with df set the
-    // modes as packed pairs (store_geometry_df).  With df set each word of
+    // modes of the positions and the velocities as packed pairs, [42][ne]
+    // (store_geometry_df).  With df set each word of
     // the corner forces fcx/fcy/fcz, of vdov and arealg and of the six
     // monotonic-Q gradients is a double-float pair (float2) as well: only the
     // step's own kernels read them, and the accessors convert.

@@ -16,7 +16,7 @@
 //                        update (:1613-1683)
 //   k_elem_kinematics_df CalcKinematicsForElems + CalcLagrangeElements +
 //                        CalcMonotonicQGradientsForElems (:1927-2180); keeps
-//                        the geometry as pairs for the next force kernel
+//                        the modes as pairs for the next force kernel
 //
 // What stays FP64: the nodal state (positions, velocities, their update),
 // the element state and the whole material kernel (monotonic-Q limiter,
@@ -45,23 +45,27 @@ __device__ __forceinline__ ModePacks field_modes(const double *__restrict__ f, c
     return walsh_packs(corners_of(c));
 }
 
-// Geometry cache (Dom::geo): the modes of x, y, z in the pairs that the
-// kernels hold them in, three 16-byte planes per coordinate, then the three
+// Geometry cache (Dom::geo): the modes of x, y, z, xd, yd, zd in the pairs
+// that the kernels hold them in, three 16-byte planes per field, then the six
 // M4.  The cross products are formed again from them: 170 instructions
-// against 288 more bytes per element written and read.
+// against 288 more bytes per element written and read.  The velocity modes
+// are worth their 336 bytes: the kinematics kernel has the linear ones in
+// hand and completes them in 6 % more time (1196 -> 1268 us at s=192), and
+// the force kernel is spared its 24 gathers, 21 FP64 differences and as many
+// conversions (1316 -> 1046 us; s=96 172 -> 134, s=47 28.9 -> 23.2).
 __device__ __forceinline__ void store_geometry_df(double *geo, size_t ne, int k, int field, const ModePacks &m)
 {
     ulonglong2 *g = reinterpret_cast<ulonglong2 *>(geo) + (size_t)(3 * field) * ne + k;
     g[0] = make_ulonglong2(m.m12.hi, m.m12.lo);
     g[ne] = make_ulonglong2(m.m56.hi, m.m56.lo);
     g[2 * ne] = make_ulonglong2(m.m73.hi, m.m73.lo);
-    reinterpret_cast<float2 *>(geo + 18 * ne)[field * ne + k] = as_float2(m.m4);
+    reinterpret_cast<float2 *>(geo + 36 * ne)[field * ne + k] = as_float2(m.m4);
 }
 __device__ __forceinline__ ModePacks load_geometry_df(const double *geo, size_t ne, int k, int field)
 {
     const ulonglong2 *g = reinterpret_cast<const ulonglong2 *>(geo) + (size_t)(3 * field) * ne + k;
     const ulonglong2 a = __ldg(g), b = __ldg(g + ne), c = __ldg(g + 2 * ne);
-    return {{a.x, a.y}, {b.x, b.y}, {c.x, c.y}, as_df(__ldg(reinterpret_cast<const float2 *>(geo + 18 * ne) + field * ne + k))};
+    return {{a.x, a.y}, {b.x, b.y}, {c.x, c.y}, as_df(__ldg(reinterpret_cast<const float2 *>(geo + 36 * ne) + field * ne + k))};
 }
 
 // The modes of the three coordinates as vectors.
@@ -122,10 +126,11 @@ __device__ __forceinline__ void elem_force_components(const Dom &d, int k, DevSc
     const double ssk = __ldg(d.ss + k), massk = __ldg(d.elem_mass + k);
     int nl[8];
     load_nodelist(d.nodelist, k, nl);
-    // the modes: kept by the previous cycle's kinematics kernel for these
-    // positions, else formed here by the same function (the same bits)
+    // the modes: kept by the previous cycle's kinematics kernel, else formed
+    // here by the same function (the same bits)
     ModePacks mx, my, mz;
-    if (d.geo && sc->geo_valid) {
+    const bool kept = d.geo && sc->geo_valid;
+    if (kept) {
         mx = load_geometry_df(d.geo, ne, k, 0);
         my = load_geometry_df(d.geo, ne, k, 1);
         mz = load_geometry_df(d.geo, ne, k, 2);
@@ -134,9 +139,9 @@ __device__ __forceinline__ void elem_force_components(const Dom &d, int k, DevSc
         my = field_modes(d.y, nl);
         mz = field_modes(d.z, nl);
     }
-    // the first velocity component's corners, in flight during the geometry
-    double un[8];
-    gather8(dim0 == 0 ? d.xd : (dim0 == 1 ? d.yd : d.zd), nl, un);
+    // the first velocity component's modes, in flight during the geometry
+    ModePacks next;
+    if (kept) next = load_geometry_df(d.geo, ne, k, 3 + dim0);
 
     V2x3 W12, W56, W34;
     V1x3 n1, n2, n3;   // normal generators, times (p + q)/64
@@ -181,8 +186,8 @@ __device__ __forceinline__ void elem_force_components(const Dom &d, int k, DevSc
     }
 
     // One velocity component per iteration, the loop kept rolled (its body
-    // is most of the kernel's instructions); each iteration issues the next
-    // component's corner gather before its own arithmetic.
+    // is most of the kernel's instructions); each iteration issues the loads
+    // of the next component's modes before its own arithmetic.
 #pragma unroll 1
     for (int dim = dim0; dim < dim1; ++dim) {
         // (the component is selected, not indexed, so that it stays in
@@ -194,8 +199,9 @@ __device__ __forceinline__ void elem_force_components(const Dom &d, int k, DevSc
         df2 F12, F56;
         df64 F3, F4, F7;
         if (hourglass) {
-            const ModePacks u = walsh_packs(corners_of(un));
-            if (dim + 1 < dim1) gather8(dim == 0 ? d.yd : d.zd, nl, un);
+            ModePacks u = next;
+            if (!kept) u = field_modes(dim == 0 ? d.xd : (dim == 1 ? d.yd : d.zd), nl);
+            else if (dim + 1 < dim1) next = load_geometry_df(d.geo, ne, k, 4 + dim);
             const df2n u12 = df2_both(u.m12), u56 = df2_both(u.m56), u34 = df2_both(df2_pack(df2_y(u.m73), u.m4));
             auto modes_dot = [&](df2 a, df2 b, df2 c) {
                 return df2_both(df2_dup(joined(Dot2(a, u12).add(b, u56)).plus(joined(Dot2(c, u34))).value()));
@@ -365,8 +371,8 @@ __device__ __forceinline__ void elem_kinematics_parts(const Dom &d, int k, DevSc
     int nl[8];
     load_nodelist(d.nodelist, k, nl);
     const ModePacks mx = field_modes(d.x, nl), my = field_modes(d.y, nl), mz = field_modes(d.z, nl);
-    // the next cycle's force kernel works on these same positions; every
-    // context that runs this kernel keeps the cache
+    // the next cycle's force kernel works on these same positions and
+    // velocities; every context that runs this kernel keeps the cache
     if constexpr (kParts & kVolume) {
         store_geometry_df(d.geo, ne, k, 0, mx);
         store_geometry_df(d.geo, ne, k, 1, my);
@@ -406,20 +412,15 @@ __device__ __forceinline__ void elem_kinematics_parts(const Dom &d, int k, DevSc
     V2x3 V12;   // velocity modes (V1, V2) and V3
     V1x3 V3v;
     {
-        double c[8];
-        LinearPacks u;
-        gather8(d.xd, nl, c);
-        u = walsh_linear_packs(corners_of(c));
-        V12.x = u.m12;
-        V3v.x = u.m3;
-        gather8(d.yd, nl, c);
-        u = walsh_linear_packs(corners_of(c));
-        V12.y = u.m12;
-        V3v.y = u.m3;
-        gather8(d.zd, nl, c);
-        u = walsh_linear_packs(corners_of(c));
-        V12.z = u.m12;
-        V3v.z = u.m3;
+        auto modes = [&](const double *f, int field, df2 &v12, df64 &v3) {
+            const ModePacks u = field_modes(f, nl);
+            if constexpr (kParts & kStrain) store_geometry_df(d.geo, ne, k, field, u);
+            v12 = u.m12;
+            v3 = df2_y(u.m73);
+        };
+        modes(d.xd, 3, V12.x, V3v.x);
+        modes(d.yd, 4, V12.y, V3v.y);
+        modes(d.zd, 5, V12.z, V3v.z);
     }
     const V2x3n V21 = swapped(both(V12));
 
