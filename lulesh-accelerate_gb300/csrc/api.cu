@@ -403,8 +403,9 @@ int create_context(const HostMesh *m, int s, int init_mode, int precision, const
     d.ne = (int)ctx->ne;
     d.nn = (int)ctx->nn;
     d.keep = 0;
-    if (params) d.prm = *params;
-    else default_params(&d.prm);
+    lulesh_params prm;
+    default_params(&prm);
+    set_params(d, params ? *params : prm);
     {
         int sms = 0;
         if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device) != cudaSuccess || sms < 1)
@@ -676,7 +677,7 @@ int lulesh_get_regions(lulesh_ctx *ctx, int *reg_num_list)
 int lulesh_set_params(lulesh_ctx *ctx, const lulesh_params *params)
 {
     if (!ctx || !params) return LULESH_ERR_ARG;
-    ctx->dom.prm = *params;
+    set_params(ctx->dom, *params);
     if (ctx->run_exec) { cudaGraphExecDestroy(ctx->run_exec); ctx->run_exec = nullptr; }
     if (ctx->chunk_exec) { cudaGraphExecDestroy(ctx->chunk_exec); ctx->chunk_exec = nullptr; }
     ctx->run_mode = 0;

@@ -543,8 +543,9 @@ int lulesh_batch_create(int n, const int *sizes, const double *e0_scale, int ini
     d.ne = (int)b->ne_tot;
     d.nn = (int)b->nn_tot;
     d.keep = 0;
-    if (params) d.prm = *params;
-    else default_params(&d.prm);
+    lulesh_params prm;
+    default_params(&prm);
+    set_params(d, params ? *params : prm);
     const size_t ne = b->ne_tot, nn = b->nn_tot;
     int rc;
     d.df = arith_of(precision);

@@ -600,16 +600,16 @@ __device__ __forceinline__ void constraint_keys(double ss, double vdov, double a
 // caller's.
 template <class Fn>
 __device__ __forceinline__ void constraint_keys_df(df64 ss, df64 vdov, df64 arealg, bool moving, bool compressing,
-                                                   const lulesh_params &P,
+                                                   const PairParams &P,
                                                    unsigned long long &kc, unsigned long long &kh)
 {
     kc = ~0ULL;
     kh = ~0ULL;
     if (moving) {
         df64 dtf = ss * ss;
-        if (compressing) dtf = fma(to_df(64.0 * P.qqc * P.qqc) * (arealg * arealg), vdov * vdov, dtf);
+        if (compressing) dtf = fma(as_df(P.qqc64) * (arealg * arealg), vdov * vdov, dtf);
         kc = order_key(to_double(arealg * Fn::rsqrt(dtf)));          // arealg / sqrt(dtf)
-        kh = order_key(to_double(Fn::div(to_df(P.dvovmax), fabs(vdov) + df64(1.e-20))));
+        kh = order_key(to_double(Fn::div(as_df(P.dvovmax), fabs(vdov) + df64(1.e-20))));
     }
 }
 

@@ -278,26 +278,26 @@ struct NewtonFn {
 // rounding toward zero (its 24 leading bits) and scaled by 2^(e-52).
 // Magnitudes outside [2^-74, 2^128), where lo or hi would leave the normal
 // float range, keep hi only (an error below 2^-98 absolute): zeros,
-// infinities and NaNs map to themselves.
+// infinities and NaNs map to themselves.  The small ones by selects in the
+// same instructions, not in a path of their own: zeros stand in most warps
+// (differences along the axes, gas at rest), and a second path took each of
+// those warps through both (at s=192 the plain kinematics kernel 1267 -> 1222
+// us, the split one 921 -> 891).
 __device__ __forceinline__ df64 to_df(double v)
 {
     const unsigned lo32 = (unsigned)__double2loint(v), hi32 = (unsigned)__double2hiint(v);
     const unsigned sign = hi32 & 0x80000000u;
     const unsigned de = (hi32 >> 20) & 0x7ffu;   // biased exponent, e + 1023
-    if (de - 949u <= 201u) {                     // e in [-74, 127]
-        const float hi = __uint_as_float((__funnelshift_r(lo32, hi32, 29) + 0x40000000u) | sign);
-        const int m = (int)hi32 >> 31;            // 0 or -1
-        const int r = (int)(((lo32 & 0x1fffffffu) ^ (unsigned)m) - (unsigned)m);   // +-remainder
-        return {hi, __int2float_rz(r) * __uint_as_float((de - 948u) << 23)};
+    unsigned hb = (__funnelshift_r(lo32, hi32, 29) + 0x40000000u) | sign;
+    const int m = (int)hi32 >> 31;            // 0 or -1
+    const int r = (int)(((lo32 & 0x1fffffffu) ^ (unsigned)m) - (unsigned)m);   // +-remainder
+    unsigned scale = (max(de, 948u) - 948u) << 23;
+    if (de < 897u) hb = sign;
+    if (de > 1150u) {
+        hb = de == 0x7ffu && ((hi32 & 0xfffffu) | lo32) != 0u ? sign | 0x7fc00000u : sign | 0x7f800000u;
+        scale = 0u;
     }
-    // outside the split's range: the high word alone (FP32 truncation,
-    // signed zero below the float range, infinity above, NaN kept)
-    unsigned hb;
-    if (de >= 897u && de <= 1150u) hb = (__funnelshift_r(lo32, hi32, 29) + 0x40000000u) | sign;
-    else if (de < 897u) hb = sign;
-    else if (de == 0x7ffu && ((hi32 & 0xfffffu) | lo32) != 0u) hb = sign | 0x7fc00000u;
-    else hb = sign | 0x7f800000u;
-    return {__uint_as_float(hb), 0.f};
+    return {__uint_as_float(hb), __int2float_rz(r) * __uint_as_float(scale)};
 }
 
 // float -> double with integer operations (normal floats and zeros exact;
@@ -305,12 +305,14 @@ __device__ __forceinline__ df64 to_df(double v)
 __device__ __forceinline__ double df_f2d(float f)
 {
     const unsigned u = __float_as_uint(f);
-    const unsigned long long sign = (unsigned long long)(u & 0x80000000u) << 32;
-    const unsigned fe = (u >> 23) & 0xffu;
-    const unsigned long long mant = (unsigned long long)(u & 0x7fffffu) << 29;
-    if (fe == 0) return __longlong_as_double((long long)sign);
-    const unsigned long long de = (fe == 0xff) ? 0x7ffULL : (unsigned long long)(fe - 127 + 1023);
-    return __longlong_as_double((long long)(sign | (de << 52) | mant));
+    const unsigned fe = u & 0x7f800000u;
+    unsigned hi = (((int)u >> 3) & 0x8fffffffu) + 0x38000000u, lo = u << 29;   // the exponent rebiased by 896
+    if (fe == 0u) {
+        hi = u & 0x80000000u;
+        lo = 0u;
+    }
+    if (fe == 0x7f800000u) hi |= 0x7ff00000u;
+    return __hiloint2double((int)hi, (int)lo);
 }
 
 // pair -> double: one FP64 addition (the correctly rounded sum of the words)

@@ -8,11 +8,10 @@
 namespace lulesh {
 
 // ---- the EOS with its arithmetic in pairs --------------------------------
-// The EOS parameters that the pair arithmetic compares against, converted
-// once per element.
+// The EOS parameters that the pair arithmetic compares against.
 struct EosCuts {
     df64 p_cut, pmin, q_cut;
-    __device__ explicit EosCuts(const lulesh_params &P) : p_cut(to_df(P.p_cut)), pmin(to_df(P.pmin)), q_cut(to_df(P.q_cut)) {}
+    __device__ explicit EosCuts(const PairParams &P) : p_cut(as_df(P.p_cut)), pmin(as_df(P.pmin)), q_cut(as_df(P.q_cut)) {}
 };
 
 // CalcPressureForElems (:2384-2413): p = (2/3)(1 + compression) e with the
@@ -74,7 +73,7 @@ __device__ __forceinline__ double material_update_df(const Dom &d, int k, DevSca
     const double rho0 = P.refdens;
     const bool unit_rho0 = ikey(rho0) == ikey(1.0);
     const double emin = P.emin, e_cut = P.e_cut;
-    const EosCuts cut(P);
+    const EosCuts cut(d.pairs);
     df64 p_new(0.f, 0.f), q_new(0.f, 0.f), ssn(0.f, 0.f), bvc;
     double e_new = 0.0;
     for (int j = 0; j < rep; ++j) {

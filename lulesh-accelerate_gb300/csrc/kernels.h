@@ -26,6 +26,17 @@ inline int node_block(const Dom &d) { return d.nblock ? d.nblock : kBlockNode; }
 // instruction fetch): 4-6 % faster at s=192 in both arithmetics.
 constexpr int kKinBlockFactor = 2;
 inline int kin_block(const Dom &d) { return kKinBlockFactor * elem_block(d); }
+// The material kernels (64 registers, 1024 threads per SM in any split) take
+// larger blocks on larger meshes for the same reason: their waits for
+// instructions were a fifth of a warp's time.  s=192: plain 528 us in blocks
+// of 128 threads, 514 of 256, 495 of 512 (and 4 % more than that in one of
+// 1024), split 492, 473, 465; s=96 77, 74, 74 and 72, 69, 69; s=47, with too
+// few blocks to spread, 15, 15, 17.
+constexpr int kMatBlockFactor = 4;
+inline int mat_block(const Dom &d)
+{
+    return elem_block(d) * (d.ne >= 1000000 ? kMatBlockFactor : d.ne >= 100000 ? 2 : 1);
+}
 // Block sizes for a mesh of ne elements and nn nodes on a GPU with sms SMs:
 // the defaults, halved (down to one warp) while a kernel would have fewer
 // than four blocks per SM -- one FP64-bound element per thread makes the SM

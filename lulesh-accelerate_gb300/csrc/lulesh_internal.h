@@ -126,6 +126,12 @@ inline int arith_of(int precision)
 // and velocities.
 inline int geo_words(int df) { return df == kArithDF64 ? 42 : 39; }
 
+// The parameters that the pair arithmetic takes as pairs (to_df's, df64.cuh),
+// converted once on the host instead of in every thread.
+struct PairParams {
+    float2 limiter_mult, max_slope, qlc_monoq, qqc_monoq, p_cut, pmin, q_cut, qqc64, dvovmax;
+};
+
 // Everything one kernel launch needs, passed by value.
 struct Dom {
     int s, ne, nn;
@@ -181,7 +187,9 @@ struct Dom {
     DevScalars *sc;
     const int *gate;                     // host-driven run loop: cycle runs while *gate != 0
     lulesh_params prm;
+    PairParams pairs;                    // of prm (set_params)
 };
+void set_params(Dom &d, const lulesh_params &p);
 
 // ---- batched ensembles -------------------------------------------------
 // Many independent Sedov instances share flat arrays: each instance's nodes

@@ -52,6 +52,36 @@ void default_params(lulesh_params *p)
     p->refdens = 1.0;
 }
 
+// df64.cuh's to_df on the host: the 24 leading significand bits, then the next
+// 24 of the remaining 29, both truncated.
+static float2 pair_of(double v)
+{
+    float2 r{(float)v, 0.f};
+    const double mag = std::fabs(v);
+    if (!(mag < 3.4028236692093846e38)) return r;   // 2^128, infinities, NaN: the high word alone
+    int e;
+    std::frexp(mag, &e);   // mag = m 2^e, m in [1/2, 1)
+    const double unit = std::ldexp(1.0, e - 24), hi = std::floor(mag / unit) * unit;
+    if (mag < 1.1754943508222875e-38) return {std::copysign(0.f, (float)v), 0.f};   // 2^-126
+    r.x = std::copysign((float)hi, (float)v);
+    if (mag >= 5.2939559203393771e-23) {   // 2^-74
+        const double rest = mag - hi;
+        if (rest != 0.0) {
+            std::frexp(rest, &e);
+            const double u = std::ldexp(1.0, e - 24);
+            r.y = std::copysign((float)(std::floor(rest / u) * u), (float)v);
+        }
+    }
+    return r;
+}
+
+void set_params(Dom &d, const lulesh_params &p)
+{
+    d.prm = p;
+    d.pairs = {pair_of(p.monoq_limiter_mult), pair_of(p.monoq_max_slope), pair_of(p.qlc_monoq), pair_of(p.qqc_monoq),
+               pair_of(p.p_cut), pair_of(p.pmin), pair_of(p.q_cut), pair_of(64.0 * p.qqc * p.qqc), pair_of(p.dvovmax)};
+}
+
 bool pair_field_name(const char *name)
 {
     for (const char *n : {"vdov", "arealg", "delv_xi", "delv_eta", "delv_zeta", "delx_xi", "delx_eta", "delx_zeta"})

@@ -200,7 +200,7 @@ extern "C" int lulesh_lagrange_nodal_noalloc(
     d.fcz = forces + 16 * ne;
     d.sc = reinterpret_cast<DevScalars *>(base + kOffScalars);
     d.gate = nullptr;
-    d.prm = *params;
+    set_params(d, *params);
 
     // the array keeps the previous call's contents: zero the scalar block
     // (error words), everything else is rewritten below before it is read

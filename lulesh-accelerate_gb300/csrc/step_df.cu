@@ -534,14 +534,13 @@ template <bool kConstraints>
 __device__ __forceinline__ void elem_material_df(const Dom &d, int k, DevScalars *sc, unsigned long long &kc,
                                                  unsigned long long &kh)
 {
-    const lulesh_params &P = d.prm;
     const int bc = __ldg(d.elem_bc + k);
     const MaterialIn in = load_material(d, k);
     const double vnew = d.vnew[k], mass = __ldg(d.elem_mass + k), volo = __ldg(d.volo + k);
     auto pairs = [](const double *f) { return reinterpret_cast<const float2 *>(f); };
     const df64 vdov = as_df(pairs(d.vdov)[k]), arealg = as_df(pairs(d.arealg)[k]);
     const FaceNeighbours nb = face_neighbours(d, sc, k);
-    const df64 lim = to_df(P.monoq_limiter_mult), maxs = to_df(P.monoq_max_slope);
+    const df64 lim = as_df(d.pairs.limiter_mult), maxs = as_df(d.pairs.max_slope);
     const float2 *dv_xi = pairs(d.delv_xi), *dv_eta = pairs(d.delv_eta), *dv_zeta = pairs(d.delv_zeta);
     const df64 own_xi = as_df(dv_xi[k]), own_eta = as_df(dv_eta[k]), own_zeta = as_df(dv_zeta[k]);
     // the neighbours' slopes without waiting for the face flags: where a flag
@@ -568,8 +567,8 @@ __device__ __forceinline__ void elem_material_df(const Dom &d, int k, DevScalars
         const df64 lin = (dxi * (one - phixi) + deta * (one - phieta)) + dzeta * (one - phizeta);
         const df64 quad = (dxi * dxi * (one - phixi * phixi) + deta * deta * (one - phieta * phieta)) +
                           dzeta * dzeta * (one - phizeta * phizeta);
-        qlin = -(to_df(P.qlc_monoq) * rho) * lin;
-        qquad = to_df(P.qqc_monoq) * rho * quad;
+        qlin = -(as_df(d.pairs.qlc_monoq) * rho) * lin;
+        qquad = as_df(d.pairs.qqc_monoq) * rho * quad;
     }
     if (d.keep & 2) {
         d.ql[k] = to_double(qlin);
@@ -577,15 +576,16 @@ __device__ __forceinline__ void elem_material_df(const Dom &d, int k, DevScalars
     }
     const double ssn = material_update_df<SeriesFn>(d, k, sc, in, vnew, qlin, qquad, d.reps ? __ldg(d.reps + k) : 1);
     if (kConstraints)
-        constraint_keys_df<SeriesFn>(to_df(ssn), vdov, arealg, vdov.hi != 0.f, vdov.hi < 0.f, P, kc, kh);
+        constraint_keys_df<SeriesFn>(to_df(ssn), vdov, arealg, vdov.hi != 0.f, vdov.hi < 0.f, d.pairs, kc, kh);
 }
 
-// Eight blocks per SM (64 registers, ~40 bytes spilled; 80 registers at six
-// blocks): the kernel waits on its neighbour loads, and the extra warps hide
-// them better than the spills cost (0.88 ms at six blocks, 0.81 at seven,
-// 0.78 at eight, s=192).
+// 32 warps per SM (64 registers, ~40 bytes spilled; 80 registers at 24): the
+// kernel waits on its neighbour loads, and the extra warps hide them better
+// than the spills cost (0.88 ms at 24 warps, 0.81 at 28, 0.78 at 32, s=192,
+// when it took that long).  With cheaper conversions and the parameters'
+// pairs from the host it takes 0.48 ms.
 template <bool kConstraints>
-__global__ void __launch_bounds__(kBlockElem, 8) k_elem_material_df(const __grid_constant__ Dom d)
+__global__ void __launch_bounds__(kMatBlockFactor * kBlockElem, 2) k_elem_material_df(const __grid_constant__ Dom d)
 {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     unsigned long long kc = ~0ULL, kh = ~0ULL;
@@ -626,8 +626,8 @@ void launch_elem_kinematics_df(const Dom &d, cudaStream_t st)
 
 void launch_elem_material_df(const Dom &d, cudaStream_t st, const CycleEnd *end)
 {
-    if (end) k_elem_material_df<true><<<blocks_for(d.ne, elem_block(d)), elem_block(d), 0, st>>>(d);
-    else k_elem_material_df<false><<<blocks_for(d.ne, elem_block(d)), elem_block(d), 0, st>>>(d);
+    if (end) k_elem_material_df<true><<<blocks_for(d.ne, mat_block(d)), mat_block(d), 0, st>>>(d);
+    else k_elem_material_df<false><<<blocks_for(d.ne, mat_block(d)), mat_block(d), 0, st>>>(d);
 }
 
 // Batched ensembles: kernels 0..3 (force, node update, kinematics, material)

@@ -431,7 +431,7 @@ __global__ void __launch_bounds__(kBlockElem) k_time_constraints(const __grid_co
             // vdov and arealg are pairs there (Dom::vdov)
             const df64 v = as_df(reinterpret_cast<const float2 *>(d.vdov)[k]);
             const df64 a = as_df(reinterpret_cast<const float2 *>(d.arealg)[k]);
-            constraint_keys_df<SeriesFn>(to_df(d.ss[k]), v, a, v.hi != 0.f, v.hi < 0.f, d.prm, kc, kh);
+            constraint_keys_df<SeriesFn>(to_df(d.ss[k]), v, a, v.hi != 0.f, v.hi < 0.f, d.pairs, kc, kh);
         }
         else constraint_keys(d.ss[k], d.vdov[k], d.arealg[k], d.prm, kc, kh);
     }

@@ -568,16 +568,17 @@ __device__ __forceinline__ void elem_material_split(const Dom &d, int k, DevScal
         const double ssn = material_update_df<NewtonFn>(d, k, sc, in, vnew, df64(qlin, 0.f), df64(qquad, 0.f),
                                               d.reps ? __ldg(d.reps + k) : 1);
         if (kConstraints)
-            constraint_keys_df<NewtonFn>(to_df(ssn), to_df(vdov), to_df(arealg), iabs(vdov) != 0ULL, lt(vdov, 0.), P,
+            constraint_keys_df<NewtonFn>(to_df(ssn), to_df(vdov), to_df(arealg), iabs(vdov) != 0ULL, lt(vdov, 0.), d.pairs,
                                          kc, kh);
     }
 }
 
-// Eight blocks per SM (64 registers, ~30 bytes spilled): the kernel waits on
-// its neighbour loads, and the extra warps hide them better than the spills
-// cost (0.61 ms at six blocks, 0.56 at seven, 0.55 at eight, s=192).
+// 32 warps per SM (64 registers, ~30 bytes spilled): the kernel waits on its
+// neighbour loads, and the extra warps hide them better than the spills cost
+// (0.61 ms at 24 warps, 0.56 at 28, 0.55 at 32, s=192, when it took that long;
+// 0.47 now).
 template <bool kConstraints>
-__global__ void __launch_bounds__(kBlockElem, 8) k_elem_material_split(const __grid_constant__ Dom d)
+__global__ void __launch_bounds__(kMatBlockFactor * kBlockElem, 2) k_elem_material_split(const __grid_constant__ Dom d)
 {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     unsigned long long kc = ~0ULL, kh = ~0ULL;
@@ -625,8 +626,8 @@ void launch_lagrange_nodal_split(const Dom &d, cudaStream_t st)
 
 static void launch_elem_material_split(const Dom &d, cudaStream_t st, const CycleEnd *end)
 {
-    if (end) k_elem_material_split<true><<<blocks_for(d.ne, elem_block(d)), elem_block(d), 0, st>>>(d);
-    else k_elem_material_split<false><<<blocks_for(d.ne, elem_block(d)), elem_block(d), 0, st>>>(d);
+    if (end) k_elem_material_split<true><<<blocks_for(d.ne, mat_block(d)), mat_block(d), 0, st>>>(d);
+    else k_elem_material_split<false><<<blocks_for(d.ne, mat_block(d)), mat_block(d), 0, st>>>(d);
 }
 
 void launch_lagrange_elements_split(const Dom &d, cudaStream_t st, const CycleEnd *end)
