@@ -25,10 +25,10 @@ struct TileCoord {
     int p, r0, c0;
 };
 
-template <int ROWS>
+template <int ROWS, int COLS = kTileCols>
 struct TileShape {
     static constexpr int kRows = ROWS;
-    static constexpr int kCols = kTileCols;
+    static constexpr int kCols = COLS;
     static constexpr int kNodeCols = kCols + 1, kNodeRows = ROWS + 1;
     static constexpr int kNodes = 2 * kNodeRows * kNodeCols;
     static constexpr int kThreads = ROWS * kCols;
@@ -92,7 +92,12 @@ struct TileShape {
     }
 };
 
-// The single-instance staged kernels' tile: 2 x 64 elements.
-using SoloTile = TileShape<2>;
+// The single-instance staged kernel's tile: a warp per row of 32 elements,
+// four rows.  Against 2 x 64 it stages 2.6 nodes an element instead of 3.0,
+// and the last column of tiles of a cube whose edge is no multiple of 64
+// leaves fewer warps without elements: split force kernel at s=192 371 -> 362
+// us, s=150 217 -> 194, s=130 161 -> 144, s=96 62 -> 57, s=70 36 -> 33 (8 x 16:
+// 369, 201, 139, 57, 30; 8 x 32 in 256 threads: 386, 207, 156, 59, 34).
+using SoloTile = TileShape<4, 32>;
 
 }  // namespace lulesh
