@@ -93,19 +93,6 @@ __device__ __forceinline__ void walsh8(const T c[8], T m[7])
     m[6] = ddp - ddm;    // xi eta zeta
 }
 
-// The three linear modes only (17 additions).
-template <typename T>
-__device__ __forceinline__ void walsh_linear(const T c[8], T m[3])
-{
-    const T s01 = c[0] + c[1], d01 = c[1] - c[0];
-    const T s32 = c[3] + c[2], d32 = c[2] - c[3];
-    const T s45 = c[4] + c[5], d45 = c[5] - c[4];
-    const T s76 = c[7] + c[6], d76 = c[6] - c[7];
-    m[0] = (d01 + d32) + (d45 + d76);
-    m[1] = (s32 - s01) + (s76 - s45);
-    m[2] = (s45 + s76) - (s01 + s32);
-}
-
 template <typename T>
 __device__ __forceinline__ V3<T> mode(const T mx[7], const T my[7], const T mz[7], int i)
 {
@@ -131,6 +118,28 @@ __device__ __forceinline__ void inv_walsh6(T q1, T q2, T q3, T q4, T q5, T q6, T
     v[5] = epm + fpm;
     v[6] = epp + fpp;
     v[7] = emp + fmp;
+}
+
+// Corner values of sum_{i=1..7} s_i(c) F_i (F[0..6] as walsh8 gives the
+// modes), 22 additions.
+template <typename T>
+__device__ __forceinline__ void inv_walsh7(const T F[7], T v[8])
+{
+    // on the face zeta = -+1: +-F3 + A xi + B eta + D xi eta
+    const T Am = F[0] - F[4], Ap = F[0] + F[4];
+    const T Bm = F[1] - F[5], Bp = F[1] + F[5];
+    const T Dm = F[3] - F[6], Dp = F[3] + F[6];
+    const T qm = Dm - F[2], nm = F[2] + Dm;      // nm: negated
+    const T qp = F[2] + Dp, np = F[2] - Dp;
+    const T pm = Am + Bm, dm = Am - Bm, pp = Ap + Bp, dp = Ap - Bp;
+    v[0] = qm - pm;
+    v[1] = dm - nm;
+    v[2] = qm + pm;
+    v[3] = -(dm + nm);
+    v[4] = qp - pp;
+    v[5] = np + dp;
+    v[6] = qp + pp;
+    v[7] = np - dp;
 }
 
 // The six cross products of the modes that the volume, the node normals, the
@@ -160,23 +169,30 @@ __device__ __forceinline__ ModeCrosses<T> mode_crosses(const V3<T> &M1, const V3
 // coefficients are taken three times over (3 W1 = 3 M2xM3 + M4xM5,
 // 3 W4 = M2xM6 + M5xM1, ...) so that no multiplication by 1/3 is needed.
 template <typename T>
+__device__ __forceinline__ void volume_derivative_modes(const V3<T> &M1, const V3<T> &M2, const V3<T> &M3,
+                                                        const V3<T> &M4, const V3<T> &M5, const V3<T> &M6,
+                                                        const ModeCrosses<T> &C, V3<T> W[6])
+{
+    auto add3 = [](const V3<T> &a, T s, const V3<T> &b) {
+        return V3<T>{a.x * s + b.x, a.y * s + b.y, a.z * s + b.z};
+    };
+    W[0] = add3(C.c23, T(3.0), C.c45);
+    W[1] = add3(C.c31, T(3.0), C.c64);
+    W[2] = add3(C.c12, T(3.0), C.c56);
+    W[3] = cross_sum(M2, M6, M5, M1);
+    W[4] = cross_sum(M6, M3, M1, M4);
+    W[5] = cross_sum(M4, M2, M3, M5);
+}
+template <typename T>
 __device__ __forceinline__ void volume_derivative(const V3<T> &M1, const V3<T> &M2, const V3<T> &M3,
                                                   const V3<T> &M4, const V3<T> &M5, const V3<T> &M6,
                                                   const ModeCrosses<T> &C, T dx[8], T dy[8], T dz[8])
 {
-    const V3<T> &c23 = C.c23, &c45 = C.c45, &c31 = C.c31, &c64 = C.c64, &c12 = C.c12, &c56 = C.c56;
-    auto add3 = [](const V3<T> &a, T s, const V3<T> &b) {
-        return V3<T>{a.x * s + b.x, a.y * s + b.y, a.z * s + b.z};
-    };
-    const V3<T> W1 = add3(c23, T(3.0), c45);
-    const V3<T> W2 = add3(c31, T(3.0), c64);
-    const V3<T> W3 = add3(c12, T(3.0), c56);
-    const V3<T> W4 = cross_sum(M2, M6, M5, M1);
-    const V3<T> W5 = cross_sum(M6, M3, M1, M4);
-    const V3<T> W6 = cross_sum(M4, M2, M3, M5);
-    inv_walsh6(W1.x, W2.x, W3.x, W4.x, W5.x, W6.x, dx);
-    inv_walsh6(W1.y, W2.y, W3.y, W4.y, W5.y, W6.y, dy);
-    inv_walsh6(W1.z, W2.z, W3.z, W4.z, W5.z, W6.z, dz);
+    V3<T> W[6];
+    volume_derivative_modes(M1, M2, M3, M4, M5, M6, C, W);
+    inv_walsh6(W[0].x, W[1].x, W[2].x, W[3].x, W[4].x, W[5].x, dx);
+    inv_walsh6(W[0].y, W[1].y, W[2].y, W[3].y, W[4].y, W[5].y, dy);
+    inv_walsh6(W[0].z, W[1].z, W[2].z, W[3].z, W[4].z, W[5].z, dz);
 }
 
 template <typename T>

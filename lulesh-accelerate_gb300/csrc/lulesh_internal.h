@@ -121,10 +121,9 @@ inline int arith_of(int precision)
     return precision == LULESH_PRECISION_FP64 ? kArithDF64 : kArithIEEE;
 }
 
-// Words per element of the geometry cache (Dom::geo): in IEEE FP64 the modes
-// and the cross products of the positions, in pairs the modes of the positions
-// and velocities.
-inline int geo_words(int df) { return df == kArithDF64 ? 42 : 39; }
+// Words per element of the geometry cache (Dom::geo): the modes of the
+// positions and velocities, and in IEEE FP64 the positions' cross products.
+inline int geo_words(int df) { return df == kArithDF64 ? 42 : 60; }
 
 // The parameters that the pair arithmetic takes as pairs (to_df's, df64.cuh),
 // converted once on the host instead of in every thread.
@@ -175,10 +174,10 @@ struct Dom {
     // FP64-state paths: element geometry of the current positions, left by
     // the kinematics kernel for the next cycle's force kernel (the positions
     // do not change between the two); valid while DevScalars::geo_valid is
-    // set.  Null: not kept.  In IEEE FP64 the Walsh modes M1..M7 (21 words)
-    // and the six shared cross products (18 words), [39][ne]; with df set the
-    // modes of the positions and the velocities as packed pairs, [42][ne]
-    // (store_geometry_df).  With df set each word of
+    // set.  Null: not kept.  In IEEE FP64 the Walsh modes M1..M7 of the
+    // positions (21 words), their six shared cross products (18) and the
+    // modes of the velocities (21), [60][ne]; with df set the modes of both as
+    // packed pairs, [42][ne] (store_geometry_df).  With df set each word of
     // the corner forces fcx/fcy/fcz, of vdov and arealg and of the six
     // monotonic-Q gradients is a double-float pair (float2) as well: only the
     // step's own kernels read them, and the accessors convert.

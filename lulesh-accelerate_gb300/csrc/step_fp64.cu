@@ -13,15 +13,16 @@
 //   k_elem_kinematics  1 thr/elem CalcKinematicsForElems + CalcLagrangeElements +
 //                                 CalcMonotonicQGradientsForElems (:1927-2180); keeps
 //                                 the element geometry (Walsh modes and cross products
-//                                 of the new positions) for the next k_elem_force
+//                                 of the new positions, modes of the velocities) for the
+//                                 next k_elem_force
 //   k_elem_material    1 thr/elem CalcMonotonicQRegionForElems, the qstop test,
 //                                 ApplyMaterialPropertiesForElems / EvalEOSForElems /
 //                                 CalcEnergyForElems / CalcSoundSpeedForElems,
 //                                 UpdateVolumesForElems and the Courant/hydro
 //                                 constraint minima (:2182-2933)
-//   k_finalize         1 thread   publishes dtcourant/dthydro (k_run_epilogue in the
-//                                 run loop, which also decides whether another cycle
-//                                 follows)
+//   k_end_cycle        1 thread   publishes dtcourant/dthydro; in the run loop it also
+//                                 decides whether another cycle follows and does its
+//                                 TimeIncrement
 // No floating-point atomics: node sums run in the reference's fixed corner
 // order and the constraint minima use an order-independent integer min.
 #include "lulesh_internal.h"
@@ -45,7 +46,8 @@ __global__ void k_time_increment(const __grid_constant__ Dom d)
 
 // ---------------------------------------------------------------------
 // Geometry cache (Dom::geo): modes M1..M7 of x, y, z, then the six shared
-// cross products, one word per element per plane
+// cross products, then modes M1..M7 of xd, yd, zd, one word per element per
+// plane
 // ---------------------------------------------------------------------
 __device__ __forceinline__ void store_geometry(double *__restrict__ g, size_t ne, int k, const double mx[7],
                                                const double my[7], const double mz[7], const ModeCrosses<double> &X)
@@ -81,140 +83,134 @@ __device__ __forceinline__ void load_geometry(const double *__restrict__ g, size
     X = {c[0], c[1], c[2], c[3], c[4], c[5]};
 }
 
+constexpr int kVelocityModes = 39;   // their first word
+__device__ __forceinline__ void store_velocity_modes(double *__restrict__ g, size_t ne, int k, int dim, const double u[7])
+{
+#pragma unroll
+    for (int i = 0; i < 7; ++i) g[(kVelocityModes + 7 * dim + i) * ne + k] = u[i];
+}
+__device__ __forceinline__ void load_velocity_modes(const double *__restrict__ g, size_t ne, int k, int dim, double u[7])
+{
+#pragma unroll
+    for (int i = 0; i < 7; ++i) u[i] = __ldg(g + (kVelocityModes + 7 * dim + i) * ne + k);
+}
+__device__ __forceinline__ void gather_modes(const double *f, const int nl[8], double m[7])
+{
+    double c[8];
+    gather8(f, nl, c);
+    walsh8(c, m);
+}
+
 // ---------------------------------------------------------------------
-// Element force: stress + Flanagan-Belytschko hourglass
+// Element force: stress + Flanagan-Belytschko hourglass, in the space of the
+// Walsh modes
 // ---------------------------------------------------------------------
+//
+// The kernel is bound by the FP64 pipe, so what counts is its operations.
+// The hourglass shape vectors hourgam_m(c) = gamma_m(c) - (dV/dx_c . H_m)/V
+// (CalcFBHourglassForceForElems, LULESH-OMP.cc:1291-1473) enter the forces
+// through two contractions, with the corner velocities and back to the
+// corners, and both need only the modes: with 192 dV/dx_c = sum_i s_i(c) W_i
+// over i = 1..6, H_m the coordinates' modes 4..7 over 192 V and U_i the modes
+// of one velocity component,
+//   G   = sum_i W_i U_i                    (192 sum_c dV/dx_c u_c)
+//   h_m = coefficient (U_m - H_m . G)
+//   K   = sum_m H_m h_m
+// and the corner forces are the inverse transform of F_i = h_i - W_i . K (h_i
+// = 0 for i < 4; no W_7), the stress forces being linear in the corner signs:
+// Y_i in F_1..F_3.  360 FP64 operations an element with the modes at hand,
+// where forming hourgam at the corners and summing over them takes 480 and
+// the velocities' modes 72 more: 88 -> 69 us at s=45, 618 -> 477 at s=90.
 __device__ __forceinline__ void elem_force_fp64(const Dom &d, int k, DevScalars *sc)
 {
     const size_t ne = (size_t)d.ne;
     int nl[8];
     load_nodelist(d.nodelist, k, nl);
-    // The Walsh modes of the corner coordinates and their shared cross
-    // products: left by the previous cycle's kinematics kernel for these
-    // same positions when it kept them (the same functions of the same
-    // values, so the same bits), else formed here.  The node update that
-    // follows moves the positions and clears the mark.
+    // The modes and the coordinates' cross products: left by the previous
+    // cycle's kinematics kernel for this same state when it kept them (the
+    // same functions of the same values, so the same bits), else formed
+    // here.  The node update that follows moves the state and clears the mark.
     double mx[7], my[7], mz[7];
     ModeCrosses<double> X;
-    if (d.geo && sc->geo_valid) {
+    const bool kept = d.geo && sc->geo_valid;
+    if (kept) {
         load_geometry(d.geo, ne, k, mx, my, mz, X);
     } else {
-        double x[8], y[8], z[8];
-        gather8(d.x, nl, x);
-        gather8(d.y, nl, y);
-        gather8(d.z, nl, z);
-        walsh8(x, mx);
-        walsh8(y, my);
-        walsh8(z, mz);
+        gather_modes(d.x, nl, mx);
+        gather_modes(d.y, nl, my);
+        gather_modes(d.z, nl, mz);
         X = mode_crosses(mode(mx, my, mz, 0), mode(mx, my, mz, 1), mode(mx, my, mz, 2), mode(mx, my, mz, 3),
                          mode(mx, my, mz, 4), mode(mx, my, mz, 5));
     }
     const V3<double> M1 = mode(mx, my, mz, 0), M2 = mode(mx, my, mz, 1), M3 = mode(mx, my, mz, 2);
     const V3<double> M4 = mode(mx, my, mz, 3), M5 = mode(mx, my, mz, 4), M6 = mode(mx, my, mz, 5);
-    double dvdx[8], dvdy[8], dvdz[8];
-    V3<double> nx[3];
-    force_geometry(M1, M2, M3, M4, M5, M6, X, dvdx, dvdy, dvdz, nx);   // 192 x dV/dx, normal generators
+    V3<double> W[6], Y[3];
+    volume_derivative_modes(M1, M2, M3, M4, M5, M6, X, W);
+    normal_generators(X, Y);
 
     // IntegrateStressForElems (LULESH-OMP.cc:853-903): sig = -p - q and the
-    // corner force -sig * (area-weighted node normal).  The normal of the
-    // corner with signs s is (s_xi X1 + s_eta X2 + s_zeta X3)/64, so the
-    // stress forces are s . (Y1, Y2, Y3) with Y = ((p + q)/64) X, and those
-    // of corners 4..7 are the forces of corners 2, 3, 0, 1 negated.  The
+    // corner force -sig * (area-weighted node normal), the normal of the
+    // corner with signs s being (s_xi X1 + s_eta X2 + s_zeta X3)/64.  The
     // Jacobian volume it checks is 8 t.(c x a) = M2.(M3 x M1) / 64; only its
     // sign matters.
-    double Y[3][3];
     {
         const double w = (1.0 / 64.0) * (d.p[k] + d.q[k]);
 #pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            Y[i][0] = w * nx[i].x;
-            Y[i][1] = w * nx[i].y;
-            Y[i][2] = w * nx[i].z;
-        }
+        for (int i = 0; i < 3; ++i) Y[i] = {w * Y[i].x, w * Y[i].y, w * Y[i].z};
         const double determ64 = dot3(M2, X.c31);
         if (determ64 <= 0.0) flag_error(sc, ERR_K1_DETERM, k);
     }
-    // stress force of corners 0..3 in one component (corners 4..7: 2, 3,
-    // 0, 1 negated)
-    auto stress4 = [&](int dim, double f[4]) {
-        const double a = Y[0][dim] + Y[1][dim], b = Y[0][dim] - Y[1][dim], z = Y[2][dim];
-        f[0] = -(a + z);   // (-,-,-)
-        f[1] = b - z;      // (+,-,-)
-        f[2] = a - z;      // (+,+,-)
-        f[3] = -(b + z);   // (-,+,-)
-    };
-    double *out[3] = {d.fcx, d.fcy, d.fcz};
 
     // CalcHourglassControlForElems (:1503-1558)
     const double vk = d.v[k];
     const double determ = d.volo[k] * vk;
     if (vk <= 0.0) flag_error(sc, ERR_K1_VOLUME, k);
-
     const double hourg = d.prm.hgcoef;
-    if (!gt(hourg, 0.0)) {
-#pragma unroll
-        for (int dim = 0; dim < 3; ++dim) {
-            double f[4];
-            stress4(dim, f);
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                out[dim][c * ne + k] = f[c];
-                out[dim][(c ^ 6) * ne + k] = neg(f[c]);
-            }
-        }
-        return;
-    }
-
-    // CalcFBHourglassForceForElems (:1291-1473): hourgam = gamma -
-    // volinv * (dV/dx . hourmod), with hourmod the gamma projections of the
-    // coordinates (modes M6, M5, M4, M7).
-    const double r = rcbrt_fast(determ);                    // determ^(-1/3)
-    const double volinv192 = (r * r * r) * (1.0 / 192.0);   // the 1/192 of the derivative
-    double hg[8][4];
-    {
+    const bool hourglass = gt(hourg, 0.0);
+    V3<double> H[4];   // modes 4..7
+    double coefficient = 0.0;
+    if (hourglass) {
+        const double r = rcbrt_fast(determ);                    // determ^(-1/3)
+        const double vi = (r * r * r) * (1.0 / 192.0);          // the 1/192 of the derivative
         const V3<double> M7 = mode(mx, my, mz, 6);
-        const V3<double> H[4] = {M6, M5, M4, M7};
-        const double gam[4][8] = {
-            { 1.,  1., -1., -1., -1., -1.,  1.,  1.},
-            { 1., -1., -1.,  1., -1.,  1.,  1., -1.},
-            { 1., -1.,  1., -1.,  1., -1.,  1., -1.},
-            {-1.,  1., -1.,  1.,  1., -1.,  1., -1.}};
-#pragma unroll
-        for (int m = 0; m < 4; ++m) {
-            // the projection enters negated, so gamma is the addend of the
-            // three fused multiply-adds
-            const double hx = -(volinv192 * H[m].x), hy = -(volinv192 * H[m].y), hz = -(volinv192 * H[m].z);
-#pragma unroll
-            for (int c = 0; c < 8; ++c)
-                hg[c][m] = fma(dvdz[c], hz, fma(dvdy[c], hy, fma(dvdx[c], hx, gam[m][c])));
-        }
+        H[0] = {vi * M4.x, vi * M4.y, vi * M4.z};
+        H[1] = {vi * M5.x, vi * M5.y, vi * M5.z};
+        H[2] = {vi * M6.x, vi * M6.y, vi * M6.z};
+        H[3] = {vi * M7.x, vi * M7.y, vi * M7.z};
+        coefficient = -hourg * 0.01 * d.ss[k] * d.elem_mass[k] * r;
     }
-    const double coefficient = -hourg * 0.01 * d.ss[k] * d.elem_mass[k] * r;
 
-    // CalcElemFBHourglassForce (:1050-1231), one velocity component at a
-    // time; each corner's stress force is the addend of its hourglass sum
-    // (the reference adds the two node sums instead, :905-926 and
-    // :1475-1496: the same total up to rounding, with one gather instead of
-    // two)
+    // one velocity component at a time
     const double *vel[3] = {d.xd, d.yd, d.zd};
+    double *out[3] = {d.fcx, d.fcy, d.fcz};
+    auto less = [](double a, const V3<double> &u, const V3<double> &v) {   // a - u.v
+        return fma(-u.z, v.z, fma(-u.y, v.y, fma(-u.x, v.x, a)));
+    };
 #pragma unroll
     for (int dim = 0; dim < 3; ++dim) {
-        double u[8];
-        gather8(vel[dim], nl, u);
-        double h[4];
+        auto comp = [&](const V3<double> &v) { return dim == 0 ? v.x : (dim == 1 ? v.y : v.z); };
+        double F[7] = {comp(Y[0]), comp(Y[1]), comp(Y[2]), 0.0, 0.0, 0.0, 0.0};
+        if (hourglass) {
+            double U[7];
+            if (kept) load_velocity_modes(d.geo, ne, k, dim, U);
+            else gather_modes(vel[dim], nl, U);
+            V3<double> G{W[0].x * U[0], W[0].y * U[0], W[0].z * U[0]};
 #pragma unroll
-        for (int m = 0; m < 4; ++m) {
-            double acc = hg[0][m] * u[0];
+            for (int i = 1; i < 6; ++i) G = {fma(W[i].x, U[i], G.x), fma(W[i].y, U[i], G.y), fma(W[i].z, U[i], G.z)};
+            double h[4];
 #pragma unroll
-            for (int c = 1; c < 8; ++c) acc = acc + hg[c][m] * u[c];
-            h[m] = coefficient * acc;
+            for (int m = 0; m < 4; ++m) h[m] = coefficient * less(U[3 + m], H[m], G);
+            V3<double> K{H[0].x * h[0], H[0].y * h[0], H[0].z * h[0]};
+#pragma unroll
+            for (int m = 1; m < 4; ++m) K = {fma(H[m].x, h[m], K.x), fma(H[m].y, h[m], K.y), fma(H[m].z, h[m], K.z)};
+#pragma unroll
+            for (int i = 0; i < 6; ++i) F[i] = less(i < 3 ? F[i] : h[i - 3], W[i], K);
+            F[6] = h[3];
         }
-        double f[4];
-        stress4(dim, f);
-        const double st[8] = {f[0], f[1], f[2], f[3], -f[2], -f[3], -f[0], -f[1]};
+        double f[8];
+        inv_walsh7(F, f);
 #pragma unroll
-        for (int c = 0; c < 8; ++c)
-            out[dim][c * ne + k] = (((st[c] + hg[c][0] * h[0]) + hg[c][1] * h[1]) + hg[c][2] * h[2]) + hg[c][3] * h[3];
+        for (int c = 0; c < 8; ++c) out[dim][c * ne + k] = f[c];
     }
 }
 
@@ -277,31 +273,24 @@ __device__ __forceinline__ void elem_kinematics_fp64(const Dom &d, int k, DevSca
 {
     int nl[8];
     load_nodelist(d.nodelist, k, nl);
-    double x[8], y[8], z[8];
-    gather8(d.x, nl, x);
-    gather8(d.y, nl, y);
-    gather8(d.z, nl, z);
     double mx[7], my[7], mz[7];
-    walsh8(x, mx);
-    walsh8(y, my);
-    walsh8(z, mz);
+    gather_modes(d.x, nl, mx);
+    gather_modes(d.y, nl, my);
+    gather_modes(d.z, nl, mz);
     const V3<double> M1 = mode(mx, my, mz, 0), M2 = mode(mx, my, mz, 1), M3 = mode(mx, my, mz, 2);
-    double vx[3], vy[3], vz[3];
-    {
-        double u[8];
-        gather8(d.xd, nl, u);
-        walsh_linear(u, vx);
-        gather8(d.yd, nl, u);
-        walsh_linear(u, vy);
-        gather8(d.zd, nl, u);
-        walsh_linear(u, vz);
-    }
+    double vx[7], vy[7], vz[7];
+    gather_modes(d.xd, nl, vx);
+    gather_modes(d.yd, nl, vy);
+    gather_modes(d.zd, nl, vz);
+    store_velocity_modes(d.geo, (size_t)d.ne, k, 0, vx);
+    store_velocity_modes(d.geo, (size_t)d.ne, k, 1, vy);
+    store_velocity_modes(d.geo, (size_t)d.ne, k, 2, vz);
     const V3<double> V1{vx[0], vy[0], vz[0]}, V2{vx[1], vy[1], vz[1]}, V3v{vx[2], vy[2], vz[2]};
 
     // CalcKinematicsForElems, volume part (:1950-1964)
     const V3<double> M4 = mode(mx, my, mz, 3), M5 = mode(mx, my, mz, 4), M6 = mode(mx, my, mz, 5);
     const ModeCrosses<double> X = mode_crosses(M1, M2, M3, M4, M5, M6);
-    // The next cycle's force kernel works on these same positions.  Every
+    // The next cycle's force kernel works on this same state.  Every
     // context that runs this kernel keeps the cache (only the nodal-only
     // entry point has none), and the store is unconditional: behind a branch
     // the compiler formed the cross products twice (36 more FP64 operations).
