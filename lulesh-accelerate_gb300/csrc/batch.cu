@@ -368,12 +368,19 @@ int grid_for(const lulesh_batch *b, int cls, int kernel, int block, int per_sm)
 // eight).
 constexpr int kDefaultWaves = 4;
 
+// The kinematics and material kernels start in larger blocks from so many
+// elements, as their single-instance forms do (kin_block, mat_block): fourteen
+// split instances of 0.9M elements in all 275 -> 269 us a cycle, eight FP64
+// ones of 0.48M 256 -> 254; with 0.13M it would cost (78 -> 82).
+constexpr long kWideElems = 300000;
+
 void default_cfg(lulesh_batch *b)
 {
     for (int c = 0; c < kMaxClasses; ++c)
         for (int k = 0; k < kBatchKernels; ++k) {
-            const int per_sm = std::max(1, max_blocks(b, k, 128));
-            b->cfg[c][k] = {128, grid_for(b, c, k, 128, kDefaultWaves * per_sm)};
+            const int block = k >= 2 && b->ne_tot >= kWideElems ? 256 : 128;
+            const int per_sm = std::max(1, max_blocks(b, k, block));
+            b->cfg[c][k] = {block, grid_for(b, c, k, block, kDefaultWaves * per_sm)};
         }
 }
 
