@@ -129,6 +129,20 @@ def algorithmic_bytes(ne: int, nn: int, precision: str = "fp64") -> dict:
     }
 
 
+def design_bytes(ne: int, nn: int, precision: str, kernels: str) -> dict:
+    """``algorithmic_bytes`` with the cache that the kernels keep: it counts
+    39 words per element, the positions' modes and cross products; the
+    double-float kernels keep 42 (the modes of the positions and velocities as
+    pairs), the IEEE ones 60 (both modes and the cross products), and the
+    force kernel then reads neither the node list nor the velocities."""
+    b = algorithmic_bytes(ne, nn, precision)
+    if precision != "split":
+        words = 60 if kernels == "fp64_ieee" else 42
+        b["elem_kinematics"] += 8 * (words - 39) * ne
+        b["elem_force"] += 8 * (words - 39) * ne - 32 * ne - 24 * nn
+    return b
+
+
 def measured_peaks() -> dict:
     p = ROOT / "MEASURED_PEAKS.json"
     if p.exists():
@@ -544,7 +558,7 @@ def main():
         profiles/traffic.json measured for these kernels (default: precision)."""
         pc, kms = ctx.run_profiled(args.profile_cycles)
         per_launch = {k: v / max(pc, 1) for k, v in kms.items()}
-        abytes = algorithmic_bytes(ne, nn, precision)
+        abytes = design_bytes(ne, nn, precision, traffic_key or precision)
         sbytes = step_bytes(ne, nn, precision)
         peaks = measured_peaks()
         top = max(("elem_force", "node_update", "elem_kinematics", "elem_material"), key=lambda k: per_launch[k])

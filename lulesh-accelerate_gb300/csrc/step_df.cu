@@ -257,8 +257,12 @@ __global__ void __launch_bounds__(kBlockElem) k_elem_force_df(const __grid_const
 
 // Meshes that leave most of the SMs' warp slots empty run one thread per
 // element and component (blockIdx.y): the geometry is formed three times, but
-// a thread's chain is 2,200 instructions instead of 4,200, and its length is
-// what the kernel takes there (the kinematics kernel likewise, below).
+// a thread's chain is little more than half as long, and its length is what
+// the kernel takes there.  A cycle at s=10 27.9 us against 29.1 in one thread
+// per element, s=22 30.6 and 31.5, s=24 the same, s=30 34.6 and 33.3.  (The
+// kinematics kernel in three parts, which would convert the positions three
+// times, gains nothing: 28.5 at s=10 and 32.7 against 30.4 at s=19.)
+constexpr int kByComponentElems = 12000;
 __global__ void __launch_bounds__(kBlockElem) k_elem_force_df_by_component(const __grid_constant__ Dom d)
 {
     if (skip_step(d)) return;
@@ -361,11 +365,7 @@ __device__ __forceinline__ df64 face_pair_max(const V1x3 &X, const V1x3 &Y)
     return fmax(df2_x(n), df2_y(n));
 }
 
-// kParts: kVolume the volume, the length and the geometry cache, kGradients
-// the Q gradients, kStrain the strain rate.
-enum : int { kVolume = 1, kGradients = 2, kStrain = 4, kAllParts = 7 };
-template <int kParts>
-__device__ __forceinline__ void elem_kinematics_parts(const Dom &d, int k, DevScalars *sc)
+__device__ __forceinline__ void elem_kinematics_df(const Dom &d, int k, DevScalars *sc)
 {
     const size_t ne = (size_t)d.ne;
     int nl[8];
@@ -373,12 +373,10 @@ __device__ __forceinline__ void elem_kinematics_parts(const Dom &d, int k, DevSc
     const ModePacks mx = field_modes(d.x, nl), my = field_modes(d.y, nl), mz = field_modes(d.z, nl);
     // the next cycle's force kernel works on these same positions and
     // velocities; every context that runs this kernel keeps the cache
-    if constexpr (kParts & kVolume) {
-        store_geometry_df(d.geo, ne, k, 0, mx);
-        store_geometry_df(d.geo, ne, k, 1, my);
-        store_geometry_df(d.geo, ne, k, 2, mz);
-        if (k == sc->elem_begin) sc->geo_valid = 1;
-    }
+    store_geometry_df(d.geo, ne, k, 0, mx);
+    store_geometry_df(d.geo, ne, k, 1, my);
+    store_geometry_df(d.geo, ne, k, 2, mz);
+    if (k == sc->elem_begin) sc->geo_valid = 1;
 
     const Modes M = modes_of(mx, my, mz);
     const Crosses X = crosses_of(M);
@@ -393,13 +391,13 @@ __device__ __forceinline__ void elem_kinematics_parts(const Dom &d, int k, DevSc
     }();
     // volume / volo, as a product with the reciprocal taken at set-up, in
     // FP64: it is state, and one product costs less than its two conversions
-    if constexpr (kParts & kVolume) {
     const double rel = to_double(df_scale(vol64, 1.f / 64.f)) * __ldg(d.inv_volo + k);
     d.vnew[k] = rel;
     d.delv[k] = rel - d.v[k];
     if (rel <= 0.0) flag_error(sc, ERR_K3_VNEW, k);
 
     // CalcElemCharacteristicLength (:1821-1862): 4V / sqrt(max AreaFace)
+    {
         // a = M3xM4, -b = M5xM2, c = M6xM1; Y1 = b - a, Y2 = c + a, Y3 = c + b
         const V2x3 bc = cross2(d56, swapped(M.m12));
         const V1x3 a = cross1(M.m3, M.m4), nb = half_x(bc), c = half_y(bc);
@@ -407,14 +405,12 @@ __device__ __forceinline__ void elem_kinematics_parts(const Dom &d, int k, DevSc
                             face_pair_max(X.n3, sum1(c, minus(nb))));
         reinterpret_cast<float2 *>(d.arealg)[k] = as_float2(df_scale(vol64, 0.25f) * df_rsqrt(f));
     }
-    if constexpr (!(kParts & (kGradients | kStrain))) return;
-
     V2x3 V12;   // velocity modes (V1, V2) and V3
     V1x3 V3v;
     {
         auto modes = [&](const double *f, int field, df2 &v12, df64 &v3) {
             const ModePacks u = field_modes(f, nl);
-            if constexpr (kParts & kStrain) store_geometry_df(d.geo, ne, k, field, u);
+            store_geometry_df(d.geo, ne, k, field, u);
             v12 = u.m12;
             v3 = df2_y(u.m73);
         };
@@ -428,7 +424,7 @@ __device__ __forceinline__ void elem_kinematics_parts(const Dom &d, int k, DevSc
     // are M/4, so each cross product is (M x M')/16 and each velocity
     // difference Mv/4; volo vnew is the volume.  eta and xi in the halves of
     // a pair (M3xM1, M3xM2), zeta beside them.  Kept as pairs (Dom::delv_xi).
-    if constexpr (kParts & kGradients) {
+    {
         const df64 ptiny(1.e-36);
         const df64 vol = df_scale(vol64, 1.f / 64.f);
         // (1/16) (1/4) / (vol + ptiny)
@@ -449,7 +445,7 @@ __device__ __forceinline__ void elem_kinematics_parts(const Dom &d, int k, DevSc
     // CalcKinematicsForElems, strain-rate part (:1975-2020): the half-step
     // Jacobian's columns (M - dt/2 V)/8, the rate their cofactors . V over
     // their determinant (strain_rate, hexmodes.cuh); cof = (CxA, CxB)
-    if constexpr (kParts & kStrain) {
+    {
         const df64 dt2 = to_df(0.5 * sc->deltatime);
         const df2n nd = df2_both(df2_dup(dt2));
         auto back2 = [&](df2 m, df2 v) { return Dot2(v, nd).minus(m).negative(); };
@@ -461,23 +457,6 @@ __device__ __forceinline__ void elem_kinematics_parts(const Dom &d, int k, DevSc
         const df64 num = dot1(cze, V3v).plus(difference(dot2(cof, V21))).value();
         reinterpret_cast<float2 *>(d.vdov)[k] = as_float2(df_div(num, dot1(C, cze).value()));
     }
-}
-
-__device__ __forceinline__ void elem_kinematics_df(const Dom &d, int k, DevScalars *sc)
-{
-    elem_kinematics_parts<kAllParts>(d, k, sc);
-}
-
-// One thread per element and part (blockIdx.y), for the meshes of
-// k_elem_force_df_by_component.
-__global__ void __launch_bounds__(kKinBlockFactor * kBlockElem, 2) k_elem_kinematics_df_by_part(const __grid_constant__ Dom d)
-{
-    if (skip_step(d)) return;
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= d.ne) return;
-    if (blockIdx.y == 0) elem_kinematics_parts<kGradients>(d, k, d.sc);
-    else if (blockIdx.y == 1) elem_kinematics_parts<kVolume>(d, k, d.sc);
-    else elem_kinematics_parts<kStrain>(d, k, d.sc);
 }
 
 __global__ void __launch_bounds__(kKinBlockFactor * kBlockElem, 2) k_elem_kinematics_df(const __grid_constant__ Dom d)
@@ -600,13 +579,12 @@ __global__ void __launch_bounds__(kMatBlockFactor * kBlockElem, 2) k_elem_materi
 // ---------------------------------------------------------------------
 // Launchers
 // ---------------------------------------------------------------------
-constexpr int kByPartElems = 7000;
 static inline unsigned blocks_for(long n, int bs) { return (unsigned)((n + bs - 1) / bs); }
 
 void launch_elem_force_df(const Dom &d, cudaStream_t st)
 {
     const unsigned grid = blocks_for(d.ne, elem_block(d));
-    if (d.ne < kByPartElems) k_elem_force_df_by_component<<<dim3(grid, 3), elem_block(d), 0, st>>>(d);
+    if (d.ne < kByComponentElems) k_elem_force_df_by_component<<<dim3(grid, 3), elem_block(d), 0, st>>>(d);
     else k_elem_force_df<<<grid, elem_block(d), 0, st>>>(d);
 }
 
@@ -619,9 +597,7 @@ void launch_node_update_df(const Dom &d, cudaStream_t st)
 
 void launch_elem_kinematics_df(const Dom &d, cudaStream_t st)
 {
-    const unsigned grid = blocks_for(d.ne, kin_block(d));
-    if (d.ne < kByPartElems) k_elem_kinematics_df_by_part<<<dim3(grid, 3), kin_block(d), 0, st>>>(d);
-    else k_elem_kinematics_df<<<grid, kin_block(d), 0, st>>>(d);
+    k_elem_kinematics_df<<<blocks_for(d.ne, kin_block(d)), kin_block(d), 0, st>>>(d);
 }
 
 void launch_elem_material_df(const Dom &d, cudaStream_t st, const CycleEnd *end)

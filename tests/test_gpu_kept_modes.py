@@ -1,7 +1,7 @@
 """The force kernel's modes kept by the kinematics kernel against modes formed
 from the state: writing a field back unchanged makes the kept ones stale, and
-the step's results stay the same bits (s = 3 and 13 in one thread per element
-and component, the larger ones in one thread per element)."""
+the step's results stay the same bits (s = 3, 13 and 20 in one thread per
+element and component, s = 33 in one thread per element)."""
 from __future__ import annotations
 
 import numpy as np
