@@ -42,13 +42,11 @@ struct lulesh_ctx {
 
 namespace {
 
-// States of up to so many bytes pass through the pinned buffer, if the host's
-// arrays are pinned themselves (s <= 17), or if any is pageable (s <= 25).
-// The copy into the buffer takes ~35 us per MB, eleven copies from or to
-// pinned arrays 27 us together and pageable ones 90-110: with 0.5 MB either
-// way is as fast for the former (s=18 staged 39 us, copied 38-44), with 2.5
-// MB for the latter (s=30).
-constexpr size_t kStagedPinned = 512 << 10, kStagedPageable = 1536 << 10;
+// States of up to so many bytes pass through the pinned buffer when the host's
+// arrays are pageable (s <= 25): the copy into the buffer takes ~35 us per MB,
+// eleven copies from or to pageable arrays 90-110 us, and at 2.5 MB (s=30) the
+// two are even.
+constexpr size_t kStagedState = 1536 << 10;
 constexpr int kChunkCycles = 16;     // cycles per graph in the host-driven fallback
 constexpr int kUnroll = 4;           // cycles per pass of the while node, on meshes of up to
 constexpr long kSmallElems = 150000; // so many elements
@@ -230,21 +228,33 @@ StateView state_view(const Dom &d, const double *const host[11])
 }
 size_t field_len(const StateView &v, int f) { return f < 6 ? v.nn : v.ne; }
 
-// Does the state pass through the pinned buffer?
-bool staged(const lulesh_ctx *ctx, const double *const host[11])
+// How a state crosses: through the context's pinned buffer, directly between
+// the kernel and the host's arrays (all pinned from their first to their last
+// value, and mapped, whose device addresses go to *direct), or copied field by
+// field.
+enum Crossing { kStaged, kDirect, kCopied };
+Crossing crossing(const lulesh_ctx *ctx, const StateView &v, const double *const host[11], HostState *direct)
 {
-    if (!ctx->h_state) return false;
-    if ((6 * (size_t)ctx->nn + 5 * (size_t)ctx->ne) * sizeof(double) <= kStagedPinned) return true;
-    for (int f = 0; f < 11; ++f) {
-        cudaPointerAttributes at{};
-        if (!host[f]) continue;
-        if (cudaPointerGetAttributes(&at, host[f]) != cudaSuccess) {
+    auto mapped = [](const double *p, double **at) {   // 1 pinned and mapped, 0 pageable, -1 anything else
+        cudaPointerAttributes a{};
+        if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
             cudaGetLastError();
-            return false;
+            return -1;
         }
-        if (at.type == cudaMemoryTypeUnregistered) return true;
+        *at = static_cast<double *>(a.devicePointer);
+        return a.type == cudaMemoryTypeUnregistered ? 0 : a.type == cudaMemoryTypeHost && a.devicePointer ? 1 : -1;
+    };
+    Crossing how = kDirect;
+    for (int f = 0; f < 11; ++f) {
+        direct->field[f] = nullptr;
+        if (!host[f]) continue;
+        const size_t last = field_len(v, f) - 1;
+        double *end = nullptr;
+        const int first = mapped(host[f], &direct->field[f]);
+        if (first == 0) return ctx->h_state ? kStaged : kCopied;
+        if (first < 0 || mapped(host[f] + last, &end) != 1 || end != direct->field[f] + last) how = kCopied;
     }
-    return false;
+    return how;
 }
 
 void nodal(lulesh_ctx *ctx, const Dom &d)
@@ -393,7 +403,7 @@ int create_context(const HostMesh *m, int s, int init_mode, int precision, const
     const size_t state = (6 * (size_t)ctx->nn + 5 * (size_t)ctx->ne) * sizeof(double);
     if (cudaMallocHost(&ctx->h_sc, sizeof(DevScalars)) != cudaSuccess ||
         cudaMallocHost(&ctx->h_stage, 16 * sizeof(int)) != cudaSuccess ||
-        (state <= kStagedPageable && cudaMallocHost(&ctx->h_state, state) != cudaSuccess)) {
+        (state <= kStagedState && cudaMallocHost(&ctx->h_state, state) != cudaSuccess)) {
         ctx->err = "cudaMallocHost failed";
         return bail(LULESH_ERR_CUDA);
     }
@@ -705,11 +715,15 @@ int lulesh_upload_domain(lulesh_ctx *ctx, const double *x, const double *y, cons
     set.deltatime = deltatime;
     set.clock = set.moved = true;
     int rc;
-    if (staged(ctx, host)) {
+    HostState direct;
+    const Crossing how = crossing(ctx, view, host, &direct);
+    if (how == kStaged) {
         double *at = ctx->h_state;
         for (int f = 0; f < 11; at += field_len(view, f++))
             if (host[f]) memcpy(at, host[f], field_len(view, f) * sizeof(double));
         launch_state_in(view, ctx->h_state, d.sc, set, ctx->stream);
+    } else if (how == kDirect) {
+        launch_state_from_host(view, direct, d.sc, set, ctx->stream);
     } else {
         for (int f = 0; f < 11; ++f)
             if ((rc = upload(ctx, view.field[f], host[f], field_len(view, f)))) return rc;
@@ -729,9 +743,13 @@ int lulesh_download_domain(lulesh_ctx *ctx, double *x, double *y, double *z, dou
     double *const host[11] = {x, y, z, xd, yd, zd, e, p, q, v, ss};
     const StateView view = state_view(d, host);
     int rc;
-    const bool through = staged(ctx, host);
-    if (through) {
+    HostState direct;
+    const Crossing how = crossing(ctx, view, host, &direct);
+    if (how == kStaged) {
         launch_state_out(view, ctx->h_state, d.sc, ctx->h_sc, ctx->stream);
+        if ((rc = check_launch(ctx))) return rc;
+    } else if (how == kDirect) {
+        launch_state_to_host(view, direct, d.sc, ctx->h_sc, ctx->stream);
         if ((rc = check_launch(ctx))) return rc;
     } else {
         for (int f = 0; f < 11; ++f)
@@ -739,7 +757,7 @@ int lulesh_download_domain(lulesh_ctx *ctx, double *x, double *y, double *z, dou
         CK(cudaMemcpyAsync(ctx->h_sc, d.sc, sizeof(DevScalars), cudaMemcpyDeviceToHost, ctx->stream));
     }
     CK(cudaStreamSynchronize(ctx->stream));
-    if (through) {
+    if (how == kStaged) {
         const double *at = ctx->h_state;
         for (int f = 0; f < 11; at += field_len(view, f++))
             if (host[f]) memcpy(host[f], at, field_len(view, f) * sizeof(double));

@@ -73,7 +73,14 @@ struct StateView {
     int nn, ne;
     unsigned present;
 };
+// The device addresses of the host's arrays, where all of them are pinned.
+struct HostState {
+    double *field[11];
+};
 void launch_set_scalars(DevScalars *sc, const ScalarSet &set, cudaStream_t st);
+// A state between its fields and the host's own pinned arrays
+void launch_state_from_host(const StateView &v, const HostState &host, DevScalars *sc, const ScalarSet &set, cudaStream_t st);
+void launch_state_to_host(const StateView &v, const HostState &host, const DevScalars *sc, DevScalars *host_sc, cudaStream_t st);
 // A whole state between its fields and a mapped host buffer that holds them
 // one after the other (state_io.cu)
 void launch_state_in(const StateView &v, const double *stage, DevScalars *sc, const ScalarSet &set, cudaStream_t st);

@@ -6,7 +6,10 @@
 // nodes (s=8: 28 us from pinned memory, 89 us to pageable memory).  A small
 // state instead passes through a buffer of mapped pinned memory, which one
 // kernel reads or writes directly: 17 us up, 12 us down, and a memory copy on
-// the host, ~35 us per MB.
+// the host, ~35 us per MB.  A larger state in pinned arrays goes the same way
+// without the buffer: the kernel reads or writes the host's own arrays, 22 us
+// against the copy engine's 42 at s=30, 57 against 75 at s=47, 2.99 ms against
+// 3.01 at s=192 (205 GB/s, the link's rate).
 // The scalars go by value with the launch, where reading them back, changing
 // them and writing them took two copies and two waits (17 us, 9 now).
 #include "lulesh_internal.h"
@@ -68,7 +71,53 @@ __global__ void __launch_bounds__(256) k_state_out(const __grid_constant__ State
     if ((v.present >> at.field) & 1) stage[t] = v.field[at.field][at.i];
 }
 
+// One field per blockIdx.y, kPerThread values per thread, all loaded before any
+// is stored: the link's latency is ~2 us.
+constexpr int kPerThread = 4;
+template <bool kIn>
+__device__ __forceinline__ void copy_field(const StateView &v, const HostState &host)
+{
+    const int f = blockIdx.y, n = f < 6 ? v.nn : v.ne;
+    if (!((v.present >> f) & 1)) return;
+    double *to = kIn ? v.field[f] : host.field[f];
+    const double *from = kIn ? host.field[f] : v.field[f];
+    const long first = (long)blockIdx.x * (256 * kPerThread) + threadIdx.x;
+    double x[kPerThread];
+#pragma unroll
+    for (int i = 0; i < kPerThread; ++i)
+        if (first + 256 * i < n) x[i] = from[first + 256 * i];
+#pragma unroll
+    for (int i = 0; i < kPerThread; ++i)
+        if (first + 256 * i < n) to[first + 256 * i] = x[i];
+}
+
+__global__ void __launch_bounds__(256) k_state_from_host(const __grid_constant__ StateView v, const __grid_constant__ HostState host,
+                                                         DevScalars *sc, const __grid_constant__ ScalarSet set)
+{
+    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) set_scalars(sc, set);
+    copy_field<true>(v, host);
+}
+
+__global__ void __launch_bounds__(256) k_state_to_host(const __grid_constant__ StateView v, const __grid_constant__ HostState host,
+                                                       const DevScalars *sc, DevScalars *host_sc)
+{
+    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *host_sc = *sc;
+    copy_field<false>(v, host);
+}
+
+dim3 field_grid(const StateView &v) { return dim3((unsigned)((v.nn + 256L * kPerThread - 1) / (256L * kPerThread)), 11); }
+
 }  // namespace
+
+void launch_state_from_host(const StateView &v, const HostState &host, DevScalars *sc, const ScalarSet &set, cudaStream_t st)
+{
+    k_state_from_host<<<field_grid(v), 256, 0, st>>>(v, host, sc, set);
+}
+
+void launch_state_to_host(const StateView &v, const HostState &host, const DevScalars *sc, DevScalars *host_sc, cudaStream_t st)
+{
+    k_state_to_host<<<field_grid(v), 256, 0, st>>>(v, host, sc, host_sc);
+}
 
 void launch_set_scalars(DevScalars *sc, const ScalarSet &set, cudaStream_t st)
 {

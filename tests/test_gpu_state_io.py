@@ -1,6 +1,6 @@
-"""The Domain record up and down on both sides of the staging limits (through
-the pinned buffer in one kernel up to s = 17, from and to pageable arrays as
-here up to s = 25; larger meshes field by field):
+"""The Domain record up and down on both sides of the staging limit (pageable
+arrays through the pinned buffer in one kernel up to s = 25, larger ones field
+by field), and between a kernel and pinned arrays:
 every bit comes back, arrays left out stay as they are, read-only and strided
 inputs are taken, and the scalars that a call does not set keep their values."""
 from __future__ import annotations
@@ -50,3 +50,37 @@ def test_state_round_trip(pkg, s, precision):
         for k in NODE + ELEM:
             if k != "zd":
                 assert np.array_equal(back[k], a[k]), k
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("s,skip", [(9, 0), (18, 0), (18, 1), (31, 1)])
+def test_pinned_arrays(pkg, s, skip, precision):
+    """Pinned arrays, read and written by the kernel itself: aligned to a value
+    only (skip), one field left out, one pageable among them."""
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(s)
+    with pkg.Lulesh(s, pkg.INIT_V2, precision) as g:
+        def pinned(k):
+            n = g.num_node if k in NODE else g.num_elem
+            t = torch.empty(n + skip, dtype=torch.float64, pin_memory=True)
+            return t, t.numpy()[skip:]
+        keep = {k: pinned(k) for k in NODE + ELEM}
+        a = {k: v for k, (_, v) in keep.items()}
+        for v in a.values():
+            v[:] = rng.standard_normal(v.size)
+        g.upload(pkg.Domain(**a, time=0.5, deltatime=2e-6))
+        for k in NODE + ELEM:
+            assert np.array_equal(g.get_field(k), a[k]), k
+        back = {k: pinned(k) for k in NODE + ELEM}
+        out = pkg.Domain(**{k: v for k, (_, v) in back.items()})
+        out.p = None
+        back["p"][1][:] = -1.0
+        g.download(out)
+        for k in NODE + ELEM:
+            assert np.array_equal(back[k][1], a[k] if k != "p" else np.full(g.num_elem, -1.0)), k
+        assert (out.time, out.deltatime) == (0.5, 2e-6)
+        mixed = pkg.Domain(**{k: v.copy() if k == "q" else v for k, (_, v) in back.items()})
+        mixed.q[:] = 7.0
+        g.upload(mixed)
+        for k in NODE + ELEM:
+            assert np.array_equal(g.get_field(k), getattr(mixed, k)), k
