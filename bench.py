@@ -450,7 +450,7 @@ def config_for(args, ne, nn) -> dict:
     return {"workload": f"sedov_s{args.size}_{args.precision}", "s": args.size,
             "elements": ne, "nodes": nn, "init": "LULESH 2.0 (e0=3.948746e7*(s/45)^3)",
             "cycles_per_step": 1, "precision": args.precision,
-            "l2": "no flush: the state (~5.4 GB) is far larger than the 129 MB L2",
+            "l2": "no flush: the state (~5.8 GB) is far larger than the 129 MB L2",
             "parallelism": "replicas" if args.gpus > 1 else "single", "launch": args.launch}
 
 

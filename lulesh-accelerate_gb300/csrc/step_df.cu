@@ -1,7 +1,7 @@
 // step_df.cu -- the plain path's element geometry and forces in double-float.
 //
-// The plain FP64 step is bound by GB300's FP64 pipe (2 FMA per SM per clock),
-// not by HBM: ~990 FP64 instructions per zone-cycle against ~1.6 kB moved.
+// In IEEE FP64 the step is bound by GB300's FP64 pipe (2 FMA per SM per clock),
+// not by HBM: ~890 FP64 instructions per zone-cycle against ~1.9 kB moved.
 // The element geometry (Walsh modes, cross products, volume derivative, node
 // normals, volume, face areas, strain rate) and the stress and
 // Flanagan-Belytschko hourglass forces are therefore evaluated here as
@@ -18,11 +18,10 @@
 //                        CalcMonotonicQGradientsForElems (:1927-2180); keeps
 //                        the modes as pairs for the next force kernel
 //
-// What stays FP64: the nodal state (positions, velocities, their update),
-// the element state and the whole material kernel (monotonic-Q limiter,
-// EOS, energy, pressure, sound speed, volume update) and the time
-// constraints, plus the corner-relative differences that every geometric
-// quantity starts from: a mode is a signed sum of corner differences, and
+// What stays FP64: the nodal state (positions, velocities, their update), the
+// element state (the material kernel's arithmetic is in pairs, the energy
+// accumulated in FP64: eos_df.cuh), plus the corner-relative differences that
+// every geometric quantity starts from: a mode is a signed sum of corner differences, and
 // the differences of neighbouring coordinates are exact in FP64, so the
 // pairs carry each mode to ~2^-47 of its own size (the FP64 transform of the
 // absolute coordinates carries it to 2^-53 of the coordinates).
@@ -247,6 +246,11 @@ __device__ __forceinline__ void elem_force_components(const Dom &d, int k, DevSc
 
 __device__ __forceinline__ void elem_force_df(const Dom &d, int k, DevScalars *sc) { elem_force_components(d, k, sc, 0, 3); }
 
+// 168 registers, three blocks of 128 threads per SM: the FP32 pipe is 71 %
+// busy, the rest dependent results.  1024 us at s=192 (1865 in scalar pairs
+// over the corners, 1316 on packed pairs over the modes, then the velocities'
+// modes kept); four blocks at 128 registers 1090, blocks of 64 threads 1036, of
+// 192 1105, of 384 1301.
 __global__ void __launch_bounds__(kBlockElem) k_elem_force_df(const __grid_constant__ Dom d)
 {
     if (skip_step(d)) return;
@@ -459,6 +463,13 @@ __device__ __forceinline__ void elem_kinematics_df(const Dom &d, int k, DevScala
     }
 }
 
+// 128 registers, two blocks of 256 threads per SM (kin_block).  The work is
+// spread over the FP32 pipe (52 % busy), the FP64 pipe (43 %: the 42 exact
+// corner differences) and the integer pipe (41 %: their conversions); what
+// remains is dependent results and the gathers.  1224 us at s=192 (1619 in
+// scalar pairs, 1196 on packed pairs, 1268 with the velocities' modes completed
+// and kept, less the conversions' second path); blocks of 192 threads, three
+// per SM, 1255, two of 288 1289, one of 512 1312.
 __global__ void __launch_bounds__(kKinBlockFactor * kBlockElem, 2) k_elem_kinematics_df(const __grid_constant__ Dom d)
 {
     if (skip_step(d)) return;

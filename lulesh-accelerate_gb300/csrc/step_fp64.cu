@@ -1,6 +1,7 @@
 // step_fp64.cu -- the plain FP64 Lagrange leapfrog step on sm_103a.
 //
-// One cycle is six launches on one stream:
+// One cycle is six launches on one stream, five in the run loop (there the
+// TimeIncrement rides in k_end_cycle):
 //   k_time_increment   1 thread   TimeIncrement                (LULESH-OMP.cc:557-604)
 //   k_elem_force       1 thr/elem IntegrateStressForElems + CalcHourglassControlForElems
 //                                 + CalcFBHourglassForceForElems, element half
