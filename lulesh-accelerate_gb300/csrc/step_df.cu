@@ -247,7 +247,7 @@ __device__ __forceinline__ void elem_force_components(const Dom &d, int k, DevSc
 __device__ __forceinline__ void elem_force_df(const Dom &d, int k, DevScalars *sc) { elem_force_components(d, k, sc, 0, 3); }
 
 // 168 registers, three blocks of 128 threads per SM: the FP32 pipe is 71 %
-// busy, the rest dependent results.  1024 us at s=192 (1865 in scalar pairs
+// busy, the rest dependent results.  1024 us at s=192 (1850 in scalar pairs
 // over the corners, 1316 on packed pairs over the modes, then the velocities'
 // modes kept); four blocks at 128 registers 1090, blocks of 64 threads 1036, of
 // 192 1105, of 384 1301.
