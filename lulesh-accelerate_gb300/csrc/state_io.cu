@@ -105,7 +105,13 @@ __global__ void __launch_bounds__(256) k_state_to_host(const __grid_constant__ S
     copy_field<false>(v, host);
 }
 
-dim3 field_grid(const StateView &v) { return dim3((unsigned)((v.nn + 256L * kPerThread - 1) / (256L * kPerThread)), 11); }
+// Wide enough for the longest field: a mesh given by its lists may have more
+// elements than nodes.
+dim3 field_grid(const StateView &v)
+{
+    const long n = v.nn > v.ne ? v.nn : v.ne;
+    return dim3((unsigned)((n + 256L * kPerThread - 1) / (256L * kPerThread)), 11);
+}
 
 }  // namespace
 
