@@ -3,7 +3,9 @@
 #include "lulesh_internal.h"
 #include "kernels.h"
 #include "common.cuh"
+#include "crossing.h"
 
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <cstdio>
@@ -228,33 +230,52 @@ StateView state_view(const Dom &d, const double *const host[11])
 }
 size_t field_len(const StateView &v, int f) { return f < 6 ? v.nn : v.ne; }
 
-// How a state crosses: through the context's pinned buffer, directly between
-// the kernel and the host's arrays (all pinned from their first to their last
-// value, and mapped, whose device addresses go to *direct), or copied field by
-// field.
-enum Crossing { kStaged, kDirect, kCopied };
-Crossing crossing(const lulesh_ctx *ctx, const StateView &v, const double *const host[11], HostState *direct)
+// What the driver knows about a host array.  The runtime tells pinned memory
+// from pageable; the extent of the piece that an address lies in, and whether
+// a kernel may write it, only the driver API tells.
+HostArray describe(const double *p, size_t n)
 {
-    auto mapped = [](const double *p, double **at) {   // 1 pinned and mapped, 0 pageable, -1 anything else
-        cudaPointerAttributes a{};
-        if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
-            cudaGetLastError();
-            return -1;
-        }
-        *at = static_cast<double *>(a.devicePointer);
-        return a.type == cudaMemoryTypeUnregistered ? 0 : a.type == cudaMemoryTypeHost && a.devicePointer ? 1 : -1;
-    };
-    Crossing how = kDirect;
-    for (int f = 0; f < 11; ++f) {
-        direct->field[f] = nullptr;
-        if (!host[f]) continue;
-        const size_t last = field_len(v, f) - 1;
-        double *end = nullptr;
-        const int first = mapped(host[f], &direct->field[f]);
-        if (first == 0) return ctx->h_state ? kStaged : kCopied;
-        if (first < 0 || mapped(host[f] + last, &end) != 1 || end != direct->field[f] + last) how = kCopied;
+    HostArray a{reinterpret_cast<uintptr_t>(p), n * sizeof(double), HostMemory::kOther, 0, 0, 0, false};
+    if (!p) return a;
+    cudaPointerAttributes attr{};
+    if (cudaPointerGetAttributes(&attr, p) != cudaSuccess) {
+        cudaGetLastError();
+        return a;
     }
-    return how;
+    if (attr.type == cudaMemoryTypeUnregistered) a.memory = HostMemory::kPageable;
+    if (attr.type != cudaMemoryTypeHost) return a;
+    a.memory = HostMemory::kPinned;
+    using Query = CUresult (*)(unsigned, CUpointer_attribute *, void **, CUdeviceptr);
+    static const Query query = [] {
+        void *f = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        const cudaError_t e = cudaGetDriverEntryPointByVersion("cuPointerGetAttributes", &f, 12000, cudaEnableDefault, &found);
+        if (e != cudaSuccess) cudaGetLastError();
+        return e == cudaSuccess && found == cudaDriverEntryPointSuccess ? reinterpret_cast<Query>(f) : nullptr;
+    }();
+    CUdeviceptr start = 0;
+    size_t bytes = 0;
+    unsigned access = 0;
+    CUpointer_attribute what[3] = {CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, CU_POINTER_ATTRIBUTE_RANGE_SIZE,
+                                   CU_POINTER_ATTRIBUTE_ACCESS_FLAGS};
+    void *to[3] = {&start, &bytes, &access};
+    // the range is of device addresses, which start where the piece does
+    if (!query || query(3, what, to, reinterpret_cast<CUdeviceptr>(attr.devicePointer)) != CUDA_SUCCESS) return a;
+    a.device = reinterpret_cast<uintptr_t>(attr.devicePointer);
+    a.piece = a.at - (a.device - static_cast<uintptr_t>(start));
+    a.piece_bytes = bytes;
+    a.writable = access == CU_POINTER_ATTRIBUTE_ACCESS_FLAG_READWRITE;
+    return a;
+}
+
+Crossing crossing_of(const lulesh_ctx *ctx, const StateView &v, const double *const host[11], bool to_host, HostState *direct)
+{
+    HostArray a[11];
+    for (int f = 0; f < 11; ++f) {
+        a[f] = describe(host[f], field_len(v, f));
+        direct->field[f] = reinterpret_cast<double *>(a[f].device);
+    }
+    return crossing(a, 11, to_host, ctx->h_state != nullptr);
 }
 
 void nodal(lulesh_ctx *ctx, const Dom &d)
@@ -717,13 +738,13 @@ int lulesh_upload_domain(lulesh_ctx *ctx, const double *x, const double *y, cons
     set.clock = set.moved = true;
     int rc;
     HostState direct;
-    const Crossing how = crossing(ctx, view, host, &direct);
-    if (how == kStaged) {
+    const Crossing how = crossing_of(ctx, view, host, false, &direct);
+    if (how == Crossing::kStaged) {
         double *at = ctx->h_state;
         for (int f = 0; f < 11; at += field_len(view, f++))
             if (host[f]) memcpy(at, host[f], field_len(view, f) * sizeof(double));
         launch_state_in(view, ctx->h_state, d.sc, set, ctx->stream);
-    } else if (how == kDirect) {
+    } else if (how == Crossing::kDirect) {
         launch_state_from_host(view, direct, d.sc, set, ctx->stream);
     } else {
         for (int f = 0; f < 11; ++f)
@@ -745,11 +766,11 @@ int lulesh_download_domain(lulesh_ctx *ctx, double *x, double *y, double *z, dou
     const StateView view = state_view(d, host);
     int rc;
     HostState direct;
-    const Crossing how = crossing(ctx, view, host, &direct);
-    if (how == kStaged) {
+    const Crossing how = crossing_of(ctx, view, host, true, &direct);
+    if (how == Crossing::kStaged) {
         launch_state_out(view, ctx->h_state, d.sc, ctx->h_sc, ctx->stream);
         if ((rc = check_launch(ctx))) return rc;
-    } else if (how == kDirect) {
+    } else if (how == Crossing::kDirect) {
         launch_state_to_host(view, direct, d.sc, ctx->h_sc, ctx->stream);
         if ((rc = check_launch(ctx))) return rc;
     } else {
@@ -758,7 +779,7 @@ int lulesh_download_domain(lulesh_ctx *ctx, double *x, double *y, double *z, dou
         CK(cudaMemcpyAsync(ctx->h_sc, d.sc, sizeof(DevScalars), cudaMemcpyDeviceToHost, ctx->stream));
     }
     CK(cudaStreamSynchronize(ctx->stream));
-    if (how == kStaged) {
+    if (how == Crossing::kStaged) {
         const double *at = ctx->h_state;
         for (int f = 0; f < 11; at += field_len(view, f++))
             if (host[f]) memcpy(host[f], at, field_len(view, f) * sizeof(double));
