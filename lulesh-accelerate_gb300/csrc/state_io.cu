@@ -34,7 +34,8 @@ __device__ void set_scalars(DevScalars *sc, const ScalarSet &v)
         sc->courant_key = ~0ULL;
         sc->hydro_key = ~0ULL;
     }
-    if (v.moved) sc->geo_valid = 0;
+    // an error stops a kinematics launch part way: what it kept is of two states
+    if (v.moved || sc->err_any) sc->geo_valid = 0;
     sc->err_any = 0;
     for (int i = 0; i < ERR_NUM; ++i) sc->err[i] = 0;
 }
