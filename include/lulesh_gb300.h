@@ -193,7 +193,11 @@ int lulesh_set_scalars(lulesh_ctx *ctx, const lulesh_scalars *in);
  * "p" "q" "ql" "qq" "v" "volo" "vnew" "delv" "vdov" "arealg" "ss" "elemMass"
  * "delv_xi" "delv_eta" "delv_zeta" "delx_xi" "delx_eta" "delx_zeta".
  * n must equal the field's length.  "fx/fy/fz" hold the nodal forces of the
- * last LagrangeNodal only when the context keeps them (lulesh_keep_forces). */
+ * last LagrangeNodal only when the context keeps them (lulesh_keep_forces).
+ * The plain FP64 step computes and holds "vdov", "arealg" and the six Q
+ * gradients as pairs of floats (48 significant bits, the floats' range): what
+ * it reads of a value that the host wrote is that; the value itself comes
+ * back as written until a cycle writes the field. */
 int lulesh_get_field(lulesh_ctx *ctx, const char *name, double *host, long n);
 int lulesh_set_field(lulesh_ctx *ctx, const char *name, const double *host, long n);
 int lulesh_keep_forces(lulesh_ctx *ctx, int keep);

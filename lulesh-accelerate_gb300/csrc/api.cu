@@ -12,6 +12,8 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <memory>
+#include <new>
 #include <string>
 #include <vector>
 
@@ -30,6 +32,10 @@ struct lulesh_ctx {
     int *d_max_cycles = nullptr;
     int *h_stage = nullptr;          // pinned staging ints
     double *h_state = nullptr;       // mapped pinned buffer for the state of a small mesh, else null
+    // What the host wrote into a pair field, null once a cycle has written the
+    // field: the accessors give a double back as it came, not to a pair's 48
+    // bits and range.
+    std::unique_ptr<double[]> written[kPairFields];
     // run loop
     cudaGraphExec_t run_exec = nullptr;
     int run_mode = 0;                // 0 not built, 1 conditional while node, 2 host-driven chunks
@@ -153,6 +159,17 @@ int read_status(lulesh_ctx *ctx)
             }
     }
     return LULESH_OK;
+}
+
+// After cycles (the last of them perhaps stopped by an error) and read_status:
+// the kinematics kernel has written the pair fields, unless the only cycle's
+// force kernel stopped it.
+void drop_written(lulesh_ctx *ctx, int cycles)
+{
+    const DevScalars *h = ctx->h_sc;
+    const bool stopped = h->err_any && (h->err[ERR_K1_DETERM] || h->err[ERR_K1_VOLUME]);
+    if (cycles < 1 || (cycles == 1 && stopped)) return;
+    for (auto &w : ctx->written) w.reset();
 }
 
 // A run loop that ended with time < stoptime although the caller's own cap
@@ -833,7 +850,13 @@ int lulesh_get_field(lulesh_ctx *ctx, const char *name, double *host, long n)
                 return LULESH_OK;
             }
     }
-    if (ctx->dom.df == kArithDF64 && pair_field_name(name)) {
+    const int pair = ctx->dom.df == kArithDF64 ? pair_field(name) : -1;
+    if (pair >= 0 && ctx->written[pair]) {
+        CK(cudaMemcpyAsync(host, ctx->written[pair].get(), n * sizeof(double), cudaMemcpyDefault, ctx->stream));
+        CK(cudaStreamSynchronize(ctx->stream));
+        return LULESH_OK;
+    }
+    if (pair >= 0) {
         // through the corner forces' array, which holds nothing between calls
         launch_pairs_to_doubles(f, ctx->dom.fcx, n, ctx->stream);
         if (int rc = check_launch(ctx)) return rc;
@@ -851,9 +874,13 @@ int lulesh_set_field(lulesh_ctx *ctx, const char *name, const double *host, long
     double *f = find_field(ctx, name, &node, &writable);
     if (!f) return fail(ctx, LULESH_ERR_ARG, std::string("unknown field ") + name);
     if (n != (node ? ctx->nn : ctx->ne)) return fail(ctx, LULESH_ERR_ARG, std::string("wrong length for field ") + name);
-    const bool pairs = ctx->dom.df == kArithDF64 && pair_field_name(name);
-    CK(cudaMemcpyAsync(pairs ? ctx->dom.fcx : f, host, n * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
-    if (pairs) {
+    const int pair = ctx->dom.df == kArithDF64 ? pair_field(name) : -1;
+    CK(cudaMemcpyAsync(pair >= 0 ? ctx->dom.fcx : f, host, n * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
+    if (pair >= 0) {
+        std::unique_ptr<double[]> &kept = ctx->written[pair];
+        if (!kept) kept.reset(new (std::nothrow) double[n]);
+        if (!kept) return fail(ctx, LULESH_ERR_ARG, std::string("no host memory for field ") + name);
+        CK(cudaMemcpyAsync(kept.get(), ctx->dom.fcx, n * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
         launch_doubles_to_pairs(ctx->dom.fcx, f, n, ctx->stream);
         if (int rc = check_launch(ctx)) return rc;
     }
@@ -889,7 +916,10 @@ int lulesh_lagrange_elements(lulesh_ctx *ctx)
     elements(ctx, ctx->dom, nullptr);
     ctx->launches += 2;
     int rc = check_launch(ctx);
-    return rc ? rc : read_status(ctx);
+    if (rc) return rc;
+    rc = read_status(ctx);
+    drop_written(ctx, 1);
+    return rc;
 }
 
 int lulesh_calc_time_constraints(lulesh_ctx *ctx)
@@ -911,7 +941,10 @@ int lulesh_lagrange_leapfrog(lulesh_ctx *ctx)
     elements(ctx, ctx->dom, &end);
     ctx->launches += 5;
     int rc = check_launch(ctx);
-    return rc ? rc : read_status(ctx);
+    if (rc) return rc;
+    rc = read_status(ctx);
+    drop_written(ctx, 1);
+    return rc;
 }
 
 int lulesh_run(lulesh_ctx *ctx, int max_cycles, int *cycles_done)
@@ -937,6 +970,7 @@ int lulesh_run(lulesh_ctx *ctx, int max_cycles, int *cycles_done)
     }
     rc = read_status(ctx);
     const int done = ctx->h_sc->run_cycles;
+    drop_written(ctx, done);
     if (cycles_done) *cycles_done = done;
     ctx->launches += 1 + (long long)done * kernels_per_cycle();
     return rc ? rc : short_of_stoptime(ctx, max_cycles, done);
@@ -973,6 +1007,7 @@ int lulesh_run_profiled(lulesh_ctx *ctx, int max_cycles, int *cycles_done, doubl
     }
     for (auto &e : ev) cudaEventDestroy(e);
     if (!rc) rc = read_status(ctx);
+    drop_written(ctx, done);
     if (cycles_done) *cycles_done = done;
     return rc ? rc : short_of_stoptime(ctx, max_cycles, done);
 }

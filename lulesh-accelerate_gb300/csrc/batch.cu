@@ -853,7 +853,7 @@ int lulesh_batch_get_field(lulesh_batch *b, int i, const char *name, double *hos
             if (n != len) return bfail(b, LULESH_ERR_ARG, std::string("wrong length for field ") + name);
             const long off = f.node ? b->noff[i] : b->eoff[i];
             const double *from = f.p + off;
-            if (d.df == kArithDF64 && pair_field_name(name)) {
+            if (d.df == kArithDF64 && pair_field(name) >= 0) {
                 // through the corner forces' array, which holds nothing between calls
                 launch_pairs_to_doubles(from, d.fcx, n, b->stream);
                 BCK(cudaGetLastError());

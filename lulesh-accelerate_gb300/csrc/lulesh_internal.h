@@ -105,8 +105,10 @@ int region_reps(int r, int nr, int cost);
 // order x y z xd yd zd e p v q; LULESH_OK or LULESH_ERR_ARG with *err set.
 int write_domain_file(const char *basename, int s, long ne, long nn, const int *nodelist, int step,
                       double time, const double *const fields[10], std::string *err);
-// Fields that the double-float kernels keep as pairs of floats, by name.
-bool pair_field_name(const char *name);
+// Fields that the double-float kernels keep as pairs of floats: the place of a
+// name among them, -1 for any other.
+constexpr int kPairFields = 8;
+int pair_field(const char *name);
 // The message lulesh_last_error(NULL) returns.
 void set_last_error(const std::string &msg);
 void default_params(lulesh_params *p);

@@ -82,11 +82,13 @@ void set_params(Dom &d, const lulesh_params &p)
                pair_of(p.p_cut), pair_of(p.pmin), pair_of(p.q_cut), pair_of(64.0 * p.qqc * p.qqc), pair_of(p.dvovmax)};
 }
 
-bool pair_field_name(const char *name)
+int pair_field(const char *name)
 {
-    for (const char *n : {"vdov", "arealg", "delv_xi", "delv_eta", "delv_zeta", "delx_xi", "delx_eta", "delx_zeta"})
-        if (!std::strcmp(name, n)) return true;
-    return false;
+    static const char *const names[kPairFields] = {"vdov", "arealg", "delv_xi", "delv_eta",
+                                                   "delv_zeta", "delx_xi", "delx_eta", "delx_zeta"};
+    for (int i = 0; i < kPairFields; ++i)
+        if (!std::strcmp(name, names[i])) return i;
+    return -1;
 }
 
 // Node-to-corner lists in (element, corner) order, reference volumes and the

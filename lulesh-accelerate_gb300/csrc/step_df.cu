@@ -665,7 +665,9 @@ __global__ void __launch_bounds__(256) k_doubles_to_pairs(const double *__restri
     const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const double a = in[i];
-    const float hi = __double2float_rn(a);
+    float hi = __double2float_rn(a);
+    // a strain rate below the floats' range still moves (constraint_keys_df)
+    if (hi == 0.f && a != 0.0) hi = copysignf(__uint_as_float(1u), hi);
     out[i] = make_float2(hi, isfinite(hi) ? __double2float_rn(a - (double)hi) : 0.f);
 }
 void launch_pairs_to_doubles(const double *pairs, double *out, long n, cudaStream_t st)
