@@ -310,6 +310,12 @@ int lulesh_probe_pipe_rates(double *rates);
  * the quotient (strain rate, density, hydro constraint) from a / x. */
 int lulesh_probe_math(double errs[4]);
 
+/* Accuracy of the double-float functions of the plain and split steps, over
+ * 2^20 pairs spread over [2^-40, 2^40): root mean square and largest relative
+ * error of 1/b, a/b, 1/sqrt(a) and sqrt(a) (errs[0..7], as the plain step
+ * forms them) and of the Newton forms of the split step (errs[8..15]). */
+int lulesh_probe_pairs(double errs[16]);
+
 /* ---- LagrangeNodal without allocation ---------------------------------
  * No counterpart in the reference: an addition for callers that cannot
  * allocate GPU memory themselves -- code whose device memory is handed out by

@@ -154,6 +154,7 @@ _SIGNATURES = {
     "lulesh_probe_fp64_peak": (C.c_int, [_dp]),
     "lulesh_probe_pipe_rates": (C.c_int, [_dp]),
     "lulesh_probe_math": (C.c_int, [_dp]),
+    "lulesh_probe_pairs": (C.c_int, [_dp]),
     "lulesh_batch_create": (C.c_int, [C.c_int, _ip, _dp, C.c_int, C.c_int, C.POINTER(Parameters),
                                       C.POINTER(C.c_void_p)]),
     "lulesh_batch_destroy": (None, [C.c_void_p]),
@@ -695,6 +696,16 @@ def probe_math() -> dict:
     e = np.zeros(4)
     _check(load_library().lulesh_probe_math(_ptr(e)))
     return dict(zip(("rcbrt", "sqrt", "rcp", "quot"), e.tolist()))
+
+
+def probe_pairs() -> dict:
+    """(root mean square, largest) relative error of the double-float
+    functions: the plain step's and, with ``newton_`` before the name, the
+    split step's."""
+    e = np.zeros(16)
+    _check(load_library().lulesh_probe_pairs(_ptr(e)))
+    names = [p + f for p in ("", "newton_") for f in ("rcp", "div", "rsqrt", "sqrt")]
+    return dict(zip(names, zip(e[::2].tolist(), e[1::2].tolist())))
 
 
 def probe_pipe_rates() -> dict:

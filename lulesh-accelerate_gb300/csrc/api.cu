@@ -1067,6 +1067,33 @@ int lulesh_probe_math(double errs[4])
     return LULESH_OK;
 }
 
+int lulesh_probe_pairs(double errs[16])
+{
+    if (!errs) return LULESH_ERR_ARG;
+    double *d = nullptr, h[16] = {};   // eight sums of squares, eight bit patterns
+    cudaStream_t st = nullptr;
+    const int n = 1 << 20;
+    if (cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) != cudaSuccess || cudaMalloc(&d, sizeof h) != cudaSuccess) {
+        if (st) cudaStreamDestroy(st);
+        return fail(nullptr, LULESH_ERR_CUDA, "lulesh_probe_pairs: no usable CUDA device");
+    }
+    cudaError_t e = cudaMemsetAsync(d, 0, sizeof h, st);
+    if (e == cudaSuccess) {
+        launch_pair_probe(d, reinterpret_cast<unsigned long long *>(d + 8), n, st);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaMemcpyAsync(h, d, sizeof h, cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    cudaFree(d);
+    cudaStreamDestroy(st);
+    if (e != cudaSuccess) return fail(nullptr, LULESH_ERR_CUDA, std::string("lulesh_probe_pairs: ") + cudaGetErrorString(e));
+    for (int j = 0; j < 8; ++j) {
+        errs[2 * j] = std::sqrt(h[j] / n);
+        errs[2 * j + 1] = h[8 + j];
+    }
+    return LULESH_OK;
+}
+
 int lulesh_probe_pipe_rates(double *rates)
 {
     lulesh_ctx *ctx = nullptr;

@@ -141,22 +141,28 @@ __device__ __forceinline__ float rsqrt_estimate(float a)
 
 // Reciprocal, quotient and roots: one series step from the FP32 estimate
 // instead of two Newton steps carried out in pairs.  The estimate is first
-// refined to a correctly rounded float or next to one; with y that float and
-// e = 1 - b y (or 1 - a y^2) its residual, formed by fused multiply-adds
-// whose large terms cancel exactly, |e| is near 2^-23, so the correction
-// needs only FP32: its roundings enter at 2^-24 |e|, near 2^-47 of the
-// result, and the first neglected term of the series is of order e^3.  Each
-// takes 9-15 FP32 operations where the Newton forms take 72-110 and the
+// refined to a correctly rounded float y or next to one; then its residual,
+// 1 - b y or 1 - a y^2 and so on, below 2^-22, is formed by fused
+// multiply-adds whose large terms cancel exactly, as a float t and a
+// remainder g that also holds the series' second term, and y (t + g) is added
+// to y with one rounding of each word.  The first neglected term is of order
+// t^3; what remains is a rounding or two of the low word, near 2^-49.  Each
+// takes 12-16 FP32 operations where the Newton forms take 72-110 and the
 // reciprocal's correctly rounded estimate is a software routine of its own.
-// Root-mean-square errors over random pairs: 1/b 2^-49.0, a/b 2^-48.5,
-// 1/sqrt(a) 2^-49.1, sqrt(a) 2^-48.5, within a quarter bit of the Newton
-// forms' (tests/test_df_functions.py).
+// Errors over 2^20 pairs (lulesh_probe_pairs), root mean square and largest,
+// the Newton forms' in brackets: 1/b 2^-49.6 and 2^-47.1 (-48.8, -46.0), a/b
+// 2^-49.5 and 2^-46.7 (-48.5, -45.5), 1/sqrt(a) 2^-49.4 and 2^-46.4 (-49.2,
+// -46.3), sqrt(a) 2^-49.1 and 2^-46.0 (-48.3, -45.5).  With the residual in
+// one float, three operations fewer, 1/b and 1/sqrt(a) were a fifth of a bit
+// above the Newton forms' instead, sqrt(a) a quarter at worst; the material
+// kernel takes 504 us for 486 at s=192 with the remainders (68.0 for 67.6 at
+// s=96), the kinematics kernel 1221 for 1228.
 
-// y + s t (|s t| << |y|) with one rounding of each word
-__device__ __forceinline__ df64 df_corrected(float y, float s, float t)
+// y + s (t + g), |s t| << |y|, |g| << |t|, with one rounding of each word
+__device__ __forceinline__ df64 df_corrected(float y, float s, float t, float g)
 {
     const float hi = __fmaf_rn(s, t, y);
-    return {hi, __fmaf_rn(s, t, __fsub_rn(y, hi))};
+    return {hi, __fmaf_rn(s, g, __fmaf_rn(s, t, __fsub_rn(y, hi)))};
 }
 
 // 1/b = y (1 + e + e^2 + ...)
@@ -164,8 +170,8 @@ __device__ __forceinline__ df64 df_rcp(df64 b)
 {
     const float y0 = rcp_estimate(b.hi);
     const float y = __fmaf_rn(y0, __fmaf_rn(-b.hi, y0, 1.f), y0);
-    const float e = __fmaf_rn(-b.lo, y, __fmaf_rn(-b.hi, y, 1.f));
-    return df_corrected(y, y, __fmaf_rn(e, e, e));
+    const float e = __fmaf_rn(-b.hi, y, 1.f), t = __fmaf_rn(-b.lo, y, e);
+    return df_corrected(y, y, t, __fmaf_rn(t, t, __fmaf_rn(-b.lo, y, __fsub_rn(e, t))));
 }
 
 // a/b: the FP32 quotient q by the refined reciprocal y, then its remainder
@@ -176,8 +182,8 @@ __device__ __forceinline__ df64 df_div(df64 a, df64 b)
     const float y = __fmaf_rn(y0, __fmaf_rn(-b.hi, y0, 1.f), y0);
     const float e = __fmaf_rn(-b.lo, y, __fmaf_rn(-b.hi, y, 1.f));
     const float q = __fmul_rn(a.hi, y);
-    const float r = __fadd_rn(__fmaf_rn(-b.hi, q, a.hi), __fmaf_rn(-b.lo, q, a.lo));
-    return df_corrected(q, y, __fmaf_rn(r, e, r));
+    const float r = __fmaf_rn(-b.hi, q, a.hi), f = __fmaf_rn(-b.lo, q, a.lo), t = __fadd_rn(r, f);
+    return df_corrected(q, y, t, __fmaf_rn(t, e, __fadd_rn(__fsub_rn(r, t), f)));
 }
 
 // 1/sqrt(a) = y (1 + e/2 + 3 e^2/8 + ...), a > 0
@@ -186,19 +192,24 @@ __device__ __forceinline__ df64 df_rsqrt(df64 a)
     const float y0 = rsqrt_estimate(a.hi);
     const float y = __fmaf_rn(__fmul_rn(0.5f, y0), __fmaf_rn(-a.hi, __fmul_rn(y0, y0), 1.f), y0);
     const df64 s = two_prod(y, y);
-    const float e = __fadd_rn(__fmaf_rn(-a.hi, s.hi, 1.f), __fmaf_rn(-a.lo, s.hi, __fmul_rn(-a.hi, s.lo)));
-    return df_corrected(y, __fmul_rn(0.5f, y), __fmaf_rn(__fmul_rn(0.75f, e), e, e));
+    const float e = __fmaf_rn(-a.hi, s.hi, 1.f), f = __fmaf_rn(-a.lo, s.hi, __fmul_rn(-a.hi, s.lo));
+    const float t = __fadd_rn(e, f);
+    return df_corrected(y, __fmul_rn(0.5f, y), t, __fmaf_rn(__fmul_rn(0.75f, t), t, __fadd_rn(__fsub_rn(e, t), f)));
 }
 
 // sqrt(a), a > 0: the FP32 root x by the refined inverse root y, then its
-// remainder a - x^2 (exact in its high words) times y/2
+// remainder r = a - x^2 (exact in its high words) times y/2 (1 + 3 u/4), u =
+// 1 - x y: of the factor's own error, that much and a quarter of x's rounding
+// is left
 __device__ __forceinline__ df64 df_sqrt(df64 a)
 {
     const float y0 = rsqrt_estimate(a.hi);
     const float y = __fmaf_rn(__fmul_rn(0.5f, y0), __fmaf_rn(-a.hi, __fmul_rn(y0, y0), 1.f), y0);
-    const float x = __fmul_rn(a.hi, y);
-    const float r = __fadd_rn(__fmaf_rn(-x, x, a.hi), a.lo);
-    return df_corrected(x, __fmul_rn(0.5f, y), r);
+    const float x = __fmul_rn(a.hi, y), u = __fmaf_rn(-x, y, 1.f);
+    const float r = __fmaf_rn(-x, x, a.hi), t = __fadd_rn(r, a.lo), h = __fmul_rn(0.5f, y);
+    const float hi = __fmaf_rn(h, t, x);
+    // (r and a.lo apart: this one needs no exact remainder of their sum)
+    return {hi, __fmaf_rn(h, __fmaf_rn(t, __fmul_rn(0.75f, u), a.lo), __fmaf_rn(h, r, __fsub_rn(x, hi)))};
 }
 
 // The Newton forms: two steps r <- r + r (1 - b r) or y <- y + y (1 - a y^2)/2

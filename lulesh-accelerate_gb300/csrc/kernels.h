@@ -104,6 +104,8 @@ void launch_cycle_timed(const Dom &d, cudaStream_t st, cudaEvent_t ev[kTimedKern
 // exact sum, a double its FP32 rounding and the remainder's.
 void launch_pairs_to_doubles(const double *pairs, double *out, long n, cudaStream_t st);
 void launch_doubles_to_pairs(const double *in, double *pairs, long n, cudaStream_t st);
+// lulesh_probe_pairs (step_df.cu)
+void launch_pair_probe(double *sums, unsigned long long *worst, int n, cudaStream_t st);
 void launch_fp64_probe(double *out, int blocks, int threads, int iters, cudaStream_t st);
 void launch_rate_probe(int which, float *out, int blocks, int threads, int iters, cudaStream_t st);
 // largest relative differences (as order keys of non-negative doubles) of the

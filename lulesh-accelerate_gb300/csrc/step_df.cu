@@ -679,4 +679,54 @@ void launch_doubles_to_pairs(const double *in, double *pairs, long n, cudaStream
     k_doubles_to_pairs<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(in, reinterpret_cast<float2 *>(pairs), n);
 }
 
+// ---------------------------------------------------------------------
+// Accuracy of the pairs' reciprocal, quotient and roots: squared relative
+// errors summed into sums[0..7] and the largest (as bit patterns) in
+// worst[0..7], 1/b, a/b, 1/sqrt(a), sqrt(a) by SeriesFn, then by NewtonFn,
+// over n pairs spread over [2^-40, 2^40).  A pair's sum fits a double but for
+// a rounding of 2^-53, so the defining equation in FP64, each product's
+// remainder included, gives its error to that.
+// ---------------------------------------------------------------------
+__device__ __forceinline__ unsigned long long mixed(unsigned long long z)   // Steele, Lea and Flood's splitmix64
+{
+    z += 0x9e3779b97f4a7c15ULL;
+    z = (z ^ (z >> 30)) * 0xbf58476d1ce4e5b9ULL;
+    z = (z ^ (z >> 27)) * 0x94d049bb133111ebULL;
+    return z ^ (z >> 31);
+}
+template <class Fn>
+__device__ void pair_errors(df64 a, df64 b, double err[4])
+{
+    auto sum = [](df64 v) { return (double)v.hi + (double)v.lo; };
+    const double x = sum(a), y = sum(b);
+    const double rcp = sum(Fn::rcp(b)), quot = sum(Fn::div(a, b)), irt = sum(Fn::rsqrt(a)), root = sum(Fn::sqrt(a));
+    const double sq = irt * irt, sq_rest = fma(irt, irt, -sq);
+    err[0] = fma(y, rcp, -1.0);
+    err[1] = fma(y, quot, -x) / x;
+    err[2] = 0.5 * fma(sq_rest, x, fma(sq, x, -1.0));
+    err[3] = 0.5 * fma(root, root, -x) / x;
+}
+__global__ void __launch_bounds__(256) k_pair_probe(double *sums, unsigned long long *worst, int n)
+{
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    if (i >= n) return;
+    auto value = [&](unsigned long long k) {
+        const unsigned long long r = mixed(2ULL * i + k);
+        return to_df(ldexp(1.0 + (double)(r >> 11) * 0x1p-53, (int)(mixed(r) % 80) - 40));
+    };
+    const df64 a = value(0), b = value(1);
+    double err[8];
+    pair_errors<SeriesFn>(a, b, err);
+    pair_errors<NewtonFn>(a, b, err + 4);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        atomicAdd(sums + j, err[j] * err[j]);
+        atomicMax(worst + j, (unsigned long long)__double_as_longlong(::fabs(err[j])));
+    }
+}
+void launch_pair_probe(double *sums, unsigned long long *worst, int n, cudaStream_t st)
+{
+    k_pair_probe<<<(n + 255) / 256, 256, 0, st>>>(sums, worst, n);
+}
+
 }  // namespace lulesh
