@@ -547,7 +547,6 @@ int create_context(const HostMesh *m, int s, int init_mode, int precision, const
         const std::vector<int> *lists[6] = {&m->lxim, &m->lxip, &m->letam, &m->letap, &m->lzetam, &m->lzetap};
         for (int i = 0; i < 6; ++i) ok = ok && up(nb[i], lists[i]->data(), ne * 4);
     } else {
-        settle_heap(ctx->ne);
         sedov_start(s, init_mode, cube_corner_volume(s), &e0, &dt0);
         if (ok) {
             launch_build_cube(d, CubeDesc{s, 0, 0, e0}, st);

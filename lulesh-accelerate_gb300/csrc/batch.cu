@@ -629,7 +629,6 @@ int lulesh_batch_create(int n, const int *sizes, const double *e0_scale, int ini
     };
     std::vector<int> iee_h(n), ine_h(n);
     std::vector<CubeDesc> cubes(n);
-    settle_heap(*std::max_element(b->ne_i.begin(), b->ne_i.end()));
     for (int i = 0; i < n; ++i) {
         double e0, dt0;
         sedov_start(sizes[i], init_mode, cube_corner_volume(sizes[i]), &e0, &dt0);

@@ -82,8 +82,6 @@ double host_elem_volume(const double x[8], const double y[8], const double z[8])
 // corner element has volume volo0 (cube_corner_volume).
 void sedov_start(int s, int init_mode, double volo0, double *e0, double *dt0);
 double cube_corner_volume(int s);
-// Prepares the C heap for host arrays of a mesh of ne elements (mesh.cpp).
-void settle_heap(long ne);
 
 // Carves device arrays out of one allocation, each on a 256-byte boundary:
 // the same sequence of take() calls first on a null base, for the size.

@@ -150,25 +150,6 @@ double cube_corner_volume(int s)
     return host_elem_volume(x, y, z);
 }
 
-// glibc takes blocks above a threshold, at first 128 kB, straight from the
-// kernel, page by zeroed page at their first touch, and raises the threshold to
-// the size of any such block that is freed (up to 32 MB), keeping twice that of
-// freed heap.  The set-up of a cube on the host freed blocks of 32 bytes an
-// element, so that the arrays of a functional step -- eleven fresh ones a call
-// -- mostly came from the heap afterwards; the set-up on the device has none,
-// and at s=86 those arrays' page faults could take a step from 1.4 to 3.1 ms.
-// So one such block is taken and given back, for meshes whose arrays are above
-// the first threshold.
-void settle_heap(long ne)
-{
-    const size_t bytes = 31u << 20;
-    if (ne * sizeof(double) < 128 << 10) return;
-    if (volatile char *block = static_cast<volatile char *>(std::malloc(bytes))) {
-        block[0] = 0;
-        std::free(const_cast<char *>(block));
-    }
-}
-
 void HostMesh::build(int s_, int init_mode)
 {
     s = s_;
