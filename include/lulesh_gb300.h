@@ -422,10 +422,11 @@ int lulesh_batch_tuning(lulesh_batch *b, int size_class, int kernel, int *block,
  * tile, 0 for gathered corners (always 0 but for the split force kernel). */
 int lulesh_batch_staging(lulesh_batch *b, int size_class, int kernel, int *rows);
 /* Set a class's kernel launch shape by hand: threads per block (a multiple
- * of 32, at most 256), resident blocks per SM of the persistent grid
- * (>= 1, capped at what fits), staging depth rows (0; or 2 or 4 for the
- * split force kernel of a class that can be staged, block then ignored).
- * The shapes change no element's arithmetic. */
+ * of 32, at most 256), blocks per SM of the grid (>= 1; at most four waves of
+ * those that fit, which is what a batch starts with, or one of the staged
+ * kernel's), staging depth rows (0; or 2 or 4 for the split force kernel of a
+ * class that can be staged, block then ignored).  The shapes change no
+ * element's arithmetic. */
 int lulesh_batch_set_tuning(lulesh_batch *b, int size_class, int kernel, int block, int blocks_per_sm, int rows);
 
 void *lulesh_batch_stream(lulesh_batch *b);

@@ -906,7 +906,7 @@ int lulesh_batch_set_tuning(lulesh_batch *b, int cls, int kernel, int block, int
             return bfail(b, LULESH_ERR_ARG, "lulesh_batch_set_tuning: block must be a multiple of 32 up to 256");
         const int fit = max_blocks(b, kernel, block);
         if (fit < 1) return bfail(b, LULESH_ERR_ARG, "lulesh_batch_set_tuning: no block of that size fits on an SM");
-        const int per_sm = std::min(blocks_per_sm, fit);
+        const int per_sm = std::min(blocks_per_sm, kDefaultWaves * fit);
         b->cfg[cls][kernel] = {block, grid_for(b, cls, kernel, block, per_sm)};
     }
     destroy_graph(b);   // the run graph bakes in the launch shapes
