@@ -403,9 +403,9 @@ int lulesh_batch_zone_cycles(lulesh_batch *b, double *zone_cycles);
  * of the force kernel: its corners gathered from global memory (0), or
  * tiles of 2 or 4 element rows x 64 columns staged in shared memory (blocks
  * of 128 or 256 threads).
- * Choices are cached in the JSON file cache_path (keyed by GPU model, SM
- * count, precision, class, kernel; NULL: no cache); retune != 0 ignores
- * cached entries. */
+ * Choices are cached in the JSON file cache_path (keyed by a number for the
+ * library's kernels, GPU model, SM count, precision, class, kernel and its
+ * form; NULL: no cache); retune != 0 ignores cached entries. */
 int lulesh_batch_autotune(lulesh_batch *b, const char *cache_path, int retune);
 
 /* lulesh_batch_run in chunks of at most chunk cycles; after a chunk, when the

@@ -386,6 +386,10 @@ void default_cfg(lulesh_batch *b)
 
 const char *kKernelNames[kBatchKernels] = {"elem_force", "node_update", "elem_kinematics", "elem_material"};
 
+// What an entry was timed for: the format counts the kernels' own changes (2:
+// a tile's elements dealt out one per thread, several waves of blocks), and
+// the node update has two forms, by the nodes of the ensemble.
+constexpr int kShapeFormat = 2;
 std::string tune_key(const lulesh_batch *b, int cls, int kernel)
 {
     cudaDeviceProp prop;
@@ -393,9 +397,10 @@ std::string tune_key(const lulesh_batch *b, int cls, int kernel)
     cudaGetDevice(&dev);
     cudaGetDeviceProperties(&prop, dev);
     std::ostringstream o;
-    o << prop.name << "|sm" << prop.multiProcessorCount << "|"
+    o << "shapes" << kShapeFormat << "|" << prop.name << "|sm" << prop.multiProcessorCount << "|"
       << (b->precision == LULESH_PRECISION_SPLIT ? "split" : (b->dom.df == kArithDF64 ? "fp64" : "fp64ieee")) << "|class" << cls << "|"
       << kKernelNames[kernel];
+    if (kernel == 1 && b->dom.nn < kEarlyNodes) o << "|early";
     return o.str();
 }
 
