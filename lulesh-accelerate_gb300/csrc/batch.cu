@@ -410,6 +410,11 @@ std::string tune_key(const lulesh_batch *b, int cls, int kernel)
 struct TuneEntry {
     int block, per_sm, stage;
 };
+// Threads of a block that every kernel takes.
+bool block_allowed(int block) { return block >= 32 && block <= 256 && block % 32 == 0; }
+// A file may hold anything: what is no launch shape counts as no entry.
+bool launchable(const TuneEntry &e) { return block_allowed(e.block) && e.per_sm >= 1; }
+
 std::map<std::string, TuneEntry> read_cache(const char *path)
 {
     std::map<std::string, TuneEntry> m;
@@ -907,7 +912,7 @@ int lulesh_batch_set_tuning(lulesh_batch *b, int cls, int kernel, int block, int
         b->cfg[cls][kernel] = {rows * kTileCols,
                                (int)std::max(1LL, std::min(staged_tiles(b, cls, rows), (long long)b->sms * per_sm)), rows};
     } else {
-        if (block < 32 || block > 256 || block % 32)
+        if (!block_allowed(block))
             return bfail(b, LULESH_ERR_ARG, "lulesh_batch_set_tuning: block must be a multiple of 32 up to 256");
         const int fit = max_blocks(b, kernel, block);
         if (fit < 1) return bfail(b, LULESH_ERR_ARG, "lulesh_batch_set_tuning: no block of that size fits on an SM");
@@ -929,7 +934,7 @@ int lulesh_batch_autotune(lulesh_batch *b, const char *cache_path, int retune)
             const int tiles = k == 1 ? b->class_ntiles[c] : b->class_etiles[c];
             if (!tiles) continue;
             auto it = cache.find(tune_key(b, c, k));
-            if (it == cache.end() || retune) { need = true; continue; }
+            if (it == cache.end() || retune || !launchable(it->second)) { need = true; continue; }
             const TuneEntry &te = it->second;
             if (k == 0 && (te.stage == 2 || te.stage == 4) && can_stage(b, c)) {
                 const int per_sm = std::max(1, std::min(te.per_sm, batch_max_blocks_split_staged(te.stage)));

@@ -40,3 +40,13 @@ def test_entries_of_other_kernels_are_not_used(pkg, tmp_path):
     with pkg.Batch(SMALL, None, pkg.INIT_V2, 0) as b:
         b.autotune(str(cache))
         assert all(b.tuning()[f"class0/{k}"]["block"] in (64, 128, 256) for k in pkg.BATCH_KERNELS)
+
+
+@pytest.mark.parametrize("shape", [(0, 4, 0), (-64, 4, 0), (100, 4, 0), (512, 1, 0), (64, 0, 0), (64, -3, 0)])
+def test_bad_entries_are_timed_again(pkg, tmp_path, shape):
+    cache = tmp_path / "tuning.json"
+    marked(pkg, cache, 0, shape=shape)
+    with pkg.Batch(SMALL, None, pkg.INIT_V2, 0) as b:
+        b.autotune(str(cache))
+        assert all(b.tuning()[f"class0/{k}"]["block"] in (64, 128, 256) for k in pkg.BATCH_KERNELS)
+        assert b.run(5) == 5
