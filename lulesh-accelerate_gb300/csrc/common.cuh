@@ -39,17 +39,21 @@ __device__ __forceinline__ bool skip_step(const Dom &d)
     return d.sc->err_any != 0 || (d.gate != nullptr && *d.gate == 0);
 }
 
+__device__ __forceinline__ unsigned long long iabs(double x);   // |x| as its bit pattern, below
+
 // ---------------------------------------------------------------------
 // TimeIncrement (LULESH-OMP.cc:557-604)
 // ---------------------------------------------------------------------
 // x / 3, correctly rounded: the remainder of the product with the rounded
-// reciprocal is exact and corrects it (Markstein 1990).  The step is one
-// thread's chain of FP64 operations, and a division is a dozen of them; the
-// halving is exact as a product.
+// reciprocal is exact and corrects it (Markstein 1990); an infinity (four
+// times a step near the largest double) has none and stays itself.  The step
+// is one thread's chain of FP64 operations, and a division is a dozen of
+// them; the halving is exact as a product.
 __device__ __forceinline__ double third(double x)
 {
     const double q = x * (1.0 / 3.0), r = fma(-3.0, q, x);
-    return fma(r, 1.0 / 3.0, q);
+    const double y = fma(r, 1.0 / 3.0, q);
+    return iabs(x) == 0x7ff0000000000000ULL ? x : y;
 }
 __device__ __forceinline__ void time_increment(DevScalars *sc, const lulesh_params &P)
 {
