@@ -440,10 +440,14 @@ int create_context(const HostMesh *m, int s, int init_mode, int precision, const
     }
     const size_t state = (6 * (size_t)ctx->nn + 5 * (size_t)ctx->ne) * sizeof(double);
     if (cudaMallocHost(&ctx->h_sc, sizeof(DevScalars)) != cudaSuccess ||
-        cudaMallocHost(&ctx->h_stage, 16 * sizeof(int)) != cudaSuccess ||
-        (state <= kStagedState && cudaMallocHost(&ctx->h_state, state) != cudaSuccess)) {
+        cudaMallocHost(&ctx->h_stage, 16 * sizeof(int)) != cudaSuccess) {
         ctx->err = "cudaMallocHost failed";
         return bail(LULESH_ERR_CUDA);
+    }
+    // without the buffer states are copied field by field
+    if (state <= kStagedState && cudaMallocHost(&ctx->h_state, state) != cudaSuccess) {
+        ctx->h_state = nullptr;
+        cudaGetLastError();
     }
 
     Dom &d = ctx->dom;
