@@ -212,11 +212,13 @@ def _arg(a: np.ndarray):
     """The array's data for a ``double *`` argument of a call: a quarter of the
     time of ``_ptr`` (0.3 us, 1.4), which a call with eleven arrays notices.
     A view over the array's own buffer; read-only, empty and strided arrays
-    have none and go the general way."""
+    have none and go the general way, as does what is no array."""
     try:
-        return C.byref(C.c_double.from_buffer(a))
+        if isinstance(a, np.ndarray):
+            return C.byref(C.c_double.from_buffer(a))
     except (TypeError, ValueError, BufferError):
-        return _ptr(a)
+        pass
+    return _ptr(a)
 
 
 def _check(rc: int, handle=None):
