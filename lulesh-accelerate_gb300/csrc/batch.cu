@@ -145,13 +145,13 @@ __device__ void rebuild_lists(const BatchView &b)
         const int i = b.etile_inst[t];
         if (!b.inst_active[i]) continue;
         const int c = b.etile_class[t], slot = atomicAdd(&n[c], 1);
-        b.active_etiles[b.eclass_off[c] + slot] = {t * kTile, min(b.inst_elem_end[i], (t + 1) * kTile), i, t};
+        b.active_etiles[b.eclass_off[c] + slot] = {t * kTile, min(b.inst_elem_end[i], (t + 1) * kTile), i};
     }
     for (int t = threadIdx.x; t < b.n_ntiles; t += blockDim.x) {
         const int i = b.ntile_inst[t];
         if (!b.inst_active[i]) continue;
         const int c = b.ntile_class[t], slot = atomicAdd(&n[kMaxClasses + c], 1);
-        b.active_ntiles[b.nclass_off[c] + slot] = {t * kTile, min(b.inst_node_end[i], (t + 1) * kTile), i, t};
+        b.active_ntiles[b.nclass_off[c] + slot] = {t * kTile, min(b.inst_node_end[i], (t + 1) * kTile), i};
     }
     __syncthreads();
     if (threadIdx.x < 2 * kMaxClasses) b.counts[threadIdx.x] = n[threadIdx.x];

@@ -85,7 +85,6 @@ __device__ __forceinline__ df2 df2_dup(df64 x) { return df2_pack(x, x); }
 __device__ __forceinline__ df64 df2_x(df2 a) { return {f2_x(a.hi), f2_x(a.lo)}; }
 __device__ __forceinline__ df64 df2_y(df2 a) { return {f2_y(a.hi), f2_y(a.lo)}; }
 __device__ __forceinline__ df2n df2_both(df2 a) { return {a.hi, a.lo, f2_neg(a.hi)}; }
-__device__ __forceinline__ df2 df2_first(df2n a) { return {a.hi, a.lo}; }
 
 __device__ __forceinline__ df2 f2_two_sum(f2 a, f2 b)
 {
@@ -120,7 +119,6 @@ __device__ __forceinline__ df64 df_sum(df64 a, df64 b)
     const df64 s = two_sum(a.hi, b.hi);
     return {s.hi, __fadd_rn(s.lo, __fadd_rn(a.lo, b.lo))};
 }
-__device__ __forceinline__ df64 df_diff(df64 a, df64 b) { return df_sum(a, -b); }
 __device__ __forceinline__ df64 df_renorm(df64 a) { return two_sum(a.hi, a.lo); }
 __device__ __forceinline__ df64 df_tidy(df64 a) { return fast_two_sum(a.hi, a.lo); }
 

@@ -211,7 +211,7 @@ constexpr int kBatchKernels = 4;   // force, node update, kinematics, material
 // A tile that a running instance still needs: its first element (or node),
 // one past the last of them, the instance.
 struct ActiveTile {
-    int begin, end, inst, tile;
+    int begin, end, inst;
 };
 struct BatchView {
     int n_inst, n_classes, n_etiles, n_ntiles;
