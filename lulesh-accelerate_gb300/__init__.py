@@ -24,6 +24,7 @@ from __future__ import annotations
 import ctypes as C
 import os
 import sys
+import threading
 import weakref
 from dataclasses import dataclass, field
 from pathlib import Path
@@ -335,38 +336,61 @@ NODE_FIELDS = {"x", "y", "z", "xd", "yd", "zd", "fx", "fy", "fz", "nodalMass"}
 
 
 class _ResultArrays:
-    """Arrays for a context's downloads: those of its last two, filled again
-    once the caller has let go of all of them, else new ones.
+    """Arrays for downloads that are given none: those of earlier results of
+    the same size, once the caller has let go of all of them, else new ones.
 
     Eleven fresh arrays a step can spend more time on page faults than the
     step takes, whenever the C library has given the last ones' pages back
     (s=86: 1.1 ms a step, up to 4.8 with the faults).  An array that anything
     else still refers to -- a Domain, a view, a tensor or buffer over it, a
-    weak reference -- is never filled again.  Kept are two downloads of up to
-    128 MB each; they go with the context."""
+    weak reference -- is never filled again.  Kept are the last four results,
+    192 MB in all (two at s=100), while a context is open; arrays below 128 kB
+    come from the C library's heap in any case and are left to it."""
 
-    KEPT, MOST_BYTES = 2, 128 << 20
+    MOST_SETS, MOST_BYTES, LEAST_ARRAY = 4, 192 << 20, 128 << 10
 
     def __init__(self):
-        self._sets = []
+        self._lock = threading.Lock()
+        self._sets, self._contexts = [], 0
 
     @staticmethod
     def _references(arrays):
         return [sys.getrefcount(a) + (1 << 20) * weakref.getweakrefcount(a) for a in arrays]
 
+    @staticmethod
+    def _bytes(arrays):
+        return sum(a.nbytes for a in arrays)
+
     def domain(self, ne: int, nn: int) -> Domain:
-        for i, arrays in enumerate(self._sets):
-            if max(self._references(arrays)) <= _UNHELD:
-                self._sets.append(self._sets.pop(i))
-                return Domain(*arrays)
-        dom = Domain.empty(ne, nn)
-        if 8 * (6 * nn + 5 * ne) <= self.MOST_BYTES:
-            self._sets = self._sets[1 - self.KEPT:] + [dom.arrays()]
-        return dom
+        if 8 * ne < self.LEAST_ARRAY:
+            return Domain.empty(ne, nn)
+        with self._lock:
+            for i in range(len(self._sets) - 1, -1, -1):   # the last one used: its pages are the warm ones
+                arrays = self._sets[i]
+                if (arrays[-1].size, arrays[0].size) == (ne, nn) and max(self._references(arrays)) <= _UNHELD:
+                    self._sets.append(self._sets.pop(i))
+                    return Domain(*arrays)
+            dom = Domain.empty(ne, nn)
+            if self._contexts:
+                self._sets.append(dom.arrays())
+                while len(self._sets) > self.MOST_SETS or sum(map(self._bytes, self._sets)) > self.MOST_BYTES:
+                    del self._sets[0]
+            return dom
+
+    def opened(self):
+        with self._lock:
+            self._contexts += 1
+
+    def closed(self):
+        with self._lock:
+            self._contexts -= 1
+            if not self._contexts:
+                self._sets = []
 
 
 # what _references counts of an array that only its list holds
 _UNHELD = _ResultArrays._references([np.empty(0)])[0]
+_results = _ResultArrays()
 
 
 class Lulesh:
@@ -388,11 +412,11 @@ class Lulesh:
         else:
             h = _handle
         self._h = h
+        _results.opened()
         es, ne, nn = C.c_int(), C.c_long(), C.c_long()
         _check(lib.lulesh_sizes(h, C.byref(es), C.byref(ne), C.byref(nn)), h)
         self.s = es.value
         self.num_elem, self.num_node = ne.value, nn.value
-        self._results = _ResultArrays()
 
     @classmethod
     def from_mesh(cls, mesh: dict, precision: int = FP64, params: Parameters | None = None) -> "Lulesh":
@@ -451,7 +475,7 @@ class Lulesh:
         if getattr(self, "_h", None):
             load_library().lulesh_destroy(self._h)
             self._h = None
-            self._results = _ResultArrays()
+            _results.closed()
 
     def __del__(self):
         try:
@@ -536,7 +560,7 @@ class Lulesh:
                                                    float(dom.time), float(dom.deltatime)), self._h)
 
     def download(self, into: Domain | None = None) -> Domain:
-        dom = into or self._results.domain(self.num_elem, self.num_node)
+        dom = into or _results.domain(self.num_elem, self.num_node)
         t, dt = C.c_double(), C.c_double()
         _check(load_library().lulesh_download_domain(self._h, *[_arg(v) for v in dom.arrays()],
                                                      C.byref(t), C.byref(dt)), self._h)
