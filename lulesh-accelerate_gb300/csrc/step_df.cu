@@ -51,7 +51,7 @@ __device__ __forceinline__ ModePacks field_modes(const double *__restrict__ f, c
 // are worth their 336 bytes: the kinematics kernel has the linear ones in
 // hand and completes them in 6 % more time (1196 -> 1268 us at s=192), and
 // the force kernel is spared its 24 gathers, 21 FP64 differences and as many
-// conversions (1316 -> 1046 us; s=96 172 -> 134, s=47 28.9 -> 23.2).
+// conversions (1316 -> 1046 us, 1004 now; s=96 172 -> 135, s=47 28.9 -> 23.2).
 __device__ __forceinline__ void store_geometry_df(double *geo, size_t ne, int k, int field, const ModePacks &m)
 {
     ulonglong2 *g = reinterpret_cast<ulonglong2 *>(geo) + (size_t)(3 * field) * ne + k;
@@ -247,9 +247,10 @@ __device__ __forceinline__ void elem_force_components(const Dom &d, int k, DevSc
 __device__ __forceinline__ void elem_force_df(const Dom &d, int k, DevScalars *sc) { elem_force_components(d, k, sc, 0, 3); }
 
 // 168 registers, three blocks of 128 threads per SM: the FP32 pipe is 71 %
-// busy, the rest dependent results.  1024 us at s=192 (1850 in scalar pairs
-// over the corners, 1316 on packed pairs over the modes, then the velocities'
-// modes kept); four blocks at 128 registers 1090, blocks of 64 threads 1036, of
+// busy, the rest dependent results.  1004 us at s=192 in mid-blast, 970 from
+// the Sedov start (in mid-blast 1850 in scalar pairs over the corners, 1316 on
+// packed pairs over the modes, then the velocities' modes kept); when it was
+// 1024, four blocks at 128 registers took 1090, blocks of 64 threads 1036, of
 // 192 1105, of 384 1301.
 __global__ void __launch_bounds__(kBlockElem) k_elem_force_df(const __grid_constant__ Dom d)
 {
@@ -573,7 +574,7 @@ __device__ __forceinline__ void elem_material_df(const Dom &d, int k, DevScalars
 // kernel waits on its neighbour loads, and the extra warps hide them better
 // than the spills cost (0.88 ms at 24 warps, 0.81 at 28, 0.78 at 32, s=192,
 // when it took that long).  With cheaper conversions and the parameters'
-// pairs from the host it takes 0.48 ms.
+// pairs from the host it took 0.48 ms, 0.50 with the functions' second word.
 template <bool kConstraints>
 __global__ void __launch_bounds__(kMatBlockFactor * kBlockElem, 2) k_elem_material_df(const __grid_constant__ Dom d)
 {
